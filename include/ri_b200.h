@@ -219,7 +219,7 @@ int ri_silu_and_mul(const void* d_in, void* d_out, int32_t rows, int32_t inter, 
  * (`retroinfer_prefill_attn`: flash_attn_with_kvcache(q, k_cache, v_cache, causal)) and attn_hub/flash_attn.py:4-13.
  * d_q, d_out: [batch, seq_len, q_heads, 128]; d_k, d_v: [batch, seq_len, kv_heads, 128] (token-major, contiguous);
  * query head h attends kv head h / (q_heads / kv_heads); causal != 0: token i sees tokens 0..i.
- * d_scratch: ri_prefill_attn_scratch_bytes() bytes (the transposed copy of V), contents irrelevant;
+ * d_scratch: not used any more, may be null (ri_prefill_attn_scratch_bytes() keeps its values);
  * d_error: [1], must be zero on entry; set non-zero if a bounded device-side wait ran out.
  * ------------------------------------------------------------------------------------------ */
 int64_t ri_prefill_attn_scratch_bytes(int32_t batch, int32_t seq_len, int32_t kv_heads);

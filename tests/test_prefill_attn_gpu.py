@@ -65,3 +65,24 @@ def test_bad_arguments_are_rejected():
     assert _lib.lib.ri_prefill_attn(None, None, None, None, None, None, 1, 128, 4, 1, 1, 0, None) == -1
     assert _lib.lib.ri_prefill_attn_scratch_bytes(1, 0, 1) == -1
     assert _lib.lib.ri_prefill_attn_scratch_bytes(2, 1000, 2) == 2 * 2 * 128 * 1024 * 2
+
+
+# two query tiles per CTA or one with its key/value tiles split over two groups (fewer pairs of query tiles than SMs), an
+# odd number of tiles, more items than SMs (persistent CTAs), rows of the next request behind a request's last tile.
+# Same tolerance as above; NaN in a neighbouring request must not leak in.
+@pytest.mark.parametrize("batch,seq,hq,hk,causal", [
+    (1, 129, 2, 1, True), (1, 257, 1, 1, False), (3, 385, 5, 1, True), (2, 1200, 40, 8, True), (2, 1300, 28, 4, False),
+    (1, 2500, 24, 8, True),
+])
+def test_query_tile_pairs_and_split_walks(batch, seq, hq, hk, causal):
+    from retrievalattention_b200.attn_hub import retroinfer_attn as ra
+
+    g = torch.Generator(device="cuda").manual_seed(seq)
+    mk = lambda h: torch.randn((batch, seq, h, 128), generator=g, device="cuda").to(torch.bfloat16)   # noqa: E731
+    q, k, v = mk(hq), mk(hk), mk(hk)
+    if batch > 1:
+        k[1:], v[1:] = float("nan"), float("nan")
+    out = ra.retroinfer_prefill_attn(q, k, v, causal)[:1]
+    ra.check_prefill_errors()
+    err = (out.float() - reference(q[:1], k[:1], v[:1], causal)).abs()
+    assert err.max() <= 2e-2 and err.mean() <= 2e-3, (float(err.max()), float(err.mean()))
