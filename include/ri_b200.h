@@ -270,6 +270,22 @@ typedef struct ri_kmeans {
 int64_t ri_kmeans_scratch_bytes(const ri_kmeans* p);
 int ri_kmeans_build(const ri_kmeans* p, void* stream);
 
+/* The same for one request's prompt as the model hands it over, without copies in between (center must be 1):
+ * p->d_keys / d_values point at the first valid token of token-major rows [n_sink + n_tokens + n_recent, Z, 128]; the
+ * n_tokens rows behind the n_sink sink rows are clustered, the sink rows and the n_recent rows behind the clustered ones
+ * are stored at rows 0 .. n_sink + n_recent - 1 of every group's steady zone.  Replaces the slicing, transposing and
+ * copying around the clustering in cache_hub/retroinfer_cache.py:383-440. */
+typedef struct ri_kmeans_prompt {
+  int32_t n_sink;
+  int32_t n_recent;
+  int64_t out_group_rows;    /* rows from one group's cluster-contiguous copy to the next one's (>= n_tokens) */
+  int64_t steady_group_rows; /* the same of the steady zone */
+  void* d_steady_keys;       /* out [Z, steady_group_rows, 128], may be NULL when n_sink + n_recent is 0 */
+  void* d_steady_values;
+  uint8_t* d_empty;          /* out [Z, C]: 1 where a cluster has no members, may be NULL */
+} ri_kmeans_prompt;
+int ri_kmeans_build_prompt(const ri_kmeans* p, const ri_kmeans_prompt* q, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Gather/copy operators of the host tier (rows of 128 16-bit elements, pages of 8 rows).  Same
  * argument order and meaning as the reference's pybind functions

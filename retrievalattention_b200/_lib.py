@@ -57,6 +57,15 @@ class KMeans(C.Structure):
     ]
 
 
+class KMeansPrompt(C.Structure):
+    """Mirror of ``struct ri_kmeans_prompt``."""
+
+    _fields_ = [
+        ("n_sink", C.c_int32), ("n_recent", C.c_int32), ("out_group_rows", C.c_int64), ("steady_group_rows", C.c_int64),
+        ("d_steady_keys", C.c_void_p), ("d_steady_values", C.c_void_p), ("d_empty", C.c_void_p),
+    ]
+
+
 class WaveViews(C.Structure):
     _fields_ = [("d_scores", C.c_void_p), ("d_dist_keys", C.c_void_p), ("d_exact_rows", C.c_void_p),
                 ("d_n_exact", C.c_void_p)]
@@ -91,6 +100,8 @@ def _load() -> C.CDLL:
     lib.ri_kmeans_scratch_bytes.argtypes = [C.POINTER(KMeans)]
     lib.ri_kmeans_build.restype = C.c_int
     lib.ri_kmeans_build.argtypes = [C.POINTER(KMeans), C.c_void_p]
+    lib.ri_kmeans_build_prompt.restype = C.c_int
+    lib.ri_kmeans_build_prompt.argtypes = [C.POINTER(KMeans), C.POINTER(KMeansPrompt), C.c_void_p]
     lib.ri_wb_create.restype = C.c_void_p
     lib.ri_wb_create.argtypes = [C.c_int32] * 9
     lib.ri_wb_destroy.restype = None

@@ -26,7 +26,7 @@ def _run(keys, values, num_centroids, num_iters, num_segments, center, want_layo
         "cluster_size": torch.empty((z, num_centroids), dtype=dt, device=dev),
         "cluster_count": torch.empty((z, num_centroids), dtype=torch.int32, device=dev),
         "cluster_offset": torch.empty((z, num_centroids + 1), dtype=torch.int32, device=dev),
-        "error": torch.zeros((1,), dtype=torch.int32, device=dev),
+        "error": torch.empty((1,), dtype=torch.int32, device=dev),
     }
     if want_lists:
         out["assign"] = torch.empty((z, n), dtype=torch.int32, device=dev)
@@ -65,6 +65,42 @@ def build_index(keys: torch.Tensor, values: torch.Tensor, num_centroids: int, nu
     dtype), ``cluster_count``, ``cluster_offset``, cluster-contiguous ``keys``/``values``,
     ``mean_key``, ``error`` (1 if a device-side wait timed out) and, on request, ``assign``/``order``."""
     return _run(keys, values, num_centroids, num_iters, num_segments, True, True, want_lists)
+
+
+def build_prompt_index(keys: torch.Tensor, values: torch.Tensor, num_segments: int, sink: int, recent: int, out: dict,
+                       num_iters: int = 10) -> torch.Tensor:
+    """Index of one request's layer straight from its prompt into the caller's tensors: ``keys``/``values``
+    ``[tokens, kv_heads, 128]`` (the valid tokens, contiguous) of which the first ``sink`` and the last ``recent`` go to
+    the steady zone and the rest are clustered.  ``out`` holds contiguous ``centroids``, ``value_sum``, ``cluster_size``,
+    ``cluster_count``, ``cluster_offset``, ``empty`` (bool) of the request's heads, and ``keys``, ``values``,
+    ``steady_keys``, ``steady_values`` ``[kv_heads, rows, 128]`` whose rows behind the used ones stay as they are.
+    Returns the status word (non-zero if a device-side wait timed out)."""
+    tokens, z, _ = keys.shape
+    dt, n, c = keys.dtype, tokens - sink - recent, out["centroids"].shape[1]
+    assert keys.is_contiguous() and values.is_contiguous() and values.shape == keys.shape
+    p, q = _lib.KMeans(), _lib.KMeansPrompt()
+    p.groups, p.n_tokens, p.n_centroids, p.n_segments, p.n_iters = z, n, c, num_segments, num_iters
+    p.dtype, p.center = _lib.dtype_code(dt), 1
+    need = _lib.lib.ri_kmeans_scratch_bytes(C.byref(p))
+    if need < 0:
+        raise ValueError(f"ri_kmeans: {_lib.lib.ri_last_error().decode()}")
+    scratch = torch.empty(need, dtype=torch.uint8, device=keys.device)
+    error = torch.empty((1,), dtype=torch.int32, device=keys.device)
+    p.d_keys, p.d_values, p.d_scratch, p.d_error = keys.data_ptr(), values.data_ptr(), scratch.data_ptr(), error.data_ptr()
+    for name in ("centroids", "value_sum", "cluster_size", "cluster_count", "cluster_offset"):
+        assert out[name].is_contiguous() and out[name].shape[0] == z
+        setattr(p, "d_" + name, out[name].data_ptr())
+    for name in ("keys", "values", "steady_keys", "steady_values"):
+        assert out[name].is_contiguous() and out[name].dtype == dt and out[name].shape[0] == z
+    assert out["keys"].shape == out["values"].shape and out["keys"].shape[1] >= n
+    assert out["steady_keys"].shape == out["steady_values"].shape and out["empty"].is_contiguous()
+    p.d_keys_out, p.d_values_out = out["keys"].data_ptr(), out["values"].data_ptr()
+    q.n_sink, q.n_recent, q.out_group_rows = sink, recent, out["keys"].shape[1]
+    q.steady_group_rows = out["steady_keys"].shape[1]
+    q.d_steady_keys, q.d_steady_values = out["steady_keys"].data_ptr(), out["steady_values"].data_ptr()
+    q.d_empty = out["empty"].data_ptr()
+    _lib.check(_lib.lib.ri_kmeans_build_prompt(C.byref(p), C.byref(q), _lib.current_stream()), "ri_kmeans_build_prompt")
+    return error          # the scratch goes back to the allocator, which reuses it in stream order
 
 
 def segment_k_means(key: torch.Tensor, value: torch.Tensor, num_centroids: int, num_iters: int = 10,

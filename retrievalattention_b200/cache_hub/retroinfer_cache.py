@@ -52,7 +52,7 @@ import torch
 
 from .. import wave
 from .cache import KV_Cache
-from .kmeans import build_index
+from .kmeans import build_index, build_prompt_index
 
 THRESHOLD_LENGTH = 1024   # reference: re-index period in generated tokens (:13)
 
@@ -227,24 +227,20 @@ class retroinfer_cache(KV_Cache):
         start, end, total = self.static_pattern_start, self.static_pattern_end, self.static_pattern_start + self.static_pattern_end
         valid_length = seq_len - total - vs
 
-        temp_keys = key_states[0, vs + start:seq_len - end].transpose(0, 1).contiguous()      # [kv_heads, N_b, d]
-        temp_values = value_states[0, vs + start:seq_len - end].transpose(0, 1).contiguous()
-
-        sk, sv = self.steady_zone_keys[layer_idx], self.steady_zone_values[layer_idx]
-        sk[batch_idx, :, :start] = key_states[0, vs:vs + start].transpose(0, 1)
-        sk[batch_idx, :, start:total] = key_states[0, seq_len - end:seq_len].transpose(0, 1)
-        sv[batch_idx, :, :start] = value_states[0, vs:vs + start].transpose(0, 1)
-        sv[batch_idx, :, start:total] = value_states[0, seq_len - end:seq_len].transpose(0, 1)
-
-        r = build_index(temp_keys, temp_values, self.n_centroids, self.n_segment)
         rows = slice(batch_idx * self.kv_head, (batch_idx + 1) * self.kv_head)
-        self.centroids[layer_idx][rows].copy_(r["centroids"])
-        self.value_sum[layer_idx][rows].copy_(r["value_sum"])
-        self.cluster_size[layer_idx][rows].copy_(r["cluster_size"])
-        self.cluster_count[layer_idx][rows].copy_(r["cluster_count"])
-        self.cluster_offset[layer_idx][rows].copy_(r["cluster_offset"])
-        self.centroids_mask[layer_idx][rows].copy_(r["cluster_count"] == 0)
-        self._error_flags.append(r["error"])
+        out = {"centroids": self.centroids[layer_idx][rows], "value_sum": self.value_sum[layer_idx][rows],
+               "cluster_size": self.cluster_size[layer_idx][rows], "cluster_count": self.cluster_count[layer_idx][rows],
+               "cluster_offset": self.cluster_offset[layer_idx][rows], "empty": self.centroids_mask[layer_idx][rows],
+               "steady_keys": self.steady_zone_keys[layer_idx][batch_idx],
+               "steady_values": self.steady_zone_values[layer_idx][batch_idx]}
+        if self.kv_on_host:
+            laid_out = torch.empty((2, self.kv_head, valid_length, head_dim), dtype=self.dtype, device=key_states.device)
+            out["keys"], out["values"] = laid_out[0], laid_out[1]
+        else:
+            out["keys"], out["values"] = self.list_keys[layer_idx][batch_idx], self.list_values[layer_idx][batch_idx]
+        self._error_flags.append(build_prompt_index(key_states[0, vs:].to(self.dtype).contiguous(),
+                                                    value_states[0, vs:].to(self.dtype).contiguous(),
+                                                    self.n_segment, start, end, out))
         if self.kv_on_host:
             # the offload of this request-layer's laid-out rows runs on a side stream, under the clustering of the next
             # request-layer (the reference's offload <-> k-means overlap, :388-403); at most two laid-out copies are
@@ -257,16 +253,13 @@ class retroinfer_cache(KV_Cache):
             off.wait_stream(torch.cuda.current_stream(dev))
             with torch.cuda.stream(off):
                 for h in range(self.kv_head):      # one contiguous run per head: a plain asynchronous copy each
-                    self.list_keys[layer_idx][batch_idx, h, :valid_length].copy_(r["keys"][h], non_blocking=True)
-                    self.list_values[layer_idx][batch_idx, h, :valid_length].copy_(r["values"][h], non_blocking=True)
+                    self.list_keys[layer_idx][batch_idx, h, :valid_length].copy_(out["keys"][h], non_blocking=True)
+                    self.list_values[layer_idx][batch_idx, h, :valid_length].copy_(out["values"][h], non_blocking=True)
                 done.record(off)
-            self._keep_alive.append((done, r))
+            self._keep_alive.append((done, out))
             while len(self._keep_alive) > 2:
                 self._keep_alive.pop(0)[0].synchronize()
-            self.wave_buffer[layer_idx].async_construction(None, r["cluster_count"], batch_idx)
-        else:
-            self.list_keys[layer_idx][batch_idx, :, :valid_length].copy_(r["keys"])
-            self.list_values[layer_idx][batch_idx, :, :valid_length].copy_(r["values"])
+            self.wave_buffer[layer_idx].async_construction(None, out["cluster_count"], batch_idx)
 
         if layer_idx == self.layer_num - 1 and batch_idx + bsz == self.batch_size:
             self.context += seq_len

@@ -32,6 +32,20 @@ int ri_fail(int status, const char* fmt, ...);
       return ri_fail(RI_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e__));      \
   } while (0)
 
+// SMs of the current device (asked once per device).
+static inline int ri_sm_count(int* out) {
+  static int cached[64] = {0};
+  int dev = 0;
+  RI_CUDA_OK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || cached[dev] == 0) {
+    RI_CUDA_OK(cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev));
+    if (dev >= 0 && dev < 64) cached[dev] = *out;
+    return RI_OK;
+  }
+  *out = cached[dev];
+  return RI_OK;
+}
+
 static inline int64_t ri_align_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 __host__ __device__ constexpr size_t ri_align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
@@ -85,6 +99,27 @@ __device__ __forceinline__ uint16_t ri_ordered_key(uint16_t b) {
 
 __device__ __forceinline__ uint4 ri_ldg16(const uint4* p) { return __ldg(p); }
 
+// ---- cp.async ----------------------------------------------------------------------------------
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// ---- split cluster barrier -----------------------------------------------------------------------
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();   // .aligned: the whole warp must execute the instruction together
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 constexpr float RI_LOG2E = 1.4426950408889634f;
 
 // ---- programmatic dependent launch ------------------------------------------------------------
@@ -101,10 +136,12 @@ constexpr float RI_LOG2E = 1.4426950408889634f;
 // on: on one GPU it makes no difference to the decode kernel, between several GPUs the wait
 // kernel's launch hides behind the decode kernel and the next decode kernel's behind the wait.
 // The element-wise kernels of the decode layer (id 8) are on: their launch hides behind the library GEMM
-// in front of them (measured: 2 % of the whole model step).
+// in front of them (measured: 2 % of the whole model step), and so are those of the clustering build (ids 9, 10).
+__device__ __forceinline__ void ri_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void ri_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void ri_pdl_enter() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  ri_pdl_trigger();
+  ri_pdl_wait();
 }
 
 template <typename... KArgs, typename... Args>
@@ -118,7 +155,7 @@ inline cudaError_t ri_launch_pdl_id(int id, void (*kernel)(KArgs...), dim3 grid,
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  static const int mask = getenv("RI_PDL_MASK") ? atoi(getenv("RI_PDL_MASK")) : 0x163;   // per-kernel switch
+  static const int mask = getenv("RI_PDL_MASK") ? atoi(getenv("RI_PDL_MASK")) : 0x763;   // per-kernel switch
   cfg.attrs = attr;
   cfg.numAttrs = (mask >> id) & 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);

@@ -10,7 +10,7 @@
 //            over blocks, eight epilogue warps.
 //   bucket   stable counting sort of the tokens of a problem by cluster: counts, offsets and
 //            the member list in ascending token order (deterministic, no global atomics).
-//   update   one warp per cluster sums its member rows in list order (fp32), forms the mean,
+//   update   a warp per run of clusters sums their member rows in list order (fp32), forms the means,
 //            optionally L2-normalises, and stores the centroid in the key dtype if the cluster
 //            is non-empty.  On the last iteration the same pass also produces the value sums
 //            and writes the cluster-contiguous copy of K and V.
@@ -21,12 +21,15 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <cooperative_groups.h>
+
 #include "ri_common.cuh"
 #include "ri_tc.cuh"
 
 namespace {
 
 using namespace ri_tc;
+namespace cg = cooperative_groups;
 
 constexpr int kTileM = 128;       // tokens per CTA tile
 constexpr int kTileN = 128;       // centroids per MMA tile
@@ -54,16 +57,30 @@ struct AssignArgs {
 // lowest index, the rule of torch.argmax), so nothing in the epilogue is a serial chain.
 // Every mbarrier wait has a time and an iteration limit; on expiry the CTA records where it gave up, releases its
 // TMEM and returns.
-constexpr int kWideThreads = 320;
+constexpr int kEpilogueWarps = 8;
+constexpr int kWideThreads = 64 + 32 * kEpilogueWarps;
 constexpr int kWideBStages = 3;
 constexpr uint32_t kWideTmemCols = 512;
-constexpr int kWideSmem = 1024 /*align*/ + 2 * 4 * kHalfBytes /*A: 2 blocks x 2 tiles*/ +
-                          kWideBStages * 2 * kHalfBytes /*B*/ + 256 /*barriers*/;
+// The dynamic block is all the shared memory there is, so that it starts on the 1024-byte boundary that tiles with the
+// 128-byte swizzle need: the small arrays stand behind the tiles.
+constexpr int kSmallBytes = 256 + 16;      // barriers, then TMEM base, abort and skip words
+constexpr int kWideTiles = 2 * 4 * kHalfBytes /*A: 2 blocks x 2 tiles*/ + kWideBStages * 2 * kHalfBytes /*B*/;
+constexpr int kWideSmem = kWideTiles + kSmallBytes;
 
 struct WideArgs {
   AssignArgs a;
-  int blocks_per_cta;    // 256-token blocks a CTA works through
+  int n_units;           // units of work over all problems: blocks of 256 tokens (wide) or tiles of 128 (resident)
+  int per_problem;       // units of one problem
 };
+// A persistent CTA's share: units [lo, hi) of the flat sequence over problems, so that the CTAs differ by one unit at most.
+__device__ __forceinline__ void unit_share(const WideArgs& w, int& lo, int& hi) {
+  lo = (int)((int64_t)w.n_units * blockIdx.x / gridDim.x);
+  hi = (int)((int64_t)w.n_units * (blockIdx.x + 1) / gridDim.x);
+}
+// first token row (of all groups' rows) of a problem
+__device__ __forceinline__ int64_t problem_row(const AssignArgs& a, int problem) {
+  return (int64_t)(problem / a.seg_per_group) * a.group_stride + (int64_t)(problem % a.seg_per_group) * a.n_tok;
+}
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
@@ -71,44 +88,99 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return d;
 }
 
-// arg-max of 32 accumulator columns against the running (best, best_idx).  FULL: all 32 columns exist.
-template <bool FULL>
-__device__ __forceinline__ void argmax32(const uint32_t (&r)[32], int col_base, int valid, float& best, int& best_idx) {
-  float v[32];
+__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+
+// Running arg-max of a token over blocks of 32 accumulator columns.  Which column of a block is the maximum is not looked
+// for in every block that raises it (with 32 tokens in a warp nearly every block does for one of them, and a search costs
+// several times the maximum itself): the 32 values of the winning block are kept, by 16 packed moves, and searched once,
+// in `index`.  The first column equal to the maximum wins, as with torch.argmax.
+struct RunningMax {
+  float best;
+  int base;              // first column of the winning block
+  uint64_t kept[16];     // its values
+
+  __device__ __forceinline__ void reset() {
+    best = -INFINITY;
+    base = 0;
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = FULL || i < valid ? __uint_as_float(r[i]) : -INFINITY;
-  float m11[11];
+    for (int i = 0; i < 16; ++i) kept[i] = 0ull;
+  }
+  // FULL: all 32 columns exist
+  template <bool FULL>
+  __device__ __forceinline__ void take(const uint32_t (&r)[32], int col_base, int valid) {
+    float v[32];
 #pragma unroll
-  for (int i = 0; i < 10; ++i) m11[i] = max3(v[3 * i], v[3 * i + 1], v[3 * i + 2]);
-  m11[10] = fmaxf(v[30], v[31]);
-  const float a0 = max3(m11[0], m11[1], m11[2]), a1 = max3(m11[3], m11[4], m11[5]), a2 = max3(m11[6], m11[7], m11[8]);
-  const float m = max3(max3(a0, a1, a2), m11[9], m11[10]);
-  if (m > best) {          // strict: an equal value in a later column never replaces an earlier one
-    // First column equal to the maximum, found on the FMA pipe (the compare-and-mask form of this search kept the
-    // ALU pipe, which also does every maximum, busier than the tensor pipe whenever a problem has few centroid
-    // tiles): v - m is exactly 0 for the maxima and negative elsewhere, so fma(v - m, 2^120, -i) is -i for them and
-    // far below -32 for the others (differences under 2^-115 do not occur between scores of ordinary magnitude);
-    // the maximum of those is minus the first index.
+    for (int i = 0; i < 32; ++i) v[i] = FULL || i < valid ? __uint_as_float(r[i]) : -INFINITY;
+    float m11[11];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) m11[i] = max3(v[3 * i], v[3 * i + 1], v[3 * i + 2]);
+    m11[10] = fmaxf(v[30], v[31]);
+    const float a0 = max3(m11[0], m11[1], m11[2]), a1 = max3(m11[3], m11[4], m11[5]), a2 = max3(m11[6], m11[7], m11[8]);
+    const float m = max3(max3(a0, a1, a2), m11[9], m11[10]);
+    const bool raise = m > best;             // strict: an equal value in a later block never replaces an earlier one
+    if (__any_sync(0xffffffffu, raise)) {
+      // two values per instruction on the FMA pipe: v + (-0) is v
+      const uint64_t neg_zero = 0x8000000080000000ull;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\t@p add.rn.f32x2 %0, %1, %2;\n\t}"
+            : "+l"(kept[i]) : "l"(pack_f2(v[2 * i], v[2 * i + 1])), "l"(neg_zero), "r"((int)raise));
+      best = raise ? m : best;
+      base = raise ? col_base : base;
+    }
+  }
+  __device__ __forceinline__ int index() const {
+    if (!(best > -INFINITY)) return 0;
+    // v - best is exactly 0 for the maxima and negative elsewhere, so fma(v - best, 2^120, -i) is -i for them and far below
+    // -32 for the others (differences under 2^-115 do not occur between scores of ordinary magnitude); the maximum of
+    // those is minus the first index.
     float w[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) w[i] = fmaf(v[i] - m, 0x1p120f, -(float)i);
+    for (int i = 0; i < 16; ++i) {
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(kept[i]));
+      w[2 * i] = fmaf(lo - best, 0x1p120f, -(float)(2 * i));
+      w[2 * i + 1] = fmaf(hi - best, 0x1p120f, -(float)(2 * i + 1));
+    }
     float t11[11];
 #pragma unroll
     for (int i = 0; i < 10; ++i) t11[i] = max3(w[3 * i], w[3 * i + 1], w[3 * i + 2]);
     t11[10] = fmaxf(w[30], w[31]);
     const float b0 = max3(t11[0], t11[1], t11[2]), b1 = max3(t11[3], t11[4], t11[5]), b2 = max3(t11[6], t11[7], t11[8]);
-    const float wm = max3(max3(b0, b1, b2), t11[9], t11[10]);
-    best = m;
-    best_idx = col_base + (int)(-wm);
+    return base + (int)(-max3(max3(b0, b1, b2), t11[9], t11[10]));
   }
-}
+  // one finished accumulator tile (128 columns) of this warp's TMEM lanes; 32 columns are on their way while others are reduced
+  template <bool FULL>
+  __device__ __forceinline__ void take_tile(uint32_t taddr, int col0, int valid) {
+    uint32_t r0[32], r1[32], r2[32];
+    tc_ld32(taddr, r0);
+    tc_ld32(taddr + 32, r1);
+    tc_wait_ld();
+    tc_ld_landed(r0);
+    tc_ld_landed(r1);
+    tc_ld32(taddr + 64, r2);
+    take<FULL>(r0, col0, valid);
+    take<FULL>(r1, col0 + 32, valid - 32);
+    tc_wait_ld();
+    tc_ld_landed(r2);
+    tc_ld32(taddr + 96, r0);
+    take<FULL>(r2, col0 + 64, valid - 64);
+    tc_wait_ld();
+    tc_ld_landed(r0);
+    take<FULL>(r0, col0 + 96, valid - 96);
+  }
+};
 
 __global__ void __launch_bounds__(kWideThreads, 1)
 kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __grid_constant__ CUtensorMap map_cent,
                           WideArgs w) {
   const AssignArgs& a = w.a;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;     // SW128 tiles need 1024-byte alignment
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
   const uint32_t sA = base;                                         // [block parity][tile][K half]
   const uint32_t sB = base + 2 * 4 * kHalfBytes;                    // [stage][K half]
   const uint32_t bars = sB + kWideBStages * 2 * kHalfBytes;
@@ -118,29 +190,29 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
   auto bar_b_empty = [&](int s) { return bars + 8u * (4 + kWideBStages + s); };
   auto bar_acc_full = [&](int b) { return bars + 8u * (4 + 2 * kWideBStages + b); };
   auto bar_acc_empty = [&](int b) { return bars + 8u * (6 + 2 * kWideBStages + b); };
-  __shared__ uint32_t s_tmem_base;
-  __shared__ int s_abort, s_skip;
+  uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + kWideTiles + 256);
+  int& s_abort = *reinterpret_cast<int*>(smem_raw + kWideTiles + 260);
+  int& s_skip = *reinterpret_cast<int*>(smem_raw + kWideTiles + 264);
 
   // once any CTA of this launch has given up, the rest leave at once (uniformly per CTA)
-  if (threadIdx.x == 0) s_skip = *reinterpret_cast<volatile int*>(a.error_flag);
+  if (threadIdx.x == 0) {
+    s_skip = *reinterpret_cast<volatile int*>(a.error_flag);
+    if (base & 1023u) *a.error_flag = s_skip = 19;      // the tiles would not lie as the descriptors say
+  }
   __syncthreads();
   if (s_skip) return;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int problem = blockIdx.y;
-  const int n_blocks_total = (a.n_tok + 2 * kTileM - 1) / (2 * kTileM);
-  const int first_block = blockIdx.x * w.blocks_per_cta;
-  const int nb = min(w.blocks_per_cta, n_blocks_total - first_block);       // > 0 by the grid's construction
-  const int64_t tok_row0 = (int64_t)(problem / a.seg_per_group) * a.group_stride +
-                           (int64_t)(problem % a.seg_per_group) * a.n_tok + (int64_t)first_block * 2 * kTileM;
-  const int cen_row0 = problem * a.n_cen;
+  int unit_lo, unit_hi;                             // this CTA's 256-token blocks
+  unit_share(w, unit_lo, unit_hi);
+  const int nb = unit_hi - unit_lo;                 // > 0 by the grid's construction
   const int n_tiles = (a.n_cen + kTileN - 1) / kTileN;
 
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int s = 0; s < 2; ++s) { mbar_init(bar_a_full(s), 1); mbar_init(bar_a_empty(s), 1); }
     for (int s = 0; s < kWideBStages; ++s) { mbar_init(bar_b_full(s), 1); mbar_init(bar_b_empty(s), 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(bar_acc_full(b), 1); mbar_init(bar_acc_empty(b), 8); }
+    for (int b = 0; b < 2; ++b) { mbar_init(bar_acc_full(b), 1); mbar_init(bar_acc_empty(b), kEpilogueWarps); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -153,6 +225,7 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
   volatile int* abort_flag = &s_abort;
+  ri_pdl_wait();           // launched programmatically: the set-up above runs under the kernel before
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -162,7 +235,8 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
         const int sa = blk & 1;
         if (!mbar_wait(bar_a_empty(sa), ((blk >> 1) & 1) ^ 1, abort_flag, 11)) return false;
         mbar_arrive_expect_tx(bar_a_full(sa), 4 * kHalfBytes);
-        const int row = (int)(tok_row0 + (int64_t)blk * 2 * kTileM);
+        const int unit = unit_lo + blk, problem = unit / w.per_problem;
+        const int row = (int)(problem_row(a, problem) + (int64_t)(unit - problem * w.per_problem) * 2 * kTileM);
 #pragma unroll
         for (int tile = 0; tile < 2; ++tile) {
           tma_load_2d(sA + (sa * 4 + tile * 2) * kHalfBytes, &map_keys, bar_a_full(sa), 0, row + tile * kTileM);
@@ -173,6 +247,7 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
       };
       bool ok = load_a(0);
       for (int blk = 0; ok && blk < nb; ++blk) {
+        const int cen_row0 = (unit_lo + blk) / w.per_problem * a.n_cen;
         for (int t = 0; ok && t < n_tiles; ++t) {
           const int s = b_issued % kWideBStages;
           ok = mbar_wait(bar_b_empty(s), ((b_issued / kWideBStages) & 1) ^ 1, abort_flag, 12);
@@ -228,52 +303,28 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
     // ---------------- epilogue: running arg-max over the centroid tiles ----------------
     const int tile = (warp - 2) >> 2;                // which token tile of the block
     const int lane_group = warp & 3;                 // TMEM lanes 32*lane_group .. +31 (a warp may touch only its quarter)
+    const int row = tile * kTileM + lane_group * 32 + lane;
     int j = 0;
     bool ok = true;
     for (int blk = 0; ok && blk < nb; ++blk) {
-      float best = -INFINITY;
-      int best_idx = 0;
+      RunningMax run;
+      run.reset();
       for (int t = 0; ok && t < n_tiles; ++t, ++j) {
         const int buf = j & 1;
         ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_full(buf), (j >> 1) & 1, abort_flag, 18));   // warp-uniform
         if (!ok) break;
         tc_fence_after();
-        const int col0 = t * kTileN;
-        const int valid = min(kTileN, a.n_cen - col0);
+        const int col0 = t * kTileN, valid = a.n_cen - col0;
         const uint32_t taddr = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * 2 * kTileN + tile * kTileN;
-        // the second half of the columns is on its way from TMEM while the first is being reduced
-        uint32_t r0[32], r1[32], r2[32], r3[32];
-        tc_ld32(taddr, r0);
-        tc_ld32(taddr + 32, r1);
-        tc_wait_ld();
-        tc_ld_landed(r0);
-        tc_ld_landed(r1);
-        tc_ld32(taddr + 64, r2);
-        tc_ld32(taddr + 96, r3);
-        if (valid == kTileN) {
-          argmax32<true>(r0, col0, 32, best, best_idx);
-          argmax32<true>(r1, col0 + 32, 32, best, best_idx);
-          tc_wait_ld();
-          tc_ld_landed(r2);
-          tc_ld_landed(r3);
-          argmax32<true>(r2, col0 + 64, 32, best, best_idx);
-          argmax32<true>(r3, col0 + 96, 32, best, best_idx);
-        } else {
-          argmax32<false>(r0, col0, valid, best, best_idx);
-          argmax32<false>(r1, col0 + 32, valid - 32, best, best_idx);
-          tc_wait_ld();
-          tc_ld_landed(r2);
-          tc_ld_landed(r3);
-          argmax32<false>(r2, col0 + 64, valid - 64, best, best_idx);
-          argmax32<false>(r3, col0 + 96, valid - 96, best, best_idx);
-        }
+        if (valid >= kTileN) run.take_tile<true>(taddr, col0, kTileN);
+        else run.take_tile<false>(taddr, col0, valid);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_acc_empty(buf));
       }
-      const int local_tok = (first_block + blk) * 2 * kTileM + tile * kTileM + lane_group * 32 + lane;
-      if (ok && local_tok < a.n_tok)
-        a.assign[tok_row0 + (int64_t)blk * 2 * kTileM + tile * kTileM + lane_group * 32 + lane] = best_idx;
+      const int unit = unit_lo + blk, problem = unit / w.per_problem;
+      const int local_tok = (unit - problem * w.per_problem) * 2 * kTileM + row;
+      if (ok && local_tok < a.n_tok) a.assign[problem_row(a, problem) + local_tok] = run.index();
     }
   }
 
@@ -295,44 +346,45 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
 // round, so a token's running arg-max lives in two warps, which meet through shared memory once per token tile
 // (equal maxima: the lower index wins, as within a warp).  Every warp runs a fixed number of token tiles and rounds
 // whatever its waits return, so the named barrier of that merge is always reached.
-// Measured on a segmented launch of configuration 2 (ncu): 580 us and the tensor pipe 48 % active, against 610 us /
-// 45 % for the wide kernel; with the epilogue's tcgen05.ld removed 388 us / 70 %, with a single 32-column load per
-// warp and round left 527 us / 52 % — the loads themselves, not the arithmetic behind them, hold the MMAs up; four
-// accumulator buffers of one centroid tile (the issuer three rounds ahead) were slower still (647 us).
+// CTAs are persistent, one per SM, each with an even run of token tiles over all problems.  A segmented launch of 8 heads x
+// 128K rows takes 152 us (before: 162); with the whole epilogue taken out 129 us, so most of what is left lies on the operand
+// side.  Sixteen epilogue warps instead of eight (176 us), token tiles asked for in L2 ten tiles ahead (no change) and
+// loading the first tokens under the kernel before (slower) were measured and left out.
 constexpr int kResSlots = 3;
-constexpr int kResSmem = 1024 /*align*/ + 4 * 2 * kHalfBytes /*B: 4 tiles*/ + kResSlots * 2 * kHalfBytes /*A ring*/ + 256;
+constexpr int kResTiles = 4 * 2 * kHalfBytes /*B: 4 tiles*/ + kResSlots * 2 * kHalfBytes /*A ring*/;
+constexpr int kResSmem = kResTiles + kSmallBytes + 2 * kTileM * 6 /*merge of a token's two warps*/;
 
 __global__ void __launch_bounds__(kWideThreads, 1)
 kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, const __grid_constant__ CUtensorMap map_cent,
                               WideArgs w) {
   const AssignArgs& a = w.a;
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
   const uint32_t sB = base;                                         // [centroid tile][K half]
   const uint32_t sA = base + 4 * 2 * kHalfBytes;                    // [slot][K half]
   const uint32_t bars = sA + kResSlots * 2 * kHalfBytes;
   auto bar_a_full = [&](int s) { return bars + 8u * s; };
   auto bar_a_empty = [&](int s) { return bars + 8u * (kResSlots + s); };
   const uint32_t bar_b_full = bars + 8u * (2 * kResSlots);
-  auto bar_acc_full = [&](int b) { return bars + 8u * (2 * kResSlots + 1 + b); };
-  auto bar_acc_empty = [&](int b) { return bars + 8u * (2 * kResSlots + 3 + b); };
-  __shared__ uint32_t s_tmem_base;
-  __shared__ int s_abort, s_skip;
-  __shared__ float s_best[2][kTileM];      // the merge of a token's two warps (indices fit 16 bits: <= 512 centroids)
-  __shared__ uint16_t s_idx[2][kTileM];
+  const uint32_t bar_b_empty = bars + 8u * (2 * kResSlots + 1);
+  auto bar_acc_full = [&](int b) { return bars + 8u * (2 * kResSlots + 2 + b); };
+  auto bar_acc_empty = [&](int b) { return bars + 8u * (2 * kResSlots + 4 + b); };
+  uint32_t& s_tmem_base = *reinterpret_cast<uint32_t*>(smem_raw + kResTiles + 256);
+  int& s_abort = *reinterpret_cast<int*>(smem_raw + kResTiles + 260);
+  int& s_skip = *reinterpret_cast<int*>(smem_raw + kResTiles + 264);
+  float (*s_best)[kTileM] = reinterpret_cast<float (*)[kTileM]>(smem_raw + kResTiles + kSmallBytes);   // [2][kTileM]
+  uint16_t (*s_idx)[kTileM] = reinterpret_cast<uint16_t (*)[kTileM]>(s_best + 2);     // <= 512 centroids: 16 bits
 
-  if (threadIdx.x == 0) s_skip = *reinterpret_cast<volatile int*>(a.error_flag);
+  if (threadIdx.x == 0) {
+    s_skip = *reinterpret_cast<volatile int*>(a.error_flag);
+    if (base & 1023u) *a.error_flag = s_skip = 19;      // the tiles would not lie as the descriptors say
+  }
   __syncthreads();
   if (s_skip) return;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int problem = blockIdx.y;
-  const int units_total = (a.n_tok + kTileM - 1) / kTileM;
-  const int first_unit = blockIdx.x * w.blocks_per_cta * 2;
-  const int nu = min(w.blocks_per_cta * 2, units_total - first_unit);       // > 0 by the grid's construction
-  const int64_t tok_row0 = (int64_t)(problem / a.seg_per_group) * a.group_stride +
-                           (int64_t)(problem % a.seg_per_group) * a.n_tok + (int64_t)first_unit * kTileM;
-  const int cen_row0 = problem * a.n_cen;
+  int unit_lo, unit_hi;                             // this CTA's 128-token tiles, over one problem or more
+  unit_share(w, unit_lo, unit_hi);
   const int n_tiles = (a.n_cen + kTileN - 1) / kTileN;              // 1 .. 4
   const int rounds = (n_tiles + 1) / 2;
 
@@ -340,7 +392,8 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
     s_abort = 0;
     for (int s = 0; s < kResSlots; ++s) { mbar_init(bar_a_full(s), 1); mbar_init(bar_a_empty(s), 1); }
     mbar_init(bar_b_full, 1);
-    for (int b = 0; b < 2; ++b) { mbar_init(bar_acc_full(b), 1); mbar_init(bar_acc_empty(b), 8); }
+    mbar_init(bar_b_empty, 1);
+    for (int b = 0; b < 2; ++b) { mbar_init(bar_acc_full(b), 1); mbar_init(bar_acc_empty(b), kEpilogueWarps); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -353,30 +406,38 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
   volatile int* abort_flag = &s_abort;
+  ri_pdl_wait();           // launched programmatically: the set-up above runs under the kernel before
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      mbar_arrive_expect_tx(bar_b_full, n_tiles * 2 * kHalfBytes);
-      for (int t = 0; t < n_tiles; ++t) {
-        tma_load_2d(sB + t * 2 * kHalfBytes, &map_cent, bar_b_full, 0, cen_row0 + t * kTileN);
-        tma_load_2d(sB + t * 2 * kHalfBytes + kHalfBytes, &map_cent, bar_b_full, 64, cen_row0 + t * kTileN);
-      }
-      int issued = 0;
+      int issued = 0, loaded = 0;                   // token tiles, problems
       bool ok = true;
-      for (int u = 0; ok && u < nu; ++u) {
-        const int s = u % kResSlots;
-        ok = mbar_wait(bar_a_empty(s), ((u / kResSlots) & 1) ^ 1, abort_flag, 21);
+      for (int unit = unit_lo; ok && unit < unit_hi;) {
+        const int problem = unit / w.per_problem, end = min(unit_hi, (problem + 1) * w.per_problem);
+        const int64_t row0 = problem_row(a, problem);
+        ok = mbar_wait(bar_b_empty, (loaded & 1) ^ 1, abort_flag, 20);      // the last problem's centroids are done with
         if (!ok) break;
-        mbar_arrive_expect_tx(bar_a_full(s), 2 * kHalfBytes);
-        const int row = (int)(tok_row0 + (int64_t)u * kTileM);
-        tma_load_2d(sA + s * 2 * kHalfBytes, &map_keys, bar_a_full(s), 0, row);
-        tma_load_2d(sA + s * 2 * kHalfBytes + kHalfBytes, &map_keys, bar_a_full(s), 64, row);
-        issued = u + 1;
+        mbar_arrive_expect_tx(bar_b_full, n_tiles * 2 * kHalfBytes);
+        for (int t = 0; t < n_tiles; ++t) {
+          tma_load_2d(sB + t * 2 * kHalfBytes, &map_cent, bar_b_full, 0, problem * a.n_cen + t * kTileN);
+          tma_load_2d(sB + t * 2 * kHalfBytes + kHalfBytes, &map_cent, bar_b_full, 64, problem * a.n_cen + t * kTileN);
+        }
+        ++loaded;
+        for (; ok && unit < end; ++unit) {
+          const int s = issued % kResSlots;
+          ok = mbar_wait(bar_a_empty(s), ((issued / kResSlots) & 1) ^ 1, abort_flag, 21);
+          if (!ok) break;
+          mbar_arrive_expect_tx(bar_a_full(s), 2 * kHalfBytes);
+          const int row = (int)(row0 + (int64_t)(unit - problem * w.per_problem) * kTileM);
+          tma_load_2d(sA + s * 2 * kHalfBytes, &map_keys, bar_a_full(s), 0, row);
+          tma_load_2d(sA + s * 2 * kHalfBytes + kHalfBytes, &map_keys, bar_a_full(s), 64, row);
+          ++issued;
+        }
       }
       if (*abort_flag) {
         // give our own copies still in flight a bounded chance to land before the CTA exits
-        mbar_wait(bar_b_full, 0, abort_flag, 26);
+        if (loaded > 0) mbar_wait(bar_b_full, (loaded - 1) & 1, abort_flag, 26);
         for (int u = max(0, issued - kResSlots); u < issued; ++u)
           mbar_wait(bar_a_full(u % kResSlots), (u / kResSlots) & 1, abort_flag, 27);
       }
@@ -384,11 +445,16 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      bool ok = mbar_wait(bar_b_full, 0, abort_flag, 22);
-      int j = 0;                       // rounds issued so far (accumulator buffer = j & 1)
-      for (int u = 0; ok && u < nu; ++u) {
+      bool ok = true;
+      int j = 0, u = 0, problem = -1, used = 0;     // rounds issued (accumulator buffer = j & 1), token tiles, problems
+      for (int unit = unit_lo; ok && unit < unit_hi; ++unit, ++u) {
         const int s = u % kResSlots;
-        ok = mbar_wait(bar_a_full(s), (u / kResSlots) & 1, abort_flag, 23);
+        if (unit / w.per_problem != problem) {
+          problem = unit / w.per_problem;
+          ok = mbar_wait(bar_b_full, used & 1, abort_flag, 22);
+          ++used;
+        }
+        ok = ok && mbar_wait(bar_a_full(s), (u / kResSlots) & 1, abort_flag, 23);
         for (int r = 0; ok && r < rounds; ++r, ++j) {
           const int buf = j & 1;
           ok = mbar_wait(bar_acc_empty(buf), ((j >> 1) & 1) ^ 1, abort_flag, 24);
@@ -410,68 +476,47 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
           }
           tc_commit(bar_acc_full(buf));
         }
-        if (ok) tc_commit(bar_a_empty(s));   // the token tile is free once all its MMAs have read it
+        if (ok) {
+          tc_commit(bar_a_empty(s));         // the token tile is free once all its MMAs have read it
+          if (unit + 1 < unit_hi && (unit + 1) / w.per_problem != problem) tc_commit(bar_b_empty);
+        }
       }
     }
   } else {
     // ---------------- epilogue: running arg-max, two warps per token ----------------
-    const int half = (warp - 2) >> 2;                // which centroid tile of a round
+    const int part = (warp - 2) >> 2;                // which centroid tile of a round
     const int lane_group = warp & 3;                 // TMEM lanes 32*lane_group .. +31 (a warp may touch only its quarter)
     const int row = lane_group * 32 + lane;          // this lane's token within the tile
     int j = 0;
     bool ok = true;
-    for (int u = 0; u < nu; ++u) {                   // fixed trip counts: the barrier below must be reached by all
-      float best = -INFINITY;
-      int best_idx = 0;
+    for (int unit = unit_lo; unit < unit_hi; ++unit) {   // fixed trip counts: the barrier below must be reached by all
+      RunningMax run;
+      run.reset();
       for (int r = 0; r < rounds; ++r, ++j) {
         const int buf = j & 1;
         ok = ok && __all_sync(0xffffffffu, mbar_wait(bar_acc_full(buf), (j >> 1) & 1, abort_flag, 25));   // warp-uniform
-        const int ct = 2 * r + half;
-        if (ok && ct < n_tiles) {
+        const int col0 = (2 * r + part) * kTileN, valid = a.n_cen - col0;
+        if (ok && valid > 0) {
           tc_fence_after();
-          const int col0 = ct * kTileN;
-          const int valid = min(kTileN, a.n_cen - col0);
-          const uint32_t taddr = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * 2 * kTileN + half * kTileN;
-          uint32_t r0[32], r1[32], r2[32], r3[32];
-          tc_ld32(taddr, r0);
-          tc_ld32(taddr + 32, r1);
-          tc_wait_ld();
-          tc_ld_landed(r0);
-          tc_ld_landed(r1);
-          tc_ld32(taddr + 64, r2);
-          tc_ld32(taddr + 96, r3);
-          if (valid == kTileN) {
-            argmax32<true>(r0, col0, 32, best, best_idx);
-            argmax32<true>(r1, col0 + 32, 32, best, best_idx);
-            tc_wait_ld();
-            tc_ld_landed(r2);
-            tc_ld_landed(r3);
-            argmax32<true>(r2, col0 + 64, 32, best, best_idx);
-            argmax32<true>(r3, col0 + 96, 32, best, best_idx);
-          } else {
-            argmax32<false>(r0, col0, valid, best, best_idx);
-            argmax32<false>(r1, col0 + 32, valid - 32, best, best_idx);
-            tc_wait_ld();
-            tc_ld_landed(r2);
-            tc_ld_landed(r3);
-            argmax32<false>(r2, col0 + 64, valid - 64, best, best_idx);
-            argmax32<false>(r3, col0 + 96, valid - 96, best, best_idx);
-          }
+          const uint32_t taddr = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * 2 * kTileN + part * kTileN;
+          if (valid >= kTileN) run.take_tile<true>(taddr, col0, kTileN);
+          else run.take_tile<false>(taddr, col0, valid);
           tc_fence_before();
         }
         __syncwarp();
         if (ok && lane == 0) mbar_arrive(bar_acc_empty(buf));
       }
       // the two warps of a token meet (buffers alternate per token tile, so one barrier per tile is enough)
-      const int par = u & 1;
-      if (half == 1) { s_best[par][row] = best; s_idx[par][row] = (uint16_t)best_idx; }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (half == 0) {
+      const int par = unit & 1;
+      int best_idx = run.index();
+      if (part == 1) { s_best[par][row] = run.best; s_idx[par][row] = (uint16_t)best_idx; }
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpilogueWarps) : "memory");
+      if (part == 0) {
         const float ob = s_best[par][row];
         const int oi = (int)s_idx[par][row];
-        if (ob > best || (ob == best && oi < best_idx)) best_idx = oi;
-        const int local_tok = (first_unit + u) * kTileM + row;
-        if (ok && local_tok < a.n_tok) a.assign[tok_row0 + (int64_t)u * kTileM + row] = best_idx;
+        if (ob > run.best || (ob == run.best && oi < best_idx)) best_idx = oi;
+        const int problem = unit / w.per_problem, local_tok = (unit - problem * w.per_problem) * kTileM + row;
+        if (ok && local_tok < a.n_tok) a.assign[problem_row(a, problem) + local_tok] = best_idx;
       }
     }
   }
@@ -485,25 +530,41 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
   }
 }
 
+// Rows of 128 channels that are not necessarily one behind the other: row r of group z starts at
+// (z * group + r * row) 256-byte units.
+struct RowPlace { int64_t group, row; };
+
 // ---- centre ---------------------------------------------------------------------------------
 constexpr int kMeanRows = 2048;   // rows per partial-sum CTA
 
 template <int DT>
-__global__ void __launch_bounds__(256) colsum_partial_kernel(const uint4* __restrict__ keys, float* __restrict__ partial,
-                                                             int n_tok, int chunks) {
+__global__ void __launch_bounds__(256) colsum_partial_kernel(const uint4* __restrict__ keys, RowPlace src,
+                                                             float* __restrict__ partial, int n_tok, int chunks) {
   const int z = blockIdx.y, chunk = blockIdx.x;
   const int piece = threadIdx.x & 15, rl = threadIdx.x >> 4;   // 16 pieces of 8 channels x 16 row lanes
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   const int r0 = chunk * kMeanRows, r1 = min(n_tok, r0 + kMeanRows);
-  for (int r = r0 + rl; r < r1; r += 16) {
-    const uint4 v = ri_ldg16(keys + ((int64_t)z * n_tok + r) * 16 + piece);
+  constexpr int kAhead = 8;          // rows in flight per thread; they are added in row order
+  auto add = [&](const uint4& v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       acc[2 * i] += Elem<DT>::from_bits((uint16_t)(w[i] & 0xffffu));
       acc[2 * i + 1] += Elem<DT>::from_bits((uint16_t)(w[i] >> 16));
     }
+  };
+  const uint4* from = keys + z * src.group * 16 + piece;
+  int r = r0 + rl;
+  for (; r + 16 * (kAhead - 1) < r1; r += 16 * kAhead) {
+    uint4 v[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[u].x), "=r"(v[u].y), "=r"(v[u].z), "=r"(v[u].w)
+                   : "l"(from + (r + 16 * u) * src.row * 16));
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) add(v[u]);
   }
+  for (; r < r1; r += 16) add(ri_ldg16(from + r * src.row * 16));
   __shared__ float red[16][128];
 #pragma unroll
   for (int i = 0; i < 8; ++i) red[rl][piece * 8 + i] = acc[i];
@@ -525,13 +586,14 @@ __global__ void colmean_final_kernel(const float* __restrict__ partial, uint16_t
 }
 
 template <int DT>
-__global__ void __launch_bounds__(256) centre_apply_kernel(const uint4* __restrict__ keys, const uint16_t* __restrict__ mean,
-                                                           uint4* __restrict__ out, int64_t pieces_per_group) {
+__global__ void __launch_bounds__(256) centre_apply_kernel(const uint4* __restrict__ keys, RowPlace src,
+                                                           const uint16_t* __restrict__ mean, uint4* __restrict__ out,
+                                                           int64_t pieces_per_group) {
   const int z = blockIdx.y;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= pieces_per_group) return;
   const int piece = (int)(i & 15);
-  const uint4 v = ri_ldg16(keys + (int64_t)z * pieces_per_group + i);
+  const uint4 v = ri_ldg16(keys + (z * src.group + (i >> 4) * src.row) * 16 + piece);
   const uint4 m = *reinterpret_cast<const uint4*>(mean + z * 128 + piece * 8);
   const uint32_t vw[4] = {v.x, v.y, v.z, v.w}, mw[4] = {m.x, m.y, m.z, m.w};
   uint32_t ow[4];
@@ -564,13 +626,15 @@ struct BucketArgs {
   int32_t* offset;         // [problems, n_cen + 1]
   int n_tok, n_cen, seg_per_group;
   int64_t group_stride;
+  int range;               // tokens per warp
 };
 
-// One CTA per problem.  The tokens are cut into `workers` contiguous ranges; a table [workers][n_cen] first holds
+// The form for what the kernel below does not take (more than about 20000 clusters or 480000 tokens per problem): one CTA
+// per problem, 32-bit counts.  The tokens are cut into `workers` contiguous ranges; a table [workers][n_cen] first holds
 // how many tokens of each range fall into each cluster, then (after the scan of the totals) where each range
 // starts writing inside each cluster, so that `workers` warps can scatter their ranges side by side and the
 // order inside a cluster is still ascending in the token id.
-__global__ void __launch_bounds__(1024) kmeans_bucket_kernel(BucketArgs a, int workers) {
+__global__ void __launch_bounds__(1024) kmeans_bucket_one_cta_kernel(BucketArgs a, int workers) {
   extern __shared__ int32_t bucket_smem[];
   int32_t* cursor = bucket_smem;                 // [n_cen]: counts, then first positions
   int32_t* table = workers == 1 ? bucket_smem : bucket_smem + a.n_cen;   // [workers][n_cen]; one range: the same array
@@ -663,23 +727,183 @@ __global__ void __launch_bounds__(1024) kmeans_bucket_kernel(BucketArgs a, int w
   }
 }
 
+// A cluster of CTAs per problem.  The tokens are cut into contiguous ranges, one per warp of the cluster; a table
+// [warps of the CTA][n_cen] of 16-bit counts first holds how many tokens of each range fall into each cluster, then how
+// many lie in the ranges before it (in this CTA); the CTAs' totals meet through distributed shared memory.  So every warp
+// scatters its own range, and the order inside a cluster is still ascending in the token id.
+// 8 problems of 131004 tokens and 8192 clusters: 350 us with one CTA per problem, 51 now; 128 problems of 8187 tokens and 512
+// clusters: 17 -> 12 us.
+template <int CL>
+__global__ void __launch_bounds__(512) kmeans_bucket_kernel(BucketArgs a) {
+  ri_pdl_trigger();
+  extern __shared__ __align__(16) uint8_t sort_smem[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int workers = (int)blockDim.x / 32;
+  uint32_t* total = reinterpret_cast<uint32_t*>(sort_smem);              // [n_cen] this CTA's tokens per cluster
+  int32_t* base = reinterpret_cast<int32_t*>(total + a.n_cen);             // [n_cen] where this CTA's tokens start
+  uint32_t* table32 = reinterpret_cast<uint32_t*>(base + a.n_cen);         // [workers][n_cen] 16-bit counts
+  __shared__ uint32_t warp_sums[16];
+  const int problem = (int)blockIdx.x / CL, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, T = blockDim.x;
+  const int64_t tok0 = (int64_t)(problem / a.seg_per_group) * a.group_stride + (int64_t)(problem % a.seg_per_group) * a.n_tok;
+  const int32_t* asg = a.assign + tok0;
+  const int t_begin = min(a.n_tok, (rank * workers + warp) * a.range), t_end = min(a.n_tok, t_begin + a.range);
+  for (int i = tid; i < a.n_cen * workers / 2; i += T) table32[i] = 0;     // n_cen is a multiple of 32
+  ri_pdl_wait();
+  __syncthreads();
+  auto clamp_id = [&](int32_t c) { return min(max(c, 0), a.n_cen - 1); };  // never index outside the table
+  constexpr int kAhead = 8;
+  for (int t0 = t_begin; t0 < t_end; t0 += 32 * kAhead) {
+    int32_t cl[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int t = t0 + u * 32 + lane;
+      cl[u] = t < t_end ? clamp_id(asg[t]) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (cl[u] >= 0) atomicAdd(&table32[(warp * a.n_cen + cl[u]) >> 1], (cl[u] & 1) ? 0x10000u : 1u);
+  }
+  __syncthreads();
+  // counts of the ranges before, per cluster pair (packed 16-bit sums: a CTA has fewer than 65536 tokens)
+  for (int i = tid; i < a.n_cen / 2; i += T) {
+    uint32_t run = 0;
+    for (int w = 0; w < workers; ++w) {
+      const uint32_t n = table32[(w * a.n_cen >> 1) + i];
+      table32[(w * a.n_cen >> 1) + i] = run;
+      run += n;
+    }
+    total[2 * i] = run & 0xffffu;
+    total[2 * i + 1] = run >> 16;
+  }
+  cluster.sync();
+  // exclusive scan of the problem's counts over the clusters: a warp takes a contiguous run of them, 32 at a time
+  const int per = ((a.n_cen / 32 + workers - 1) / workers) * 32, c_lo = min(a.n_cen, warp * per), c_hi = min(a.n_cen, c_lo + per);
+  uint32_t running = 0;
+  for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
+    const int c = c0 + lane;
+    uint32_t all = 0, lower = 0;
+#pragma unroll
+    for (int r = 0; r < CL; ++r) {
+      const uint32_t n = CL == 1 ? total[c] : cluster.map_shared_rank(total, r)[c];
+      lower += r < rank ? n : 0u;
+      all += n;
+    }
+    if (rank == 0) a.count[(int64_t)problem * a.n_cen + c] = (int32_t)all;
+    uint32_t inc = all;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t n = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += n;
+    }
+    base[c] = (int32_t)(running + inc - all + lower);      // relative to the warp's first cluster, for now
+    running += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  if (lane == 0) warp_sums[warp] = running;
+  __syncthreads();
+  uint32_t before = 0;
+  for (int w = 0; w < warp; ++w) before += warp_sums[w];
+  for (int c = c_lo + lane; c < c_hi; c += 32) {
+    base[c] += (int32_t)before;
+    if (rank == 0) a.offset[(int64_t)problem * (a.n_cen + 1) + c] = base[c];     // no CTA of lower rank: the cluster's first
+  }
+  if (rank == 0 && warp == workers - 1 && lane == 0) a.offset[(int64_t)problem * (a.n_cen + 1) + a.n_cen] = (int32_t)(before + running);
+  if (CL > 1) cluster_arrive();                   // this CTA's remote reads are over (awaited before it exits)
+  __syncthreads();
+  // stable scatter: 32 tokens of the warp's range at a time, in token order
+  int32_t* ord = a.order + tok0;
+  for (int t0 = t_begin; t0 < t_end; t0 += 32 * kAhead) {
+    int32_t cl[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int t = t0 + u * 32 + lane;
+      cl[u] = t < t_end ? clamp_id(asg[t]) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int t = t0 + u * 32 + lane;
+      // the lane's place behind the tokens of the steps before; lanes that share a cluster with an earlier lane find the
+      // counter moved on and are put in token order one cluster after the other (few: __match_any_sync on 32 mostly
+      // different clusters took most of this kernel's time)
+      const int slot = warp * a.n_cen + max(cl[u], 0), shift = (slot & 1) * 16;
+      const uint32_t cur = (table32[slot >> 1] >> shift) & 0xffffu;
+      __syncwarp();
+      uint32_t old = cur;
+      if (cl[u] >= 0) old = (atomicAdd(&table32[slot >> 1], 1u << shift) >> shift) & 0xffffu;
+      uint32_t rank_in = 0;
+      for (unsigned todo = __ballot_sync(0xffffffffu, old != cur); todo;) {
+        const int c = __shfl_sync(0xffffffffu, cl[u], __ffs(todo) - 1);
+        const unsigned peers = __ballot_sync(0xffffffffu, cl[u] == c);
+        if (cl[u] == c) rank_in = __popc(peers & ((1u << lane) - 1u));
+        todo &= ~peers;
+      }
+      if (cl[u] >= 0) ord[base[cl[u]] + cur + rank_in] = t;
+      __syncwarp();
+    }
+  }
+  if (CL > 1) cluster_wait();
+}
+
+// Launch plan of the bucket pass: CTAs per problem, warps per CTA, tokens per warp.
+struct BucketPlan { int cl, workers; size_t smem; };
+
+BucketPlan bucket_plan(int problems, int n_tok, int n_cen) {
+  BucketPlan p;
+  // as many CTAs per problem as the chip has room for beside the other problems (two CTAs per SM), up to 8
+  p.cl = 8;
+  while (p.cl > 1 && p.cl * problems > 2 * 148) p.cl >>= 1;
+  // 16-bit counts and packed sums: a CTA's tokens stay below 65536
+  while (p.cl < 8 && (n_tok + p.cl - 1) / p.cl > 60000) p.cl <<= 1;
+  p.workers = 16;
+  auto bytes = [&](int w) { return (size_t)n_cen * (8 + 2 * (size_t)w); };
+  while (p.workers > 1 && bytes(p.workers) > 200 * 1024) p.workers >>= 1;
+  p.smem = bytes(p.workers);
+  return p;
+}
+
+template <int CL>
+int launch_bucket(BucketArgs a, const BucketPlan& p, int problems, cudaStream_t s) {
+  a.range = ((a.n_tok + p.cl * p.workers - 1) / (p.cl * p.workers) + 31) & ~31;
+  if (p.smem > 48 * 1024)
+    RI_CUDA_OK(cudaFuncSetAttribute(kmeans_bucket_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(problems * CL);
+  cfg.blockDim = dim3(p.workers * 32);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CL;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  RI_CUDA_OK(cudaLaunchKernelEx(&cfg, kmeans_bucket_kernel<CL>, a));
+  return RI_OK;
+}
+
 // ---- update ---------------------------------------------------------------------------------
 struct UpdateArgs {
-  const uint2* centred;      // [Z, N, 128] centred keys
-  const uint2* raw_keys;     // optional: uncentred keys for the cluster-contiguous copy
-  const uint2* values;       // optional: V rows (value sums + copy)
+  const uint2* rows;         // rows to average: centred keys, or the raw keys with `mean` to be subtracted (LAST)
+  const uint2* values;       // LAST: V rows (value sums + copy)
+  RowPlace src;              // place of a row of `rows` and `values`
   const int32_t* order;
   const int32_t* count;
   const int32_t* offset;
   uint2* centroids;          // [problems, n_cen, 128] in/out (centred)
   uint2* out_centroids;      // optional final: centroid + mean
   const uint16_t* mean;      // optional [Z, 128]
-  uint2* value_sum;          // optional [Z, C, 128]
-  uint16_t* size_dt;         // optional [Z, C]
-  uint2* keys_out;           // optional [Z, N, 128]
+  uint2* value_sum;          // LAST: [Z, C, 128]
+  uint16_t* size_dt;         // LAST: [Z, C]
+  uint8_t* empty;            // LAST, optional: [Z, C] whether the cluster has no members
+  uint2* keys_out;           // LAST, optional: cluster-contiguous copy, group stride `out_group` rows
   uint2* values_out;
+  int64_t out_group;
   int n_tok, n_cen, seg_per_group, normalize;
   int64_t group_stride;
+  int clusters_per_warp, n_clusters;   // n_clusters: over all problems
 };
 
 template <int DT>
@@ -689,101 +913,170 @@ __device__ __forceinline__ void add_row(float (&acc)[4], uint2 v) {
   acc[2] += Elem<DT>::from_bits((uint16_t)(v.y & 0xffffu));
   acc[3] += Elem<DT>::from_bits((uint16_t)(v.y >> 16));
 }
+template <int DT>
+__device__ __forceinline__ uint2 sub_row(uint2 v, uint2 m) {      // round(v - m), channel by channel
+  uint2 o;
+  o.x = Elem<DT>::pack2(Elem<DT>::from_bits((uint16_t)(v.x & 0xffffu)) - Elem<DT>::from_bits((uint16_t)(m.x & 0xffffu)),
+                        Elem<DT>::from_bits((uint16_t)(v.x >> 16)) - Elem<DT>::from_bits((uint16_t)(m.x >> 16)));
+  o.y = Elem<DT>::pack2(Elem<DT>::from_bits((uint16_t)(v.y & 0xffffu)) - Elem<DT>::from_bits((uint16_t)(m.y & 0xffffu)),
+                        Elem<DT>::from_bits((uint16_t)(v.y >> 16)) - Elem<DT>::from_bits((uint16_t)(m.y >> 16)));
+  return o;
+}
 
-// LAST: the pass that also sums the values and writes the cluster-contiguous copy (three rows per member).
-// Cluster sizes are very uneven (median of a few members, a tail of thousands).  With one short-lived CTA per
-// eight clusters most CTAs had next to nothing to do and the kernel was bound by CTA turnover (about 220 CTAs
-// per SM in a row), so the warps are persistent instead: a few CTAs per SM, warp w of the grid takes clusters
-// w, w + W, w + 2W, ... of all problems, which also evens out the large clusters.
+// A warp takes `clusters_per_warp` consecutive clusters of one problem, lane l the channels 4l .. 4l+3.  Their members are
+// one run of the order list, so the rows stream through a ring in shared memory (cp.async, windows of four rows: half a
+// warp copies a row in 16-byte pieces) whatever the clusters' sizes, about 15 members as a rule: three windows are on
+// their way while one is added.  A cluster's rows are added one after the other in list order, so the sums are those of a
+// serial sum (the rows of a window that belong to another cluster add +0, which changes no sum that began at +0).
+// A segmented launch of 8 heads x 128K rows: 155 -> 69 us, bound by issue slots (78 %, 45 instructions a row, a third of them
+// the divisions and the root at a cluster's end) beside 273 MB from DRAM; fetching count, offset, list and rows of one
+// cluster after the other spent its time waiting.
+constexpr int kUpdateThreads = 128;
+constexpr int kWindow = 4;          // rows per step
+constexpr int kWindows = 4;         // steps in the ring
+
 template <int DT, bool LAST>
-__global__ void __launch_bounds__(256) kmeans_update_kernel(UpdateArgs a, int n_problems) {
+__global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArgs a) {
+  ri_pdl_enter();
+  constexpr int kWarps = kUpdateThreads / 32, kRowsBytes = kWindows * kWindow * 256;
+  __shared__ __align__(16) uint8_t ring[kWarps][(LAST ? 2 : 1) * kRowsBytes];
   const int lane = threadIdx.x & 31;
-  // most clusters hold a handful of rows, so the per-cluster index arithmetic counts: 32-bit, and (problem, c)
-  // advance by a fixed step instead of being divided out of the running index (the launcher checks the range)
-  const int n_total = n_problems * a.n_cen;
-  const int n_warps = (int)gridDim.x * 8;
-  const int step_p = n_warps / a.n_cen, step_c = n_warps - step_p * a.n_cen;
-  const int idx0 = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5);
-  int problem = idx0 / a.n_cen, c = idx0 - problem * a.n_cen;
-  for (int idx = idx0; idx < n_total; idx += n_warps, problem += step_p, c += step_c) {
-  if (c >= a.n_cen) { c -= a.n_cen; ++problem; }
-  const int z = (int)((unsigned)problem / (unsigned)a.seg_per_group);
-  const int64_t tok0 = (int64_t)z * a.group_stride + (int64_t)(problem - z * a.seg_per_group) * a.n_tok;
-  const int cnt = a.count[(int64_t)problem * a.n_cen + c];
-  const int off = a.offset[(int64_t)problem * (a.n_cen + 1) + c];
-  const int32_t* ord = a.order + tok0 + off;
-  const int64_t crow = ((int64_t)problem * a.n_cen + c) * 32 + lane;    // uint2 index of this lane's 4 channels
-  if (a.size_dt) a.size_dt[(int64_t)problem * a.n_cen + c] = Elem<DT>::bits((float)cnt);
+  const int job = (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5);
+  const int idx0 = job * a.clusters_per_warp;                 // clusters_per_warp divides n_cen: one problem per warp
+  if (idx0 >= a.n_clusters) return;
+  const int problem = idx0 / a.n_cen, z = problem / a.seg_per_group;
+  int c = idx0 - problem * a.n_cen;
+  const int tok_in_group = (problem - z * a.seg_per_group) * a.n_tok;
+  const int32_t* off = a.offset + (int64_t)problem * (a.n_cen + 1) + c;
+  // ends of this warp's clusters (at most 32), one per lane
+  const int my_end = off[min(lane, a.clusters_per_warp - 1) + 1];
+  const int first = off[0];
+  const int last = __shfl_sync(0xffffffffu, my_end, a.clusters_per_warp - 1);
+  const int32_t* ord = a.order + (int64_t)z * a.group_stride + tok_in_group;
+  const int half = lane >> 4;                                 // copies the first or the second row of a step
+  const int64_t src0 = ((int64_t)z * a.src.group + (int64_t)tok_in_group * a.src.row) * 16 + (lane & 15);   // 16-byte pieces
+  const int64_t row_step = a.src.row * 16;
+  uint2 mean = make_uint2(0u, 0u);
+  if (a.mean) mean = *reinterpret_cast<const uint2*>(a.mean + z * 128 + lane * 4);
 
   float ks[4] = {0, 0, 0, 0}, vs[4] = {0, 0, 0, 0};
-  constexpr int kUnroll = LAST ? 8 : 4;
-  for (int b0 = 0; b0 < cnt; b0 += 32) {
-    // the member list of up to 32 rows in one coalesced load; the rows are then fetched kUnroll at a time
-    const int my_row = b0 + lane < cnt ? ord[b0 + lane] : -1;
-    const int n_here = min(32, cnt - b0);
-    for (int j0 = 0; j0 < n_here; j0 += kUnroll) {
-      int rows[kUnroll];
-      uint2 kv[kUnroll], vv[kUnroll], rk[kUnroll];
+  int done = 0, end = __shfl_sync(0xffffffffu, my_end, 0), start = first;
+  auto finish = [&]() {       // cluster c + done is complete
+    const int cnt = end - start;
+    const int64_t cl = (int64_t)problem * a.n_cen + c + done, crow = cl * 32 + lane;
+    if (LAST) {
+      if (a.size_dt) a.size_dt[cl] = Elem<DT>::bits((float)cnt);
+      if (a.empty) a.empty[cl] = cnt == 0;
+      if (a.value_sum) a.value_sum[crow] = make_uint2(Elem<DT>::pack2(vs[0], vs[1]), Elem<DT>::pack2(vs[2], vs[3]));
+    }
+    uint2 cd;
+    if (cnt > 0) {
+      const float fc = (float)cnt;
+      float x[4];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u) rows[u] = __shfl_sync(0xffffffffu, my_row, (j0 + u) & 31);
+      for (int i = 0; i < 4; ++i) x[i] = ks[i] / fc;
+      if (a.normalize) {
+        float ss = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u)
-        if (j0 + u < n_here) {
-          const int64_t r = (tok0 + rows[u]) * 32 + lane;
-          kv[u] = __ldg(a.centred + r);
-          if (LAST && a.values) vv[u] = __ldg(a.values + r);
-          if (LAST && a.raw_keys) rk[u] = __ldg(a.raw_keys + r);
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        const float nrm = sqrtf(ss);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = x[i] / nrm;
+      }
+      cd = make_uint2(Elem<DT>::pack2(x[0], x[1]), Elem<DT>::pack2(x[2], x[3]));
+      a.centroids[crow] = cd;
+    } else if (LAST && a.out_centroids) {
+      cd = a.centroids[crow];
+    }
+    if (LAST && a.out_centroids) {
+      // stored centroid = round(centroid_dt + mean_dt), both already in the key dtype
+      // (cache_hub/retroinfer_cache.py:429)
+      uint2 o;
+      o.x = Elem<DT>::pack2(Elem<DT>::from_bits((uint16_t)(cd.x & 0xffffu)) + Elem<DT>::from_bits((uint16_t)(mean.x & 0xffffu)),
+                            Elem<DT>::from_bits((uint16_t)(cd.x >> 16)) + Elem<DT>::from_bits((uint16_t)(mean.x >> 16)));
+      o.y = Elem<DT>::pack2(Elem<DT>::from_bits((uint16_t)(cd.y & 0xffffu)) + Elem<DT>::from_bits((uint16_t)(mean.y & 0xffffu)),
+                            Elem<DT>::from_bits((uint16_t)(cd.y >> 16)) + Elem<DT>::from_bits((uint16_t)(mean.y >> 16)));
+      a.out_centroids[crow] = o;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { ks[i] = 0.f; vs[i] = 0.f; }
+    start = end;
+    ++done;
+    end = __shfl_sync(0xffffffffu, my_end, min(done, 31));
+  };
+
+  const int n = last - first;                                 // members of all of this warp's clusters
+  uint8_t* my_ring = ring[threadIdx.x >> 5];
+  const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(my_ring);
+  int ids = lane < n ? ord[first + lane] : 0;                 // 32 list entries; the next 32 below
+  int ids_next = 32 + lane < n ? ord[first + 32 + lane] : 0;
+  int filled = 0;                                             // members asked for so far
+  auto fetch = [&]() {
+    if (filled < n) {
+      const uint32_t dst = ring_s + (filled & (kWindows * kWindow - 1)) * 256 + lane * 16;
+#pragma unroll
+      for (int u = 0; u < kWindow; u += 2) {
+        const int row = __shfl_sync(0xffffffffu, ids, (filled + u + half) & 31);
+        if (filled + u + half < n) {
+          const int64_t at = src0 + row * row_step;
+          cp_async16(dst + u * 256, reinterpret_cast<const uint4*>(a.rows) + at);
+          if (LAST) cp_async16(dst + u * 256 + kRowsBytes, reinterpret_cast<const uint4*>(a.values) + at);
         }
+      }
+      filled += kWindow;
+      if ((filled & 31) == 0) {
+        ids = ids_next;
+        ids_next = filled + 32 + lane < n ? ord[first + filled + 32 + lane] : 0;
+      }
+    }
+    cp_async_commit();
+  };
 #pragma unroll
-      for (int u = 0; u < kUnroll; ++u)
-        if (j0 + u < n_here) {
-          add_row<DT>(ks, kv[u]);           // sequential in list order: bit-identical to a serial sum
-          if (LAST && a.values) add_row<DT>(vs, vv[u]);
-          if (LAST && a.keys_out) {
-            const int64_t o = ((int64_t)z * a.group_stride + off + b0 + j0 + u) * 32 + lane;
-            a.keys_out[o] = rk[u];
-            a.values_out[o] = vv[u];
-          }
+  for (int i = 0; i < kWindows - 1; ++i) fetch();
+#pragma unroll 1
+  for (int r = 0; r < n; r += kWindow) {
+    cp_async_wait<kWindows - 2>();
+    __syncwarp();                                             // the other half's rows; and everyone is done with the slots below
+    fetch();
+    const uint8_t* src = my_ring + (r & (kWindows * kWindow - 1)) * 256 + lane * 8;
+    uint2 kv[kWindow], vv[kWindow];
+#pragma unroll
+    for (int u = 0; u < kWindow; ++u) {
+      kv[u] = *reinterpret_cast<const uint2*>(src + u * 256);
+      if (LAST) {
+        vv[u] = *reinterpret_cast<const uint2*>(src + u * 256 + kRowsBytes);
+        if (a.keys_out && r + u < n) {
+          const int64_t o = ((int64_t)z * a.out_group + first + r + u) * 32 + lane;
+          a.keys_out[o] = kv[u];
+          a.values_out[o] = vv[u];
         }
+        if (a.mean) kv[u] = sub_row<DT>(kv[u], mean);         // the centred key, rounded as the copy the assignment reads
+      }
+    }
+    int lo = 0;                                               // rows of the window behind the last finished cluster
+    for (;;) {
+      const int hi = end - first - r;                         // the current cluster's end, from the window's first row
+      if (lo == 0 && hi >= kWindow) {
+#pragma unroll
+        for (int u = 0; u < kWindow; ++u) {
+          add_row<DT>(ks, kv[u]);
+          if (LAST) add_row<DT>(vs, vv[u]);
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < kWindow; ++u) {
+          const bool in = u >= lo && u < hi;
+          add_row<DT>(ks, in ? kv[u] : make_uint2(0u, 0u));
+          if (LAST) add_row<DT>(vs, in ? vv[u] : make_uint2(0u, 0u));
+        }
+      }
+      if (hi > kWindow || done == a.clusters_per_warp) break;
+      finish();
+      lo = hi;
+      if (done == a.clusters_per_warp) break;
     }
   }
-  if (a.value_sum) {
-    uint2 o;
-    o.x = Elem<DT>::pack2(vs[0], vs[1]);
-    o.y = Elem<DT>::pack2(vs[2], vs[3]);
-    a.value_sum[crow] = o;
-  }
-  float x[4];
-  if (cnt > 0) {
-    const float fc = (float)cnt;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = ks[i] / fc;
-    if (a.normalize) {
-      float ss = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      const float nrm = sqrtf(ss);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = x[i] / nrm;
-    }
-    uint2 o;
-    o.x = Elem<DT>::pack2(x[0], x[1]);
-    o.y = Elem<DT>::pack2(x[2], x[3]);
-    a.centroids[crow] = o;
-  }
-  if (a.out_centroids) {
-    // stored centroid = round(centroid_dt + mean_dt), both already in the key dtype
-    // (cache_hub/retroinfer_cache.py:429)
-    const uint2 cd = a.centroids[crow];
-    const uint2 m = *reinterpret_cast<const uint2*>(a.mean + z * 128 + lane * 4);
-    uint2 o;
-    o.x = Elem<DT>::pack2(Elem<DT>::from_bits((uint16_t)(cd.x & 0xffffu)) + Elem<DT>::from_bits((uint16_t)(m.x & 0xffffu)),
-                          Elem<DT>::from_bits((uint16_t)(cd.x >> 16)) + Elem<DT>::from_bits((uint16_t)(m.x >> 16)));
-    o.y = Elem<DT>::pack2(Elem<DT>::from_bits((uint16_t)(cd.y & 0xffffu)) + Elem<DT>::from_bits((uint16_t)(m.y & 0xffffu)),
-                          Elem<DT>::from_bits((uint16_t)(cd.y >> 16)) + Elem<DT>::from_bits((uint16_t)(m.y >> 16)));
-    a.out_centroids[crow] = o;
-  }
-  }   // next cluster of this warp
+  while (done < a.clusters_per_warp) finish();
 }
 
 // ---- host side --------------------------------------------------------------------------------
@@ -830,11 +1123,14 @@ int validate_fit(const ri_kmeans* p) {
   return RI_OK;
 }
 
+// Where the caller's rows lie: places of a K or V row, of a row of the cluster-contiguous copy, optional mask of empty clusters.
+struct Place { RowPlace src; int64_t out_group; uint8_t* empty; };
+
 template <int DT>
-int run_fit(const ri_kmeans* p, const FitLayout& L, const void* centred, cudaStream_t s) {
+int run_fit(const ri_kmeans* p, const FitLayout& L, const Place& pl, const void* centred, cudaStream_t s) {
   uint8_t* sc = static_cast<uint8_t*>(p->d_scratch);
   const int Z = p->groups, N = p->n_tokens, C = p->n_centroids, S = p->n_segments;
-  int* err = reinterpret_cast<int*>(sc + L.error);
+  int* err = p->d_error ? p->d_error : reinterpret_cast<int*>(sc + L.error);
   void* cent = sc + L.cent_work;
   int32_t* assign = p->d_assign ? p->d_assign : reinterpret_cast<int32_t*>(sc + L.assign);
   int32_t* order = p->d_order ? p->d_order : reinterpret_cast<int32_t*>(sc + L.order);
@@ -857,6 +1153,8 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const void* centred, cudaStr
   RI_CUDA_OK(cudaFuncSetAttribute(kmeans_assign_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem));
   RI_CUDA_OK(cudaFuncSetAttribute(kmeans_assign_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem));
 
+  int sms = 0;
+  if ((rc = ri_sm_count(&sms)) != RI_OK) return rc;
   for (int it = 0; it < p->n_iters; ++it) {
     const bool last = it == p->n_iters - 1;
     const int seg = last ? 1 : S;
@@ -868,22 +1166,18 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const void* centred, cudaStr
     aa.group_stride = N;
     aa.idesc = idesc_f16(DT, kTileM, kTileN);
     {
-      // blocks per CTA: enough CTAs for about six waves over the SMs, at most 16 blocks each (config 2: 16 blocks in
-      // both the segmented and the last iteration, an even split of 32 and 512 blocks; 9 blocks per CTA with a dozen
-      // waves left one CTA in four with 5 blocks and cost 2 % of the build)
+      // persistent CTAs, one per SM, an even share of the units each
       WideArgs wa;
       wa.a = aa;
-      const int n_blocks = (n_tok + 2 * kTileM - 1) / (2 * kTileM);
-      int per = (int)(((int64_t)n_blocks * problems) / (148 * 6));
-      per = per < 1 ? 1 : (per > 16 ? 16 : per);
-      wa.blocks_per_cta = per;
-      dim3 wgrid((n_blocks + per - 1) / per, problems);
-      if (n_cen <= 4 * kTileN) {        // the problem's centroids fit shared memory: they stay there
-        kmeans_assign_resident_kernel<<<wgrid, kWideThreads, kResSmem, s>>>(map_keys, map_cent, wa);
-        RI_LAUNCH_OK("kmeans_assign_resident_kernel");
+      const bool resident = n_cen <= 4 * kTileN;        // the problem's centroids fit shared memory: they stay there
+      wa.per_problem = resident ? (n_tok + kTileM - 1) / kTileM : (n_tok + 2 * kTileM - 1) / (2 * kTileM);
+      RI_REQUIRE((int64_t)wa.per_problem * problems < (1ll << 30), "too many token tiles in one launch");
+      wa.n_units = wa.per_problem * problems;
+      const dim3 wgrid((unsigned)(wa.n_units < sms ? wa.n_units : sms));
+      if (resident) {
+        RI_CUDA_OK(ri_launch_pdl_id(10, kmeans_assign_resident_kernel, wgrid, dim3(kWideThreads), kResSmem, s, map_keys, map_cent, wa));
       } else {
-        kmeans_assign_wide_kernel<<<wgrid, kWideThreads, kWideSmem, s>>>(map_keys, map_cent, wa);
-        RI_LAUNCH_OK("kmeans_assign_wide_kernel");
+        RI_CUDA_OK(ri_launch_pdl_id(10, kmeans_assign_wide_kernel, wgrid, dim3(kWideThreads), kWideSmem, s, map_keys, map_cent, wa));
       }
     }
 
@@ -892,18 +1186,26 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const void* centred, cudaStr
     ba.count = last && p->d_cluster_count ? p->d_cluster_count : count_work;
     ba.offset = last && p->d_cluster_offset ? p->d_cluster_offset : offset_work;
     ba.n_tok = n_tok; ba.n_cen = n_cen; ba.seg_per_group = seg; ba.group_stride = N;
-    // as many token ranges (scattering warps) as fit the shared memory: a table of [ranges + 1][n_cen] words
-    int workers = 32;
-    while (workers > 1 && (size_t)(workers + 1) * n_cen * 4 > 200 * 1024) workers >>= 1;
-    const size_t bsmem = (size_t)(workers == 1 ? 1 : workers + 1) * n_cen * 4;
-    RI_REQUIRE(bsmem <= 227 * 1024, "n_centroids per problem = %d too large for the bucket pass", n_cen);
-    if (bsmem > 48 * 1024)
-      RI_CUDA_OK(cudaFuncSetAttribute(kmeans_bucket_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
-    kmeans_bucket_kernel<<<problems, 1024, bsmem, s>>>(ba, workers);
-    RI_LAUNCH_OK("kmeans_bucket_kernel");
+    const BucketPlan bp = bucket_plan(problems, n_tok, n_cen);
+    if ((n_tok + bp.cl - 1) / bp.cl <= 60000 && bp.smem <= 200 * 1024) {
+      rc = bp.cl == 8 ? launch_bucket<8>(ba, bp, problems, s) : bp.cl == 4 ? launch_bucket<4>(ba, bp, problems, s)
+         : bp.cl == 2 ? launch_bucket<2>(ba, bp, problems, s) : launch_bucket<1>(ba, bp, problems, s);
+      if (rc != RI_OK) return rc;
+    } else {
+      // as many token ranges (scattering warps) as fit the shared memory: a table of [ranges + 1][n_cen] words
+      int workers = 32;
+      while (workers > 1 && (size_t)(workers + 1) * n_cen * 4 > 200 * 1024) workers >>= 1;
+      const size_t bsmem = (size_t)(workers == 1 ? 1 : workers + 1) * n_cen * 4;
+      RI_REQUIRE(bsmem <= 227 * 1024, "n_centroids per problem = %d too large for the bucket pass", n_cen);
+      if (bsmem > 48 * 1024)
+        RI_CUDA_OK(cudaFuncSetAttribute(kmeans_bucket_one_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsmem));
+      kmeans_bucket_one_cta_kernel<<<problems, 1024, bsmem, s>>>(ba, workers);
+      RI_LAUNCH_OK("kmeans_bucket_one_cta_kernel");
+    }
 
     UpdateArgs ua = {};
-    ua.centred = static_cast<const uint2*>(centred);
+    ua.rows = static_cast<const uint2*>(centred);
+    ua.src = {N, 1};
     ua.order = order; ua.count = ba.count; ua.offset = ba.offset;
     ua.centroids = static_cast<uint2*>(cent);
     ua.n_tok = n_tok; ua.n_cen = n_cen; ua.seg_per_group = seg; ua.normalize = last ? 0 : 1; ua.group_stride = N;
@@ -911,42 +1213,35 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const void* centred, cudaStr
       ua.values = static_cast<const uint2*>(p->d_values);
       ua.value_sum = static_cast<uint2*>(p->d_value_sum);
       ua.size_dt = static_cast<uint16_t*>(p->d_cluster_size);
-      if (p->d_keys_out) {
-        ua.raw_keys = static_cast<const uint2*>(p->d_keys);
-        ua.keys_out = static_cast<uint2*>(p->d_keys_out);
-        ua.values_out = static_cast<uint2*>(p->d_values_out);
-      }
+      ua.empty = pl.empty;
+      ua.src = pl.src;
+      ua.rows = static_cast<const uint2*>(p->d_keys);         // raw keys: centred on the fly, copied as they are
+      ua.keys_out = static_cast<uint2*>(p->d_keys_out);
+      ua.values_out = static_cast<uint2*>(p->d_values_out);
+      ua.out_group = pl.out_group;
       if (p->center) {
         ua.mean = reinterpret_cast<const uint16_t*>(sc + L.mean);
         ua.out_centroids = static_cast<uint2*>(p->d_centroids);
       }
     }
-    // persistent warps: as many CTAs as are resident at once
-    static int resident[2] = {0, 0};
-    const int form = ua.values ? 1 : 0;
-    if (resident[form] == 0) {
-      int per_sm = 0, sms = 0, dev = 0;
-      RI_CUDA_OK(cudaGetDevice(&dev));
-      RI_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      if (form) RI_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kmeans_update_kernel<DT, true>, 256, 0));
-      else RI_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kmeans_update_kernel<DT, false>, 256, 0));
-      resident[form] = (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 148);
-    }
     RI_REQUIRE((int64_t)n_cen * problems < (1ll << 30), "too many clusters in one launch (%d x %d)", n_cen, problems);
-    const int64_t ctas_needed = ((int64_t)n_cen * problems + 7) / 8;
-    const int ugrid = (int)(ctas_needed < resident[form] ? ctas_needed : resident[form]);
-    if (form) kmeans_update_kernel<DT, true><<<ugrid, 256, 0, s>>>(ua, problems);
-    else kmeans_update_kernel<DT, false><<<ugrid, 256, 0, s>>>(ua, problems);
-    RI_LAUNCH_OK("kmeans_update_kernel");
+    ua.n_clusters = n_cen * problems;
+    // clusters per warp: a longer run of rows hides more latency, but enough warps for a few rounds of the chip
+    int cpw = 8;
+    while (cpw > 1 && ua.n_clusters / cpw < 148 * 96) cpw >>= 1;
+    ua.clusters_per_warp = cpw;
+    constexpr int per_cta = kUpdateThreads / 32;
+    const dim3 ugrid((ua.n_clusters / cpw + per_cta - 1) / per_cta);
+    RI_CUDA_OK(last ? ri_launch_pdl_id(9, kmeans_update_kernel<DT, true>, ugrid, dim3(kUpdateThreads), 0, s, ua)
+                    : ri_launch_pdl_id(9, kmeans_update_kernel<DT, false>, ugrid, dim3(kUpdateThreads), 0, s, ua));
   }
   if (!p->center)
     RI_CUDA_OK(cudaMemcpyAsync(p->d_centroids, cent, (size_t)Z * C * 256, cudaMemcpyDeviceToDevice, s));
-  if (p->d_error) RI_CUDA_OK(cudaMemcpyAsync(p->d_error, err, 4, cudaMemcpyDeviceToDevice, s));
   return RI_OK;
 }
 
 template <int DT>
-int run_build(const ri_kmeans* p, cudaStream_t s) {
+int run_build(const ri_kmeans* p, const Place& pl, cudaStream_t s) {
   const FitLayout L = fit_layout(p, p->center != 0);
   uint8_t* sc = static_cast<uint8_t*>(p->d_scratch);
   const void* centred = p->d_keys;
@@ -954,18 +1249,18 @@ int run_build(const ri_kmeans* p, cudaStream_t s) {
     const int Z = p->groups, N = p->n_tokens;
     float* partial = reinterpret_cast<float*>(sc + L.partial);
     uint16_t* mean = reinterpret_cast<uint16_t*>(sc + L.mean);
-    colsum_partial_kernel<DT><<<dim3(L.chunks, Z), 256, 0, s>>>(static_cast<const uint4*>(p->d_keys), partial, N, L.chunks);
+    colsum_partial_kernel<DT><<<dim3(L.chunks, Z), 256, 0, s>>>(static_cast<const uint4*>(p->d_keys), pl.src, partial, N, L.chunks);
     RI_LAUNCH_OK("colsum_partial_kernel");
     colmean_final_kernel<DT><<<Z, 128, 0, s>>>(partial, mean, N, L.chunks);
     RI_LAUNCH_OK("colmean_final_kernel");
     const int64_t pieces = (int64_t)N * 16;
     centre_apply_kernel<DT><<<dim3((unsigned)((pieces + 255) / 256), Z), 256, 0, s>>>(
-        static_cast<const uint4*>(p->d_keys), mean, reinterpret_cast<uint4*>(sc + L.centred), pieces);
+        static_cast<const uint4*>(p->d_keys), pl.src, mean, reinterpret_cast<uint4*>(sc + L.centred), pieces);
     RI_LAUNCH_OK("centre_apply_kernel");
     centred = sc + L.centred;
     if (p->d_mean_key) RI_CUDA_OK(cudaMemcpyAsync(p->d_mean_key, mean, (size_t)Z * 256, cudaMemcpyDeviceToDevice, s));
   }
-  return run_fit<DT>(p, L, centred, s);
+  return run_fit<DT>(p, L, pl, centred, s);
 }
 
 }  // namespace
@@ -975,8 +1270,10 @@ extern "C" int64_t ri_kmeans_scratch_bytes(const ri_kmeans* p) {
   return fit_layout(p, p->center != 0).total;
 }
 
-extern "C" int ri_kmeans_build(const ri_kmeans* p, void* stream) {
-  int rc = validate_fit(p);
+namespace {
+
+int validate_build(const ri_kmeans* p) {
+  const int rc = validate_fit(p);
   if (rc != RI_OK) return rc;
   RI_REQUIRE(p->d_keys && p->d_values && p->d_centroids && p->d_value_sum && p->d_cluster_size && p->d_scratch,
              "ri_kmeans: a required pointer is null");
@@ -984,6 +1281,57 @@ extern "C" int ri_kmeans_build(const ri_kmeans* p, void* stream) {
   RI_REQUIRE(((uintptr_t)p->d_keys | (uintptr_t)p->d_values | (uintptr_t)p->d_centroids | (uintptr_t)p->d_value_sum |
               (uintptr_t)p->d_scratch | (uintptr_t)p->d_keys_out | (uintptr_t)p->d_values_out) % 16 == 0,
              "tensor pointers must be 16-byte aligned");
+  return RI_OK;
+}
+
+int build(const ri_kmeans* p, const Place& pl, cudaStream_t s) {
+  return p->dtype == RI_BF16 ? run_build<RI_BF16>(p, pl, s) : run_build<RI_F16>(p, pl, s);
+}
+
+// Sink and recent rows of every head into the steady zone: rows [0, n_sink) and [n_tokens_total - n_recent, n_tokens_total)
+// of the prompt, one 16-byte piece of K and of V per thread.
+__global__ void __launch_bounds__(256) steady_fill_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, RowPlace src,
+                                                          uint4* __restrict__ sk, uint4* __restrict__ sv, int n_sink,
+                                                          int n_recent, int64_t recent_row, int64_t stride) {
+  const int i = blockIdx.x * 256 + threadIdx.x, row = i >> 4, piece = i & 15, z = blockIdx.y;
+  if (row >= n_sink + n_recent) return;
+  const int64_t r = row < n_sink ? row : recent_row + row - n_sink;
+  const int64_t from = (z * src.group + r * src.row) * 16 + piece, to = (z * stride + row) * 16 + piece;
+  sk[to] = ri_ldg16(k + from);
+  sv[to] = ri_ldg16(v + from);
+}
+
+}  // namespace
+
+extern "C" int ri_kmeans_build(const ri_kmeans* p, void* stream) {
+  const int rc = validate_build(p);
+  if (rc != RI_OK) return rc;
+  const Place pl = {{p->n_tokens, 1}, p->n_tokens, nullptr};
+  return build(p, pl, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ri_kmeans_build_prompt(const ri_kmeans* p, const ri_kmeans_prompt* q, void* stream) {
+  int rc = validate_build(p);
+  if (rc != RI_OK) return rc;
+  RI_REQUIRE(q != nullptr, "ri_kmeans_prompt is null");
+  RI_REQUIRE(p->center == 1, "ri_kmeans_build_prompt: center must be 1");
+  RI_REQUIRE(q->n_sink >= 0 && q->n_recent >= 0 && q->out_group_rows >= p->n_tokens, "ri_kmeans_prompt: bad sizes");
+  RI_REQUIRE((q->n_sink + q->n_recent == 0) || (q->d_steady_keys && q->d_steady_values && q->steady_group_rows >= q->n_sink + q->n_recent),
+             "ri_kmeans_prompt: bad steady zone");
+  RI_REQUIRE(((uintptr_t)q->d_steady_keys | (uintptr_t)q->d_steady_values) % 16 == 0, "tensor pointers must be 16-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return p->dtype == RI_BF16 ? run_build<RI_BF16>(p, s) : run_build<RI_F16>(p, s);
+  // token-major prompt [tokens, Z, 128]: the clustered rows lie behind the sink rows
+  const RowPlace src = {1, p->groups};
+  if (q->n_sink + q->n_recent > 0) {
+    steady_fill_kernel<<<dim3(((q->n_sink + q->n_recent) * 16 + 255) / 256, p->groups), 256, 0, s>>>(
+        static_cast<const uint4*>(p->d_keys), static_cast<const uint4*>(p->d_values), src, static_cast<uint4*>(q->d_steady_keys),
+        static_cast<uint4*>(q->d_steady_values), q->n_sink, q->n_recent, (int64_t)q->n_sink + p->n_tokens, q->steady_group_rows);
+    RI_LAUNCH_OK("steady_fill_kernel");
+  }
+  ri_kmeans c = *p;
+  const int64_t skip = (int64_t)q->n_sink * p->groups * 256;
+  c.d_keys = static_cast<const uint8_t*>(p->d_keys) + skip;
+  c.d_values = static_cast<const uint8_t*>(p->d_values) + skip;
+  const Place pl = {src, q->out_group_rows, q->d_empty};
+  return build(&c, pl, s);
 }

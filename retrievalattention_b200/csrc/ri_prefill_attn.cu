@@ -453,19 +453,6 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
 }
 
-int sm_count(int* out) {
-  static int cached[64] = {0};
-  int dev = 0;
-  RI_CUDA_OK(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || cached[dev] == 0) {
-    RI_CUDA_OK(cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev));
-    if (dev >= 0 && dev < 64) cached[dev] = *out;
-    return RI_OK;
-  }
-  *out = cached[dev];
-  return RI_OK;
-}
-
 template <int DT>
 int launch(const void* q, const void* k, const void* v, void* out, int32_t* error, int B, int S, int Hq, int Hk, int causal,
            cudaStream_t s) {
@@ -480,7 +467,7 @@ int launch(const void* q, const void* k, const void* v, void* out, int32_t* erro
   a.idesc_qk = idesc_f16(DT, kTile, kTile);
   a.idesc_pv = a.idesc_qk | (1u << 16);      // B = V is MN-major (channels contiguous)
   int sms = 0;
-  if ((rc = sm_count(&sms)) != RI_OK) return rc;
+  if ((rc = ri_sm_count(&sms)) != RI_OK) return rc;
   const int tiles = (S + kTile - 1) / kTile;
   // Pairs of query tiles share K and V and are 15 % faster where there are enough of them to fill the chip; below one
   // pair per SM a single query tile per CTA, its key/value tiles shared out to both groups, uses more SMs and halves the

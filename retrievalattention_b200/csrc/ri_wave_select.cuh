@@ -98,15 +98,6 @@ __device__ __forceinline__ T block_scan(T v, T* warp_sums, T& total) {
   return base + inc - v;
 }
 
-__device__ __forceinline__ void cluster_arrive() {
-  __syncwarp();   // .aligned: the whole warp must execute the instruction together
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  __syncwarp();
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // Two histograms of 256 bins (bin 255 = largest keys), each given as the cluster-wide sum (ga, gb)
 // and this CTA's own counts (la, lb); counts fit 16 bits.  For histogram a find the bin where the
 // count from the top first reaches ka (>= 1), likewise b/kb, with ONE packed scan; a thread looks

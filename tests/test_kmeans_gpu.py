@@ -183,3 +183,48 @@ def test_rejects_bad_shapes():
     p.groups, p.n_tokens, p.n_centroids, p.n_segments, p.n_iters = 1, 100, 48, 1, 3
     assert _lib.lib.ri_kmeans_scratch_bytes(C.byref(p)) == -1
     assert b"multiple of 32" in _lib.lib.ri_last_error()
+
+
+# sizes where the sort, the update and the assignment change form: one problem per 8, 4, 2, 1 CTAs of the sort, more tokens
+# than its 16-bit counts take (the one-CTA form), one partial centroid tile, 512 centroids (resident) and 544 (streamed),
+# a prompt whose clustered rows are no multiple of anything.  Everything below is exact: the list is a stable sort of the
+# assignment, and the prompt form is the array form on the same rows.
+@pytest.mark.parametrize("heads,n,c,seg,dtype", [
+    (1, 333, 32, 1, torch.bfloat16), (3, 5003, 512, 1, torch.bfloat16), (2, 9001, 544, 1, torch.float16),
+    (8, 16411, 1024, 16, torch.bfloat16), (8, 20000, 1024, 8, torch.bfloat16), (5, 20011, 1280, 40, torch.float16),
+    (1, 500009, 96, 1, torch.bfloat16),
+])
+def test_lists_and_prompt_form(heads, n, c, seg, dtype):
+    from retrievalattention_b200.cache_hub.kmeans import build_index, build_prompt_index
+
+    sink, recent, z = 4, 64, heads
+    g = torch.Generator(device="cuda").manual_seed(n)
+    k, v = (torch.randn((sink + n + recent, z, 128), generator=g, device="cuda").to(dtype) for _ in range(2))
+    mid_k, mid_v = (t[sink:sink + n].transpose(0, 1).contiguous() for t in (k, v))
+    r = build_index(mid_k, mid_v, c, seg, 3, want_lists=True)
+    assert int(r["error"]) == 0
+    count = torch.stack([torch.bincount(a, minlength=c) for a in r["assign"].long()])
+    assert torch.equal(r["cluster_count"].long(), count)
+    assert torch.equal(r["cluster_offset"][:, 1:].long(), count.cumsum(1)) and int(r["cluster_offset"][:, 0].abs().max()) == 0
+    assert torch.equal(r["order"].long(), torch.sort(r["assign"].long(), dim=1, stable=True)[1])
+    pick = r["order"].long()[:, :, None].expand(-1, -1, 128)
+    assert torch.equal(r["keys"], torch.gather(mid_k, 1, pick)) and torch.equal(r["values"], torch.gather(mid_v, 1, pick))
+    owner = torch.gather(r["assign"].long(), 1, r["order"].long())[:, :, None].expand(-1, -1, 128)
+    total = torch.zeros((z, c, 128), dtype=torch.float64, device="cuda").scatter_add_(1, owner, r["values"].double())
+    bound = torch.zeros_like(total).scatter_add_(1, owner, r["values"].double().abs())
+    # one rounding to 16 bits of a serial fp32 sum: half an ulp of the result plus n_c * 2^-24 of the summed magnitudes
+    ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert bool(((r["value_sum"].double() - total).abs() <= ulp * total.abs() + count.max() * 2.0 ** -24 * bound + 1e-12).all())
+    mk = lambda *s, dt=dtype: torch.full(s, 7, dtype=dt, device="cuda")        # noqa: E731
+    rows, steady = n + 9, sink + recent + 5
+    out = dict(centroids=mk(z, c, 128), value_sum=mk(z, c, 128), cluster_size=mk(z, c), cluster_count=mk(z, c, dt=torch.int32),
+               cluster_offset=mk(z, c + 1, dt=torch.int32), empty=torch.zeros((z, c), dtype=torch.bool, device="cuda"),
+               keys=mk(z, rows, 128), values=mk(z, rows, 128), steady_keys=mk(z, steady, 128), steady_values=mk(z, steady, 128))
+    assert int(build_prompt_index(k, v, seg, sink, recent, out, 3)) == 0
+    for name in ("centroids", "value_sum", "cluster_size", "cluster_count", "cluster_offset"):
+        assert torch.equal(out[name], r[name]), name
+    assert torch.equal(out["empty"], r["cluster_count"] == 0)
+    for name, raw in (("keys", k), ("values", v)):
+        assert torch.equal(out[name][:, :n], r[name]) and bool((out[name][:, n:] == 7).all())
+        ends = torch.cat((raw[:sink], raw[sink + n:]), 0).transpose(0, 1)
+        assert torch.equal(out["steady_" + name][:, :sink + recent], ends) and bool((out["steady_" + name][:, sink + recent:] == 7).all())
