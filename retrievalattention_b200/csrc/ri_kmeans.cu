@@ -134,24 +134,16 @@ struct RunningMax {
     }
   }
   __device__ __forceinline__ int index() const {
-    if (!(best > -INFINITY)) return 0;
-    // v - best is exactly 0 for the maxima and negative elsewhere, so fma(v - best, 2^120, -i) is -i for them and far below
-    // -32 for the others (differences under 2^-115 do not occur between scores of ordinary magnitude); the maximum of
-    // those is minus the first index.
-    float w[32];
+    // once per token: plain comparisons, right for infinite and for very small scores too
+    int first = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
+    for (int i = 15; i >= 0; --i) {
       float lo, hi;
       asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(kept[i]));
-      w[2 * i] = fmaf(lo - best, 0x1p120f, -(float)(2 * i));
-      w[2 * i + 1] = fmaf(hi - best, 0x1p120f, -(float)(2 * i + 1));
+      if (hi == best) first = 2 * i + 1;
+      if (lo == best) first = 2 * i;
     }
-    float t11[11];
-#pragma unroll
-    for (int i = 0; i < 10; ++i) t11[i] = max3(w[3 * i], w[3 * i + 1], w[3 * i + 2]);
-    t11[10] = fmaxf(w[30], w[31]);
-    const float b0 = max3(t11[0], t11[1], t11[2]), b1 = max3(t11[3], t11[4], t11[5]), b2 = max3(t11[6], t11[7], t11[8]);
-    return base + (int)(-max3(max3(b0, b1, b2), t11[9], t11[10]));
+    return best > -INFINITY ? base + first : 0;
   }
   // one finished accumulator tile (128 columns) of this warp's TMEM lanes; 32 columns are on their way while others are reduced
   template <bool FULL>

@@ -228,3 +228,22 @@ def test_lists_and_prompt_form(heads, n, c, seg, dtype):
         assert torch.equal(out[name][:, :n], r[name]) and bool((out[name][:, n:] == 7).all())
         ends = torch.cat((raw[:sink], raw[sink + n:]), 0).transpose(0, 1)
         assert torch.equal(out["steady_" + name][:, :sink + recent], ends) and bool((out["steady_" + name][:, sink + recent:] == 7).all())
+
+
+def test_infinite_scores_keep_every_token():
+    """fp16 keys whose centred form overflows give scores of +inf and -inf beside one another: every token still lands in
+    exactly one cluster."""
+    from retrievalattention_b200.cache_hub.kmeans import build_index
+
+    n = 1024
+    keys = torch.randn((1, n, 128), generator=torch.Generator().manual_seed(3)).half()
+    keys[0, ::2, 0], keys[0, 1::2, 0] = -60000.0, -20000.0
+    keys[0, 7::256, 0] = 65504.0
+    values = torch.zeros_like(keys)
+    values[0, :, 0], values[0, :, 1] = torch.arange(n) % 32, torch.arange(n) // 32
+    for n_cen in (64, 1024):         # centroids resident in shared memory, and streamed
+        r = build_index(keys.cuda(), values.cuda(), n_cen, 1)
+        torch.cuda.synchronize()
+        assert int(r["error"].item()) == 0 and int(r["cluster_count"].sum()) == n
+        got = r["values"][0].float().cpu()
+        assert (got[:, 0] + 32 * got[:, 1]).sort().values.tolist() == list(range(n))
