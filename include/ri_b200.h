@@ -314,6 +314,19 @@ int ri_weighted_flash_decoding(const void* d_q, const void* d_k, const void* d_v
                                void* d_out, float* d_lse_out, int32_t groups, int32_t group_size, int64_t rows_stride,
                                int32_t dtype, void* stream);
 
+/* Decoding with full attention over a dense cache [batch, kv_heads, rows_stride, 128] (cache_hub/flash_attn_cache.py:133-151,
+ * attn_hub/flash_attn.py:17-30).  ri_dense_append stores d_k/d_v [batch, kv_heads, 128] at row d_valid_length[b] of every
+ * head of request b (nothing where that row lies outside the cache).  ri_dense_decode attends rows
+ * [0, d_valid_length[b] + extra) (at most rows_stride) with d_q [batch, kv_heads, group_size, 128]; d_scratch: that many
+ * bytes of 16-byte aligned device memory, for this call alone, with any contents; *d_error stays as it is unless a
+ * device-side wait gave up. */
+int ri_dense_append(const void* d_k, const void* d_v, void* d_keys, void* d_values, const int32_t* d_valid_length,
+                    int32_t batch, int32_t kv_heads, int64_t rows_stride, void* stream);
+int64_t ri_dense_decode_scratch_bytes(int32_t batch, int32_t kv_heads, int32_t group_size);
+int ri_dense_decode(const void* d_q, const void* d_k, const void* d_v, const int32_t* d_valid_length, int32_t extra,
+                    void* d_out, void* d_scratch, int32_t* d_error, int32_t batch, int32_t kv_heads, int32_t group_size,
+                    int64_t rows_stride, int32_t dtype, void* stream);
+
 /* gather_copy.cu:25-96 — rows data_offsets[g, copy_start : copy_start+copy_num] of keys, values and
  * the per-row 16-bit metadata go to the first copy_num rows of the buffers. */
 int ri_gather_copy_vectors(const void* key_data, void* key_buffer, const void* value_data, void* value_buffer,

@@ -130,6 +130,13 @@ def _load() -> C.CDLL:
     lib.ri_batch_gemm_softmax.argtypes = [C.c_void_p] * 6 + [C.c_int32] * 4 + [C.c_float, C.c_float, C.c_int32, C.c_void_p]
     lib.ri_weighted_flash_decoding.restype = C.c_int
     lib.ri_weighted_flash_decoding.argtypes = [C.c_void_p] * 9 + [C.c_int32, C.c_int32, C.c_int64, C.c_int32, C.c_void_p]
+    lib.ri_dense_append.restype = C.c_int
+    lib.ri_dense_append.argtypes = [C.c_void_p] * 5 + [C.c_int32, C.c_int32, C.c_int64, C.c_void_p]
+    lib.ri_dense_decode_scratch_bytes.restype = C.c_int64
+    lib.ri_dense_decode_scratch_bytes.argtypes = [C.c_int32] * 3
+    lib.ri_dense_decode.restype = C.c_int
+    lib.ri_dense_decode.argtypes = ([C.c_void_p] * 4 + [C.c_int32] + [C.c_void_p] * 3 + [C.c_int32] * 3 +
+                                    [C.c_int64, C.c_int32, C.c_void_p])
     lib.ri_gather_copy_vectors.restype = C.c_int
     lib.ri_gather_copy_vectors.argtypes = [C.c_void_p] * 7 + [C.c_int32] * 6 + [C.c_void_p]
     lib.ri_gather_copy_and_concat.restype = C.c_int

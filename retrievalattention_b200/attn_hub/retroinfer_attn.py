@@ -5,7 +5,7 @@ import torch
 
 from .. import _lib
 
-# Status words of the prefill kernels, one per device: 0, or where a device-side wait gave up.  A word stays set until
+# Status words of the prefill and dense decode kernels, one per device: 0, or where a device-side wait gave up.  A word stays set until
 # ``check_prefill_errors`` reports it; every CHECK_EVERY calls a copy of it is sent to the host and looked at when it has
 # arrived, so that a failure surfaces without a call ever waiting for the GPU.
 CHECK_EVERY = 64
@@ -23,8 +23,9 @@ class _StatusWord:
 
     def tick(self):
         self.calls += 1
-        if self.host is not None:
-            copy, arrived = self.host
+        pending = self.host                                  # read once: another thread's call may clear it
+        if pending is not None:
+            copy, arrived = pending
             if arrived.query():
                 self.host = None
                 if int(copy):
@@ -85,7 +86,7 @@ def check_prefill_errors() -> None:
             torch.cuda.synchronize(status.word.device)
         status.calls, status.host = 0, None
     if bad:
-        raise RuntimeError(f"ri_prefill_attn gave up on a device-side wait (codes {sorted(bad)})")
+        raise RuntimeError(f"ri_prefill_attn or ri_dense_decode gave up on a device-side wait (codes {sorted(bad)})")
 
 
 def retroinfer_decode_attn(query_states, key_states, value_states, layer_idx, retroinfer_cache, query_states_next=None):

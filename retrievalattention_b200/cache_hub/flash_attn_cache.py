@@ -12,6 +12,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from .. import _lib
 from .cache import KV_Cache
 
 
@@ -24,6 +25,7 @@ class flash_attn_cache(KV_Cache):
         if head_dim != 128:
             raise ValueError("the decode kernel is built for head_dim 128")
         self.valid_start = valid_start
+        self._longest = None                # rows of the longest request, counted on the host from the first prefill call on
         self.valid_length = None            # [batch] int32 on the first layer's device, set by the first prefill call
         self.allocated = True
         mk = lambda ldx: torch.zeros((batch_size, self.kv_head, max_length, head_dim), dtype=dtype,   # noqa: E731
@@ -43,6 +45,7 @@ class flash_attn_cache(KV_Cache):
         assert seq_len <= self.max_length, f"Prefilling sequence length {seq_len} exceeds max length {self.max_length}."
         if self.valid_length is None:
             vs = np.asarray(self.valid_start)
+            self._longest = int(seq_len - vs.min())
             self.valid_length = torch.from_numpy(seq_len - vs).to(torch.int32).to(self.layer_mapping[str(0)])
         vs = int(self.valid_start[start_bdx])
         n = seq_len - vs
@@ -56,12 +59,34 @@ class flash_attn_cache(KV_Cache):
         """The reference waits for its side-stream copy (:129-130); the copy above is in stream order."""
         return None
 
+    def _one_launch(self, keys, key_states, value_states) -> bool:
+        """Whether the rows can be appended by one kernel for both tensors: what a decode step hands over, 16-bit rows of
+        the cache's own type, dense and aligned, on the current device, and rows that fit (a full cache is
+        refused by the indexing below).  Six launches of indexing kernels otherwise."""
+        shape, dev, n = (self.batch_size, 1, self.kv_head, self.head_dim), keys.device, self.valid_length
+        if not (keys.is_cuda and dev.index == torch.cuda.current_device() and n.device == dev and n.dtype == torch.int32
+                and n.is_contiguous() and self._longest is not None and self._longest < self.max_length):
+            return False
+        for x in (key_states, value_states):
+            if not (x.shape == shape and x.dtype == keys.dtype and x.element_size() == 2 and x.device == dev
+                    and x.is_contiguous() and x.data_ptr() % 16 == 0 and not x.requires_grad):
+                return False
+        return True
+
     def decode_update_kv_cache(self, key_states, value_states, layer_idx):
         """Append one token per request (:133-151).  key/value_states: [batch, 1, kv_heads, head_dim]."""
-        pos = self.valid_length.to(self.key_cache[layer_idx].device).long()
-        self.key_cache[layer_idx][self._rows.to(pos.device), :, pos] = key_states[:, 0]
-        self.value_cache[layer_idx][self._rows.to(pos.device), :, pos] = value_states[:, 0]
+        keys, values = self.key_cache[layer_idx], self.value_cache[layer_idx]
+        if self._one_launch(keys, key_states, value_states):
+            _lib.check(_lib.lib.ri_dense_append(key_states.data_ptr(), value_states.data_ptr(), keys.data_ptr(),
+                                                values.data_ptr(), self.valid_length.data_ptr(), self.batch_size,
+                                                self.kv_head, self.max_length, _lib.current_stream()), "ri_dense_append")
+        else:
+            pos = self.valid_length.to(keys.device).long()
+            keys[self._rows.to(pos.device), :, pos] = key_states[:, 0]
+            values[self._rows.to(pos.device), :, pos] = value_states[:, 0]
         if layer_idx == self.layer_num - 1:
             self.context += 1
             self.valid_length += 1
+            if self._longest is not None:
+                self._longest += 1
         return self.key_cache[layer_idx], self.value_cache[layer_idx]

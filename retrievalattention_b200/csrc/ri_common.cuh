@@ -136,7 +136,8 @@ constexpr float RI_LOG2E = 1.4426950408889634f;
 // on: on one GPU it makes no difference to the decode kernel, between several GPUs the wait
 // kernel's launch hides behind the decode kernel and the next decode kernel's behind the wait.
 // The element-wise kernels of the decode layer (id 8) are on: their launch hides behind the library GEMM
-// in front of them (measured: 2 % of the whole model step), and so are those of the clustering build (ids 9, 10).
+// in front of them (measured: 2 % of the whole model step), and so are those of the clustering build (ids 9, 10)
+// and of the dense cache (id 11: append, attention, merge).
 __device__ __forceinline__ void ri_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void ri_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void ri_pdl_enter() {
@@ -155,7 +156,7 @@ inline cudaError_t ri_launch_pdl_id(int id, void (*kernel)(KArgs...), dim3 grid,
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  static const int mask = getenv("RI_PDL_MASK") ? atoi(getenv("RI_PDL_MASK")) : 0x763;   // per-kernel switch
+  static const int mask = getenv("RI_PDL_MASK") ? atoi(getenv("RI_PDL_MASK")) : 0xf63;   // per-kernel switch
   cfg.attrs = attr;
   cfg.numAttrs = (mask >> id) & 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);

@@ -58,3 +58,73 @@ def test_dense_decode_matches_fp32_attention_beside_the_wave_index():
                 # random, the worst case for clustering), so only its sanity is checked here
                 assert torch.isfinite(approx[b, 0].float()).all()
     assert dense.context == seq_len + 3 and dense.valid_length.tolist() == [seq_len + 3, seq_len - 37 + 3]
+
+
+@pytest.mark.parametrize("lengths,kv_heads,group,extra,dtype", [
+    ((1,), 1, 1, 0, torch.bfloat16),                        # one row: one step, one warp
+    ((0, 15, 16, 17), 2, 3, 0, torch.float16),              # a request without rows, edges of a 16-row step
+    ((0, 0, 1), 1, 8, 0, torch.bfloat16),                   # requests without rows in front
+    ((2047, 0, 130), 3, 5, 1, torch.float16),               # partial last steps, a CTA's range over several groups
+    ((4095,), 1, 7, 1, torch.bfloat16),                     # one group over the whole chip
+    ((37,) * 90, 8, 2, 1, torch.bfloat16),                  # more groups than warps
+])
+def test_dense_decode_kernel_equals_fp32_attention(lengths, kv_heads, group, extra, dtype):
+    """Tolerances as above: probabilities and outputs are rounded to 16 bits (2^-8 relative for bf16)."""
+    from types import SimpleNamespace
+
+    from retrievalattention_b200.attn_hub import decode_full_flash_attn, flash_attn
+
+    batch, room = len(lengths), max(lengths) + 3
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q = torch.randn((batch, 1, kv_heads * group, 128), generator=gen, device="cuda").to(dtype)
+    k, v = (torch.randn((batch, kv_heads, room, 128), generator=gen, device="cuda").to(dtype) for _ in range(2))
+    cache = SimpleNamespace(valid_length=torch.tensor(lengths, dtype=torch.int32, device="cuda"), layer_num=2)
+    assert flash_attn._dense_form(q, k, v, cache.valid_length)
+    out = decode_full_flash_attn(q, k, v, 1 - extra, cache)
+    for b, n in enumerate(lengths):
+        n += extra
+        if n == 0:
+            assert not out[b].any()
+            continue
+        s = torch.einsum("hgd,htd->hgt", q[b, 0].float().view(kv_heads, group, 128), k[b, :, :n].float()) / 128 ** 0.5
+        ref = torch.einsum("hgt,htd->hgd", torch.softmax(s, -1), v[b, :, :n].float()).reshape(-1, 128)
+        err = (out[b, 0].float() - ref).abs()
+        assert err.max() <= 2e-2 and err.mean() <= 2e-3, (b, float(err.max()), float(err.mean()))
+    # a view that is not dense takes the general operator: the same attention up to the order of the sums
+    wide = torch.randn((batch, 1, kv_heads * group, 256), generator=gen, device="cuda").to(dtype)
+    wide[..., :128] = q
+    assert flash_attn._dense_form(wide[..., :128], k, v, cache.valid_length) == (kv_heads * group == 1)
+    other = decode_full_flash_attn(wide[..., :128], k, v, 1 - extra, cache)
+    assert (other.float() - out.float()).abs().max() <= 2e-2
+
+
+@pytest.mark.parametrize("form", ["dense", "strided", "one_request", "full"])
+def test_dense_append_forms(form):
+    """Rows go where the indexing form puts them, whatever their strides; a full cache is refused."""
+    from retrievalattention_b200.cache_hub import flash_attn_cache
+
+    batch, hk, n = 3, 2, 40
+    cache = flash_attn_cache([0, 7, 3], 2, batch, n + (0 if form == "full" else 2), hk, 8, 128, torch.bfloat16,
+                             {"0": "cuda:0", "1": "cuda:0"}, 1, 8)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    for layer in range(2):
+        for b in range(batch):
+            k, v = (torch.randn((1, n, hk, 128), generator=gen, device="cuda").bfloat16() for _ in range(2))
+            cache.prefill_update_kv_cache(None, k, v, layer, b)
+    new = torch.randn((batch, 1, hk, 256), generator=gen, device="cuda").bfloat16()
+    k, v = new[..., :128], new[..., 128:]
+    if form == "dense":
+        k, v = k.contiguous(), v.contiguous()
+    if form == "one_request":
+        k, v = k[:1], v[:1]
+    wanted = form == "dense"
+    assert cache._one_launch(cache.key_cache[0], k, v) == wanted
+    if form == "full":                 # refused by the rule already: the indexing form is not run into its device check
+        assert not cache._one_launch(cache.key_cache[0], k.contiguous(), v.contiguous())
+        return
+    before = [t.clone() for t in (cache.key_cache[0], cache.value_cache[0])]
+    got = cache.decode_update_kv_cache(k, v, 0)
+    for old, now, rows in zip(before, got, (k, v)):
+        for b, start in enumerate((0, 7, 3)):
+            old[b, :, n - start] = rows[b if rows.shape[0] > 1 else 0, 0]
+        assert torch.equal(old, now)
