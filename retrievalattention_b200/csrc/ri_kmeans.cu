@@ -338,10 +338,11 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
 // round, so a token's running arg-max lives in two warps, which meet through shared memory once per token tile
 // (equal maxima: the lower index wins, as within a warp).  Every warp runs a fixed number of token tiles and rounds
 // whatever its waits return, so the named barrier of that merge is always reached.
-// CTAs are persistent, one per SM, each with an even run of token tiles over all problems.  A segmented launch of 8 heads x
-// 128K rows takes 152 us (before: 162); with the whole epilogue taken out 129 us, so most of what is left lies on the operand
-// side.  Sixteen epilogue warps instead of eight (176 us), token tiles asked for in L2 ten tiles ahead (no change) and
-// loading the first tokens under the kernel before (slower) were measured and left out.
+// CTAs are persistent, one per SM, each with an even run of token tiles over all problems.  The two centroid tiles of a round
+// are one product of N 256: as two of N 128 they read the token tile twice, and shared memory, which the operands of an N 128
+// product fill to the last byte a clock, held the tensor pipe up (8 heads x 128K rows: 164 -> 134 us a segmented launch).
+// Measured and left out, with the two products: sixteen epilogue warps instead of eight (176 against 162 us), token tiles asked
+// for in L2 ten tiles ahead (no change), the first tokens loaded under the kernel before (slower).
 constexpr int kResSlots = 3;
 constexpr int kResTiles = 4 * 2 * kHalfBytes /*B: 4 tiles*/ + kResSlots * 2 * kHalfBytes /*A ring*/;
 constexpr int kResSmem = kResTiles + kSmallBytes + 2 * kTileM * 6 /*merge of a token's two warps*/;
@@ -352,7 +353,7 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
   const AssignArgs& a = w.a;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
-  const uint32_t sB = base;                                         // [centroid tile][K half]
+  const uint32_t sB = base;                                         // [round][K half][centroid tile]
   const uint32_t sA = base + 4 * 2 * kHalfBytes;                    // [slot][K half]
   const uint32_t bars = sA + kResSlots * 2 * kHalfBytes;
   auto bar_a_full = [&](int s) { return bars + 8u * s; };
@@ -412,8 +413,10 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
         if (!ok) break;
         mbar_arrive_expect_tx(bar_b_full, n_tiles * 2 * kHalfBytes);
         for (int t = 0; t < n_tiles; ++t) {
-          tma_load_2d(sB + t * 2 * kHalfBytes, &map_cent, bar_b_full, 0, problem * a.n_cen + t * kTileN);
-          tma_load_2d(sB + t * 2 * kHalfBytes + kHalfBytes, &map_cent, bar_b_full, 64, problem * a.n_cen + t * kTileN);
+          // the two tiles of a round behind one another in either half: 256 rows for one product
+          const uint32_t dst = sB + ((t >> 1) * 4 + (t & 1)) * kHalfBytes;
+          tma_load_2d(dst, &map_cent, bar_b_full, 0, problem * a.n_cen + t * kTileN);
+          tma_load_2d(dst + 2 * kHalfBytes, &map_cent, bar_b_full, 64, problem * a.n_cen + t * kTileN);
         }
         ++loaded;
         for (; ok && unit < end; ++unit) {
@@ -452,19 +455,14 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
           ok = mbar_wait(bar_acc_empty(buf), ((j >> 1) & 1) ^ 1, abort_flag, 24);
           if (!ok) break;
           tc_fence_after();
+          // both centroid tiles of the round as one product of N 256 (the token tile is read once for the two)
+          const uint32_t idesc = 2 * r + 1 < n_tiles ? a.idesc + ((uint32_t)(kTileN >> 3) << 17) : a.idesc;
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int ct = 2 * r + h;
-            if (ct < n_tiles) {
-              const uint32_t d_tmem = tmem_base + buf * 2 * kTileN + h * kTileN;
+          for (int kb = 0; kb < 2; ++kb) {
+            const uint64_t da = umma_desc_sw128(sA + (s * 2 + kb) * kHalfBytes);
+            const uint64_t db = umma_desc_sw128(sB + (r * 2 + kb) * 2 * kHalfBytes);
 #pragma unroll
-              for (int kb = 0; kb < 2; ++kb) {
-                const uint64_t da = umma_desc_sw128(sA + (s * 2 + kb) * kHalfBytes);
-                const uint64_t db = umma_desc_sw128(sB + (ct * 2 + kb) * kHalfBytes);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) tc_mma_f16(d_tmem, da + 2 * k, db + 2 * k, a.idesc, (kb | k) != 0);
-              }
-            }
+            for (int k = 0; k < 4; ++k) tc_mma_f16(tmem_base + buf * 2 * kTileN, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
           }
           tc_commit(bar_acc_full(buf));
         }
