@@ -933,8 +933,7 @@ def prefill_summary(geo, log, seq=16384):
     ms, out = timed(lambda: ra.retroinfer_prefill_attn(q, k, v, True))
     ra.check_prefill_errors()
     _, burst, kind = measured_peaks()
-    res = {"workload": f"causal attention over one prompt of {seq} tokens, {geo.q_heads}q/{geo.kv_heads}kv heads, d128, bf16 "
-                       "(V transposed inside the call)",
+    res = {"workload": f"causal attention over one prompt of {seq} tokens, {geo.q_heads}q/{geo.kv_heads}kv heads, d128, bf16",
            "ms": round(ms, 3), "tflops": round(flop / ms / 1e9, 1), "bound": "tensor", "peak": burst,
            "peak_kind": "of " + kind, "frac": round(flop / ms / 1e9 / burst, 4)}
     try:
