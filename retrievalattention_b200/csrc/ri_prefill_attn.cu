@@ -8,8 +8,8 @@
 //                   straight from the token-major tensors, fp32 accumulator in TMEM;
 //   softmax         one group of 128 threads per query tile, one thread per query row (= TMEM lane): a row of S comes
 //                   down with tcgen05.ld into registers; online softmax in the log2 domain with a LAZY reference maximum
-//                   (the running maximum is only adopted when it has grown by more than 2^8, so an accumulator is
-//                   rescaled rarely); P goes back to TMEM as packed 16-bit pairs over the columns of S it came from;
+//                   (the running maximum is only adopted when it has grown by more than a step, so an accumulator
+//                   is rescaled rarely); P goes back to TMEM as packed 16-bit pairs over the columns of S it came from;
 //   O_g += P_g.V    tcgen05.mma with A = P_g from TMEM and B = the V tile as TMA brought it (channels contiguous:
 //                   an MN-major operand), accumulator in TMEM for the whole walk.
 // TMEM: S_0 | S_1 | O_0 | O_1, 128 columns each.  Warps: TMA producer, MMA issuer, two idle, eight softmax/epilogue warps,
@@ -43,7 +43,13 @@ constexpr uint32_t kTmemCols = 512;        // S_0 | S_1 | O_0 | O_1, 128 columns
 constexpr int smem_bytes(bool split) {
   return 1024 /*align*/ + (split ? 1 : 2) * 2 * kHalf /*Q_0, Q_1*/ + kSlots * 2 * kHalf /*K, V*/ + 256 /*barriers*/;
 }
-constexpr float kLazy = 8.0f;              // the reference maximum follows the running one in steps of more than 2^8
+// The reference maximum follows the running one in steps of more than 2^lazy.  A key whose score is the reference has a
+// probability of exactly 1, any other one is rounded to 16 bits, so a reference that lags behind costs accuracy: for keys
+// with a few near ones among many (a trained model's) the paired form's one walk per row was 3 % further from 64-bit
+// attention at 2^8 than two walks, which start from two references, are at the same step.  Relative error of the paired
+// form, bf16, 32768 tokens: 2.12e-3 at 2^8, 1.97e-3 at 2^4 with rows catching up together (two walks 2.06e-3, rounding the
+// result alone 1.65e-3), for 1 % of the time (8.28 -> 8.36 ms a repeated run, 32 query heads).
+__host__ __device__ constexpr float lazy_step(bool split) { return split ? 8.0f : 4.0f; }
 
 struct AttnArgs {
   void* out;             // [B, S, Hq, 128]
@@ -341,10 +347,11 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         for (int i = 2; i < 32; i += 2) mx[c] = max3(mx[c], __uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1]));
       }
       const float m_tile = max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]) * a.scale2;
-      // lazy reference maximum: adopt the running maximum only when it has grown by more than kLazy
-      const bool move = m_tile > m_ref + kLazy;            // also true for the first tile (m_ref = -inf)
+      // lazy reference maximum: adopt the running maximum only when it has grown by more than the step
+      const bool move = m_tile > m_ref + lazy_step(SPLIT);      // also true for the first tile (m_ref = -inf)
       if (__any_sync(0xffffffffu, move)) {
-        const float m_new = move ? m_tile : m_ref;
+        // pairs: the warp's accumulator rows are multiplied anyway, so every row of it catches up with its maximum
+        const float m_new = SPLIT ? (move ? m_tile : m_ref) : fmaxf(m_ref, m_tile);
         const float factor = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);      // 1 when the maximum stays
         l_run *= factor;
         m_ref = m_new;

@@ -86,3 +86,49 @@ def test_query_tile_pairs_and_split_walks(batch, seq, hq, hk, causal):
     ra.check_prefill_errors()
     err = (out.float() - reference(q[:1], k[:1], v[:1], causal)).abs()
     assert err.max() <= 2e-2 and err.mean() <= 2e-3, (float(err.max()), float(err.mean()))
+
+
+def two_walks(scores, v, tiles, dtype):
+    """Attention of rows of scores (log2 domain, fp32, masked) as two walks over the even and the odd tiles of 128 keys give
+    it, each with its own reference maximum that follows in steps of more than 2^8, probabilities rounded to `dtype`."""
+    parts = []
+    for first in (0, 1):
+        m = torch.full(scores.shape[:1], -torch.inf, device=scores.device)
+        total, acc = torch.zeros_like(m), torch.zeros((scores.shape[0], 128), device=scores.device)
+        for t in range(first, tiles, 2):
+            s = scores[:, t * 128:(t + 1) * 128]
+            top = s.max(1).values
+            new = torch.where(top > m + 8, top, m)
+            ref = new.nan_to_num(neginf=0.0)
+            factor, p = torch.exp2(m - ref), torch.exp2(s - ref[:, None])
+            total = total * factor + p.sum(1)
+            acc = acc * factor[:, None] + p.to(dtype).float() @ v[t * 128:(t + 1) * 128].float()
+            m = new
+        parts.append((m, total, acc))
+    top = torch.maximum(parts[0][0], parts[1][0])
+    weight = [torch.exp2(m - top) for m, _, _ in parts]
+    return sum(w[:, None] * a for w, (_, _, a) in zip(weight, parts)) / sum(w * t for w, (_, t, _) in zip(weight, parts))[:, None]
+
+
+@pytest.mark.parametrize("seq,hq,hk,dtype", [(2500, 32, 8, torch.bfloat16), (5001, 28, 4, torch.float16), (8192, 8, 8, torch.bfloat16)])
+def test_pairs_are_as_accurate_as_two_walks(seq, hq, hk, dtype):
+    """Where two query tiles share the keys there is one walk per row.  Its distance from 64-bit attention must not exceed
+    that of the same rows in two walks (computed here); the keys are clustered, so some scores stand out."""
+    from retrievalattention_b200.attn_hub import retroinfer_attn as ra
+    from retrievalattention_b200.synthetic import make_kv
+
+    q = torch.randn((1, seq, hq, 128), generator=torch.Generator(device="cuda").manual_seed(17), device="cuda").to(dtype)
+    k, v = make_kv(hk, seq, 128, seed=93, device="cuda", dtype=dtype)
+    out = ra.retroinfer_prefill_attn(q, k, v, True)
+    ra.check_prefill_errors()
+    rows = torch.randperm(seq, generator=torch.Generator().manual_seed(1))[:1024].cuda()
+    mine = theirs = 0.0
+    torch.backends.cuda.matmul.allow_tf32 = False
+    for h in range(0, hq, hq // 8):
+        keys, vals = k[0, :, h // (hq // hk)], v[0, :, h // (hq // hk)]
+        s = q[0, rows, h].double() @ keys.double().T * (1.4426950408889634 / 128 ** 0.5)
+        s = s.masked_fill(torch.arange(seq, device="cuda")[None] > rows[:, None], -torch.inf)
+        exact = torch.softmax(s * 0.6931471805599453, -1) @ vals.double()
+        mine += float((out[0, rows, h].double() - exact).pow(2).sum())
+        theirs += float((two_walks(s.float(), vals, -(-seq // 128), dtype).to(dtype).double() - exact).pow(2).sum())
+    assert mine <= theirs, ((mine / theirs) ** 0.5)
