@@ -192,7 +192,10 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
     if (base & 1023u) *a.error_flag = s_skip = 19;      // the tiles would not lie as the descriptors say
   }
   __syncthreads();
-  if (s_skip) return;
+  if (s_skip) {              // not before the kernel in front has ended: the one behind waits for this grid alone
+    ri_pdl_wait();
+    return;
+  }
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int unit_lo, unit_hi;                             // this CTA's 256-token blocks
@@ -373,7 +376,10 @@ kmeans_assign_resident_kernel(const __grid_constant__ CUtensorMap map_keys, cons
     if (base & 1023u) *a.error_flag = s_skip = 19;      // the tiles would not lie as the descriptors say
   }
   __syncthreads();
-  if (s_skip) return;
+  if (s_skip) {              // not before the kernel in front has ended: the one behind waits for this grid alone
+    ri_pdl_wait();
+    return;
+  }
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int unit_lo, unit_hi;                             // this CTA's 128-token tiles, over one problem or more
