@@ -75,9 +75,16 @@ def build_prompt_index(keys: torch.Tensor, values: torch.Tensor, num_segments: i
     ``cluster_count``, ``cluster_offset``, ``empty`` (bool) of the request's heads, and ``keys``, ``values``,
     ``steady_keys``, ``steady_values`` ``[kv_heads, rows, 128]`` whose rows behind the used ones stay as they are.
     Returns the status word (non-zero if a device-side wait timed out)."""
-    tokens, z, _ = keys.shape
+    assert keys.is_cuda and values.is_cuda, "k-means runs on the GPU only"
+    assert keys.dim() == 3 and keys.shape == values.shape and keys.shape[-1] == 128, "expected [tokens, kv_heads, 128]"
+    assert keys.is_contiguous() and values.is_contiguous() and values.dtype == keys.dtype
+    tokens, z, d = keys.shape
     dt, n, c = keys.dtype, tokens - sink - recent, out["centroids"].shape[1]
-    assert keys.is_contiguous() and values.is_contiguous() and values.shape == keys.shape
+    assert all(t.device == keys.device for t in (values, *out.values())), "prompt and index lie on one GPU"
+    assert out["centroids"].shape == out["value_sum"].shape == (z, c, d) and out["cluster_offset"].shape == (z, c + 1)
+    assert all(out[name].shape == (z, c) for name in ("cluster_size", "cluster_count", "empty"))
+    assert all(out[name].dtype == dt for name in ("centroids", "value_sum", "cluster_size"))
+    assert out["cluster_count"].dtype == out["cluster_offset"].dtype == torch.int32 and out["empty"].dtype == torch.bool
     p, q = _lib.KMeans(), _lib.KMeansPrompt()
     p.groups, p.n_tokens, p.n_centroids, p.n_segments, p.n_iters = z, n, c, num_segments, num_iters
     p.dtype, p.center = _lib.dtype_code(dt), 1
@@ -88,12 +95,13 @@ def build_prompt_index(keys: torch.Tensor, values: torch.Tensor, num_segments: i
     error = torch.empty((1,), dtype=torch.int32, device=keys.device)
     p.d_keys, p.d_values, p.d_scratch, p.d_error = keys.data_ptr(), values.data_ptr(), scratch.data_ptr(), error.data_ptr()
     for name in ("centroids", "value_sum", "cluster_size", "cluster_count", "cluster_offset"):
-        assert out[name].is_contiguous() and out[name].shape[0] == z
+        assert out[name].is_contiguous()
         setattr(p, "d_" + name, out[name].data_ptr())
     for name in ("keys", "values", "steady_keys", "steady_values"):
-        assert out[name].is_contiguous() and out[name].dtype == dt and out[name].shape[0] == z
+        assert out[name].is_contiguous() and out[name].dtype == dt and out[name].shape == (z, out[name].shape[1], d)
     assert out["keys"].shape == out["values"].shape and out["keys"].shape[1] >= n
     assert out["steady_keys"].shape == out["steady_values"].shape and out["empty"].is_contiguous()
+    assert out["steady_keys"].shape[1] >= sink + recent
     p.d_keys_out, p.d_values_out = out["keys"].data_ptr(), out["values"].data_ptr()
     q.n_sink, q.n_recent, q.out_group_rows = sink, recent, out["keys"].shape[1]
     q.steady_group_rows = out["steady_keys"].shape[1]

@@ -218,6 +218,16 @@ class retroinfer_cache(KV_Cache):
         self._keep_alive = []
 
     # ------------------------------------------------------------------ prefill
+    def _prompt_form(self, key_states, value_states, centroids, clustered) -> bool:
+        """Whether the clustering can read the prompt where it lies and write into the cache's own tensors: rows of the
+        cache's type and heads, on the cache's GPU, which is the current one.  Any other prompt is clustered by itself
+        (in its own type, on its own GPU) and copied into the cache, or refused there."""
+        shape, dev = (*key_states.shape[:2], self.kv_head, self.head_dim), centroids.device
+        return (dev.type == "cuda" and dev.index == torch.cuda.current_device() and clustered > 0
+                and centroids.shape[1] == self.n_centroids
+                and all(x.shape == shape and x.dtype == self.dtype and x.device == dev
+                        and not (x.requires_grad and torch.is_grad_enabled()) for x in (key_states, value_states)))
+
     def prefill_update_kv_cache(self, query_states, key_states, value_states, layer_idx, batch_idx):
         """One request, one layer (:368-441).  key/value_states: [1, seq_len, kv_heads, head_dim]."""
         bsz, seq_len, group_num, head_dim = key_states.shape
@@ -233,14 +243,31 @@ class retroinfer_cache(KV_Cache):
                "cluster_offset": self.cluster_offset[layer_idx][rows], "empty": self.centroids_mask[layer_idx][rows],
                "steady_keys": self.steady_zone_keys[layer_idx][batch_idx],
                "steady_values": self.steady_zone_values[layer_idx][batch_idx]}
-        if self.kv_on_host:
-            laid_out = torch.empty((2, self.kv_head, valid_length, head_dim), dtype=self.dtype, device=key_states.device)
-            out["keys"], out["values"] = laid_out[0], laid_out[1]
+        if self._prompt_form(key_states, value_states, out["centroids"], valid_length):
+            if self.kv_on_host:
+                laid_out = torch.empty((2, self.kv_head, valid_length, head_dim), dtype=self.dtype, device=key_states.device)
+                out["keys"], out["values"] = laid_out[0], laid_out[1]
+            else:
+                out["keys"], out["values"] = self.list_keys[layer_idx][batch_idx], self.list_values[layer_idx][batch_idx]
+            prompt = [x[0, vs:].contiguous() for x in (key_states, value_states)]
+            prompt = [x if x.data_ptr() % 16 == 0 else x.clone() for x in prompt]      # the kernels load 16 bytes at a time
+            self._error_flags.append(build_prompt_index(*prompt, self.n_segment, start, end, out))
         else:
-            out["keys"], out["values"] = self.list_keys[layer_idx][batch_idx], self.list_values[layer_idx][batch_idx]
-        self._error_flags.append(build_prompt_index(key_states[0, vs:].to(self.dtype).contiguous(),
-                                                    value_states[0, vs:].to(self.dtype).contiguous(),
-                                                    self.n_segment, start, end, out))
+            temp_keys = key_states[0, vs + start:seq_len - end].transpose(0, 1).contiguous()      # [kv_heads, N_b, d]
+            temp_values = value_states[0, vs + start:seq_len - end].transpose(0, 1).to(temp_keys.dtype).contiguous()
+            for zone, states in ((out["steady_keys"], key_states), (out["steady_values"], value_states)):
+                zone[:, :start] = states[0, vs:vs + start].transpose(0, 1)
+                zone[:, start:total] = states[0, seq_len - end:seq_len].transpose(0, 1)
+            r = build_index(temp_keys, temp_values, self.n_centroids, self.n_segment)
+            for name in ("centroids", "value_sum", "cluster_size", "cluster_count", "cluster_offset"):
+                out[name].copy_(r[name])
+            out["empty"].copy_(r["cluster_count"] == 0)
+            self._error_flags.append(r["error"])
+            if self.kv_on_host:
+                out = r
+            else:
+                self.list_keys[layer_idx][batch_idx, :, :valid_length].copy_(r["keys"])
+                self.list_values[layer_idx][batch_idx, :, :valid_length].copy_(r["values"])
         if self.kv_on_host:
             # the offload of this request-layer's laid-out rows runs on a side stream, under the clustering of the next
             # request-layer (the reference's offload <-> k-means overlap, :388-403); at most two laid-out copies are

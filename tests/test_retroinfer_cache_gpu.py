@@ -160,3 +160,58 @@ def test_use_cluster_estimation_attends_clusters_searched_one_layer_ahead():
             if l != 1:          # no estimate, or a perfect one: the same clusters as the ordinary path
                 assert (out.float() - base.float()).abs().max() <= 1e-2
     assert not any(ahead._ahead)
+
+
+@pytest.mark.parametrize("form,on_host", [(f, h) for f in ("plain", "strided", "unaligned", "other_type", "values_other_type", "one_head")
+                                          for h in (False, True) if not (h and f == "one_head")])
+def test_prompts_of_any_form_give_the_index_of_their_rows(form, on_host):
+    """Whatever strides, offset, type or heads a prompt comes with: the cache holds what ``build_index`` gives for its
+    clustered rows (in the keys' type, as they lie), converted to the cache's type and repeated over its heads, and the
+    sink and recent rows."""
+    from retrievalattention_b200.cache_hub import retroinfer_cache
+    from retrievalattention_b200.cache_hub.kmeans import build_index
+
+    seq_len, kv_heads, vs, dev = 1024 + 68 + 37, 2, 37, "cuda:0"
+    cfg = generate_config(seq_len, 0.05, 0.2, n_segments=1)
+    cache = retroinfer_cache([vs], 1, 1, seq_len + 6, kv_heads, 8, 128, torch.bfloat16, {"0": dev}, 6, num_gpus=1,
+                             model_size=8, kv_on_host=on_host, **cfg.as_kwargs())
+    k, v = make_kv(kv_heads, seq_len, 128, seed=5, device="cuda")
+    if form == "strided":
+        both = torch.cat((k, v), dim=-1)
+        k, v = both[..., :128], both[..., 128:]
+        assert not k.is_contiguous()
+    if form == "unaligned":
+        k, v = (torch.cat((x.new_zeros(1), x.reshape(-1)))[1:].view(x.shape) for x in (k, v))
+        assert k.is_contiguous() and k.data_ptr() % 16 == 2
+    if form == "other_type":
+        k, v = k.half(), v.half()
+    if form == "values_other_type":
+        v = v.half()
+    if form == "one_head":
+        k, v = k[:, :, :1].contiguous(), v[:, :, :1].contiguous()
+    cache.prefill_update_kv_cache(None, k, v, 0, 0)
+    torch.cuda.synchronize()
+    mid = [x[0, vs + 4:seq_len - 64].transpose(0, 1).to(k.dtype).contiguous().clone() for x in (k, v)]
+    r = build_index(*mid, cfg.n_centroids, cfg.n_segment)
+    for name in ("centroids", "value_sum", "cluster_size", "cluster_count", "cluster_offset"):
+        got = getattr(cache, name)[0]
+        assert torch.equal(got, r[name].to(got.dtype).expand_as(got)), name
+    assert torch.equal(cache.centroids_mask[0], (r["cluster_count"] == 0).expand(kv_heads, -1))
+    n = seq_len - 68 - vs
+    for name, raw in (("keys", k), ("values", v)):
+        rows = getattr(cache, "list_" + name)[0][0]
+        assert torch.equal(rows[:, :n].cpu(), r[name].to(rows.dtype).expand(kv_heads, n, 128).cpu()) and not rows[:, n:].any()
+        ends = torch.cat((raw[0, vs:vs + 4], raw[0, seq_len - 64:]), 0).transpose(0, 1).to(torch.bfloat16)
+        assert torch.equal(getattr(cache, "steady_zone_" + name)[0][0, :, :68], ends.expand(kv_heads, 68, 128))
+    cache.prepare_cache()
+
+
+@pytest.mark.parametrize("form", ["head_dim_64", "head_dim_256", "host", "float32"])
+def test_prompts_that_are_refused(form):
+    cache, _ = make_cache(1, 1, 2, 8, 1024 + 68, 6, [0], n_segment=1)
+    d = {"head_dim_64": 64, "head_dim_256": 256}.get(form, 128)
+    k = torch.zeros((1, 1024 + 68, 2, d), dtype=torch.float32 if form == "float32" else torch.bfloat16,
+                    device="cpu" if form == "host" else "cuda")
+    with pytest.raises((AssertionError, RuntimeError, TypeError)):
+        cache.prefill_update_kv_cache(None, k, k, 0, 0)
+    assert not cache.list_keys[0].any() and not cache._error_flags
