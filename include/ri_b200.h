@@ -35,6 +35,11 @@ enum { RI_HEAD_DIM = 128 };
 const char* ri_last_error(void);
 int ri_version(void);
 
+/* A 32-bit status word in page-locked host memory, one for the whole process and valid on every GPU: what d_error pointers
+ * of the kernels may point at.  Cleared when it is made, by the first call; the caller reads and clears it on the host.
+ * May be called while a stream is being captured.  NULL (with ri_last_error()) when the memory cannot be had. */
+int32_t* ri_status_word(void);
+
 /* ------------------------------------------------------------------------------------------
  * Fused decode path (all clusters resident in HBM in cluster-contiguous order).
  * Replaces, per layer and decode step, the whole body of
@@ -220,7 +225,7 @@ int ri_silu_and_mul(const void* d_in, void* d_out, int32_t rows, int32_t inter, 
  * d_q, d_out: [batch, seq_len, q_heads, 128]; d_k, d_v: [batch, seq_len, kv_heads, 128] (token-major, contiguous);
  * query head h attends kv head h / (q_heads / kv_heads); causal != 0: token i sees tokens 0..i.
  * d_scratch: not used any more, may be null (ri_prefill_attn_scratch_bytes() keeps its values);
- * d_error: [1], must be zero on entry; set non-zero if a bounded device-side wait ran out.
+ * d_error: [1], stays as it is unless a bounded device-side wait runs out (then non-zero: which one); not read.
  * ------------------------------------------------------------------------------------------ */
 int64_t ri_prefill_attn_scratch_bytes(int32_t batch, int32_t seq_len, int32_t kv_heads);
 int ri_prefill_attn(const void* d_q, const void* d_k, const void* d_v, void* d_out, void* d_scratch, int32_t* d_error,

@@ -96,6 +96,8 @@ def _load() -> C.CDLL:
     lib.ri_wave_gather_wait.argtypes = [C.POINTER(WaveGather), C.c_void_p]
     lib.ri_wave_scratch_views.restype = C.c_int
     lib.ri_wave_scratch_views.argtypes = [C.POINTER(WaveLayer), C.POINTER(WaveViews)]
+    lib.ri_status_word.restype = C.c_void_p
+    lib.ri_status_word.argtypes = []
     lib.ri_kmeans_scratch_bytes.restype = C.c_int64
     lib.ri_kmeans_scratch_bytes.argtypes = [C.POINTER(KMeans)]
     lib.ri_kmeans_build.restype = C.c_int

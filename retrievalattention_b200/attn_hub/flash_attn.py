@@ -3,11 +3,13 @@ of the wave-index path.  Decoding runs ``ri_dense_decode`` over the head-major c
 ``check_prefill_errors()`` reports its device-side waits too."""
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 
 from .. import _lib
 from ..kernels import weighted_flash_decoding
-from .retroinfer_attn import _status_word, retroinfer_prefill_attn
+from .retroinfer_attn import _status_word, check_prefill_errors, retroinfer_prefill_attn
 
 
 def prefill_full_flash_attn(query_states, key_states, value_states, causal):
@@ -41,15 +43,14 @@ def decode_full_flash_attn(query_states, key_states, value_states, layer_idx, fu
     g, gs = b * hk, hq // hk
     if _dense_form(query_states, key_states, value_states, c.valid_length):
         out = torch.empty_like(query_states)
-        capturing = torch.cuda.is_current_stream_capturing()
-        status = _status_word(out.device, capturing)
+        status = _status_word(out.device)
         scratch = torch.empty((_lib.lib.ri_dense_decode_scratch_bytes(b, hk, gs),), dtype=torch.uint8, device=out.device)
         _lib.check(_lib.lib.ri_dense_decode(
             query_states.data_ptr(), key_states.data_ptr(), value_states.data_ptr(), c.valid_length.data_ptr(), extra,
-            out.data_ptr(), scratch.data_ptr(), status.address, b, hk, gs, length, _lib.dtype_code(out.dtype), _lib.current_stream()),
+            out.data_ptr(), scratch.data_ptr(), C.addressof(status), b, hk, gs, length, _lib.dtype_code(out.dtype), _lib.current_stream()),
             "ri_dense_decode")
-        if not capturing:
-            status.tick()
+        if status.value and not torch.cuda.is_current_stream_capturing():
+            check_prefill_errors()
         return out
     valid = c.valid_length + extra
     seqlens = valid.to(query_states.device).to(torch.int32).repeat_interleave(hk)

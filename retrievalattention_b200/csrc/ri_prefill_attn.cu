@@ -25,7 +25,9 @@
 // clocks per tile and group; tensor pipe 59 % and exponentials 59 % of the time, issue slots 36 %.  Doing a quarter of the
 // exponentials as polynomials on the FMA pipe was slower (1170 TFLOP/s): they are not what the chain waits for.
 // SPLIT: for few query tiles a CTA takes one of them, and its groups take the even and the odd key/value tiles.
-// Every mbarrier wait is bounded; on expiry the kernel records where, releases its TMEM and returns.
+// Every mbarrier wait is bounded; on expiry a CTA records where, releases its TMEM and returns.  The word it is recorded in
+// is only written: what an earlier call left there makes no later one give up (all CTAs of a launch are resident at once, so
+// one that gives up saves the others nothing).
 #include <cuda.h>
 
 #include "ri_common.cuh"
@@ -139,12 +141,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   auto bar_q_empty = [&](int g) { return bars + 8u * (10 + 2 * kSlots + g); };
   auto bar_p_part = [&](int g) { return bars + 8u * (8 + 2 * kSlots + g); };
   __shared__ uint32_t s_tmem_base;
-  __shared__ int s_abort, s_skip;
+  __shared__ int s_abort;
   __shared__ float2 s_stat[2][SPLIT ? kTile : 1];          // SPLIT: a row's (maximum, sum) in either group
-
-  if (threadIdx.x == 0) s_skip = *reinterpret_cast<volatile int*>(a.error_flag);
-  __syncthreads();
-  if (s_skip) return;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_items = a.units * a.Hq * a.B;

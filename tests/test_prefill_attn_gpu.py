@@ -132,3 +132,76 @@ def test_pairs_are_as_accurate_as_two_walks(seq, hq, hk, dtype):
         mine += float((out[0, rows, h].double() - exact).pow(2).sum())
         theirs += float((two_walks(s.float(), vals, -(-seq // 128), dtype).to(dtype).double() - exact).pow(2).sum())
     assert mine <= theirs, ((mine / theirs) ** 0.5)
+
+
+@pytest.mark.parametrize("seq,hq", [(300, 2), (1300, 32)])       # one query tile per CTA, and pairs
+def test_a_recorded_failure_is_reported_once_and_stops_no_later_call(seq, hq):
+    import ctypes as C
+
+    from retrievalattention_b200 import _lib
+    from retrievalattention_b200.attn_hub import retroinfer_attn as ra
+
+    g = torch.Generator(device="cuda").manual_seed(seq)
+    q, k, v = (torch.randn((1, seq, h, 128), generator=g, device="cuda").to(torch.bfloat16) for h in (hq, 2, 2))
+    good = ra.retroinfer_prefill_attn(q, k, v, True)
+    ra.check_prefill_errors()
+    status = ra._status_word(q.device)
+    out = torch.zeros_like(q)
+    status.value = 31                                     # as a kernel of an earlier call would have left it
+    _lib.check(_lib.lib.ri_prefill_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), None, C.addressof(status), 1, seq,
+                                        hq, 2, 1, _lib.dtype_code(q.dtype), _lib.current_stream()))
+    torch.cuda.synchronize()
+    assert status.value == 31 and torch.equal(good, out)
+    with pytest.raises(RuntimeError, match="31"):         # the first call that finds it says so
+        ra.retroinfer_prefill_attn(q, k, v, True)
+    assert torch.equal(good, ra.retroinfer_prefill_attn(q, k, v, True))
+    ra.check_prefill_errors()
+
+
+def test_status_of_captured_calls():
+    """The word is clear before a captured call's first replay, and failures of any replay are reported, also behind an
+    earlier check."""
+    from types import SimpleNamespace
+
+    from retrievalattention_b200.attn_hub import decode_full_flash_attn, retroinfer_attn as ra
+
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn((1, 300, h, 128), generator=g, device="cuda").to(torch.bfloat16) for h in (4, 2, 2))
+    kc, vc = (x.transpose(1, 2).contiguous() for x in (k, v))
+    cache = SimpleNamespace(valid_length=torch.tensor([290], dtype=torch.int32, device="cuda"), layer_num=1)
+    calls = (lambda: ra.retroinfer_prefill_attn(q, k, v, True), lambda: decode_full_flash_attn(q[:, :1], kc, vc, 0, cache))
+    want = [f() for f in calls]
+    ra.check_prefill_errors()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = [f() for f in calls]
+    ra.check_prefill_errors()
+    for _ in range(2):
+        for x in got:
+            x.zero_()
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        ra.check_prefill_errors()
+        ra._status_word(q.device).value = 24
+        with pytest.raises(RuntimeError, match="24"):
+            ra.check_prefill_errors()
+
+
+def test_first_call_of_a_process_may_be_captured():
+    """Its status word is made under the capture."""
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from retrievalattention_b200.attn_hub import retroinfer_attn as ra
+q, k = (torch.randn((1, 300, h, 128), device="cuda").bfloat16() for h in (4, 2))
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    out = ra.retroinfer_prefill_attn(q, k, k, True)
+ra.check_prefill_errors()
+graph.replay()
+ra.check_prefill_errors()
+assert torch.equal(out, ra.retroinfer_prefill_attn(q, k, k, True))
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)

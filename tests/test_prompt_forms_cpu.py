@@ -54,3 +54,11 @@ def test_rule_for_reading_the_prompt_in_place(monkeypatch, wanted, change):
     with torch.set_grad_enabled(change.get("grad", True)):
         for keys, values in ((other, plain), (plain, other)):      # either tensor decides
             assert retroinfer_cache._prompt_form(cache, keys, values, centroids, change.get("clustered", 132)) is wanted
+
+
+def test_prefill_attention_refuses_host_tensors():
+    from retrievalattention_b200.attn_hub import retroinfer_prefill_attn
+
+    x = torch.zeros((1, 8, 2, 128), dtype=torch.bfloat16)
+    with pytest.raises(ValueError, match="one GPU"):
+        retroinfer_prefill_attn(x, x, x, True)
