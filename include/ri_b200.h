@@ -31,6 +31,7 @@ typedef enum ri_status {
 
 enum { RI_BF16 = 0, RI_F16 = 1 };
 enum { RI_HEAD_DIM = 128 };
+enum { RI_STATUS_CACHE_FULL = 60 };   /* in a status word: a row did not fit its cache; other values name the wait that gave up */
 
 const char* ri_last_error(void);
 int ri_version(void);
@@ -321,12 +322,12 @@ int ri_weighted_flash_decoding(const void* d_q, const void* d_k, const void* d_v
 
 /* Decoding with full attention over a dense cache [batch, kv_heads, rows_stride, 128] (cache_hub/flash_attn_cache.py:133-151,
  * attn_hub/flash_attn.py:17-30).  ri_dense_append stores d_k/d_v [batch, kv_heads, 128] at row d_valid_length[b] of every
- * head of request b (nothing where that row lies outside the cache).  ri_dense_decode attends rows
+ * head of request b (where that row lies outside the cache nothing, and *d_error becomes RI_STATUS_CACHE_FULL).  ri_dense_decode attends rows
  * [0, d_valid_length[b] + extra) (at most rows_stride) with d_q [batch, kv_heads, group_size, 128]; d_scratch: that many
  * bytes of 16-byte aligned device memory, for this call alone, with any contents; *d_error stays as it is unless a
  * device-side wait gave up. */
 int ri_dense_append(const void* d_k, const void* d_v, void* d_keys, void* d_values, const int32_t* d_valid_length,
-                    int32_t batch, int32_t kv_heads, int64_t rows_stride, void* stream);
+                    int32_t* d_error, int32_t batch, int32_t kv_heads, int64_t rows_stride, void* stream);
 int64_t ri_dense_decode_scratch_bytes(int32_t batch, int32_t kv_heads, int32_t group_size);
 int ri_dense_decode(const void* d_q, const void* d_k, const void* d_v, const int32_t* d_valid_length, int32_t extra,
                     void* d_out, void* d_scratch, int32_t* d_error, int32_t batch, int32_t kv_heads, int32_t group_size,

@@ -15,6 +15,7 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("RI_B200_LIB") or os.path.join(_PKG, "lib", "libri_b200.so")
 
 RI_BF16, RI_F16 = 0, 1
+RI_STATUS_CACHE_FULL = 60
 
 
 class WaveLayer(C.Structure):
@@ -133,7 +134,7 @@ def _load() -> C.CDLL:
     lib.ri_weighted_flash_decoding.restype = C.c_int
     lib.ri_weighted_flash_decoding.argtypes = [C.c_void_p] * 9 + [C.c_int32, C.c_int32, C.c_int64, C.c_int32, C.c_void_p]
     lib.ri_dense_append.restype = C.c_int
-    lib.ri_dense_append.argtypes = [C.c_void_p] * 5 + [C.c_int32, C.c_int32, C.c_int64, C.c_void_p]
+    lib.ri_dense_append.argtypes = [C.c_void_p] * 6 + [C.c_int32, C.c_int32, C.c_int64, C.c_void_p]
     lib.ri_dense_decode_scratch_bytes.restype = C.c_int64
     lib.ri_dense_decode_scratch_bytes.argtypes = [C.c_int32] * 3
     lib.ri_dense_decode.restype = C.c_int

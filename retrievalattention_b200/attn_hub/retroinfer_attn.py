@@ -7,8 +7,8 @@ import torch
 
 from .. import _lib
 
-# Where the prefill and dense decode kernels record that a device-side wait gave up (0: none did): one word in page-locked
-# host memory for all devices and streams, replays of CUDA graphs among them.  The kernels only write it, so a failure stays
+# Where the prefill and dense decode kernels record that a device-side wait gave up, and the dense append that a row did not
+# fit (0: none of it): one word in page-locked host memory for all devices and streams, replays of CUDA graphs among them.  The kernels only write it, so a failure stays
 # inside its call; it stays set until it is reported, by ``check_prefill_errors`` or by the first call that finds it set.
 _word = None
 _devices: set = set()
@@ -50,12 +50,14 @@ def retroinfer_prefill_attn(query_states, key_states, value_states, causal):
 
 def check_prefill_errors() -> None:
     """Raise if any prefill or dense decode call since the last check, replays of captured ones among them, gave up on a
-    device-side wait (synchronises)."""
+    device-side wait, or a dense cache was full when a row was appended (synchronises)."""
     for device in list(_devices):
         torch.cuda.synchronize(device)
     code = 0 if _word is None else _word.value
     if code:
         _word.value = 0
+        if code == _lib.RI_STATUS_CACHE_FULL:
+            raise RuntimeError("a token's rows did not fit the dense cache (more decode steps than max_length has room for)")
         raise RuntimeError(f"ri_prefill_attn or ri_dense_decode gave up on a device-side wait (code {code})")
 
 

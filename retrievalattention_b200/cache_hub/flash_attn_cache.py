@@ -9,10 +9,13 @@ reference falls back to pinned host memory during prefill when HBM is short, :54
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import torch
 
 from .. import _lib
+from ..attn_hub.retroinfer_attn import _status_word
 from .cache import KV_Cache
 
 
@@ -62,7 +65,9 @@ class flash_attn_cache(KV_Cache):
     def _one_launch(self, keys, key_states, value_states) -> bool:
         """Whether the rows can be appended by one kernel for both tensors: what a decode step hands over, 16-bit rows of
         the cache's own type, dense and aligned, on the current device, and rows that fit (a full cache is
-        refused by the indexing below).  Six launches of indexing kernels otherwise."""
+        refused by the indexing below).  The lengths are counted on the host here; where they move on without it, as in
+        replays of a CUDA graph, the kernel itself leaves out a row that does not fit, and ``check_prefill_errors`` or the
+        next ``decode_full_flash_attn`` says so.  Six launches of indexing kernels otherwise."""
         shape, dev, n = (self.batch_size, 1, self.kv_head, self.head_dim), keys.device, self.valid_length
         if not (keys.is_cuda and dev.index == torch.cuda.current_device() and n.device == dev and n.dtype == torch.int32
                 and n.is_contiguous() and self._longest is not None and self._longest < self.max_length):
@@ -78,8 +83,9 @@ class flash_attn_cache(KV_Cache):
         keys, values = self.key_cache[layer_idx], self.value_cache[layer_idx]
         if self._one_launch(keys, key_states, value_states):
             _lib.check(_lib.lib.ri_dense_append(key_states.data_ptr(), value_states.data_ptr(), keys.data_ptr(),
-                                                values.data_ptr(), self.valid_length.data_ptr(), self.batch_size,
-                                                self.kv_head, self.max_length, _lib.current_stream()), "ri_dense_append")
+                                                values.data_ptr(), self.valid_length.data_ptr(),
+                                                C.addressof(_status_word(keys.device)), self.batch_size, self.kv_head,
+                                                self.max_length, _lib.current_stream()), "ri_dense_append")
         else:
             pos = self.valid_length.to(keys.device).long()
             keys[self._rows.to(pos.device), :, pos] = key_states[:, 0]

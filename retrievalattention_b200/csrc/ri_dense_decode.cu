@@ -363,14 +363,17 @@ __global__ void __launch_bounds__(kCombineThreads) dense_combine_kernel(DenseArg
 }
 
 __global__ void __launch_bounds__(256) dense_append_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, uint4* keys,
-                                                           uint4* values, const int32_t* __restrict__ valid, int hk, int pieces,
-                                                           int64_t stride) {
+                                                           uint4* values, const int32_t* __restrict__ valid, int* error_flag,
+                                                           int hk, int pieces, int64_t stride) {
   ri_pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;      // one 16-byte piece of K and of V
   if (i >= pieces) return;
   const int g = i >> 4;
   const int64_t row = valid[g / hk];
-  if (row < 0 || row >= stride) return;
+  if (row < 0 || row >= stride) {      // a replayed graph may come here: the host does not see the lengths
+    if ((i & 15) == 0) *error_flag = RI_STATUS_CACHE_FULL;
+    return;
+  }
   keys[(g * stride + row) * 16 + (i & 15)] = k[i];
   values[(g * stride + row) * 16 + (i & 15)] = v[i];
 }
@@ -442,15 +445,15 @@ extern "C" int ri_dense_decode(const void* d_q, const void* d_k, const void* d_v
 }
 
 extern "C" int ri_dense_append(const void* d_k, const void* d_v, void* d_keys, void* d_values, const int32_t* d_valid_length,
-                               int32_t batch, int32_t kv_heads, int64_t rows_stride, void* stream) {
-  RI_REQUIRE(d_k && d_v && d_keys && d_values && d_valid_length, "ri_dense_append: null pointer");
+                               int32_t* d_error, int32_t batch, int32_t kv_heads, int64_t rows_stride, void* stream) {
+  RI_REQUIRE(d_k && d_v && d_keys && d_values && d_valid_length && d_error, "ri_dense_append: null pointer");
   RI_REQUIRE(batch >= 1 && kv_heads >= 1 && (int64_t)batch * kv_heads < (1ll << 26) && rows_stride >= 1, "ri_dense_append: bad sizes");
   RI_REQUIRE(((uintptr_t)d_k | (uintptr_t)d_v | (uintptr_t)d_keys | (uintptr_t)d_values) % 16 == 0,
              "ri_dense_append: tensors must be 16-byte aligned");
   const int pieces = batch * kv_heads * 16;
   RI_CUDA_OK(ri_launch_pdl_id(11, ri_wave::dense_append_kernel, dim3((pieces + 255) / 256), dim3(256), 0,
                               static_cast<cudaStream_t>(stream), static_cast<const uint4*>(d_k), static_cast<const uint4*>(d_v),
-                              static_cast<uint4*>(d_keys), static_cast<uint4*>(d_values), d_valid_length, kv_heads, pieces,
-                              rows_stride));
+                              static_cast<uint4*>(d_keys), static_cast<uint4*>(d_values), d_valid_length, d_error, kv_heads,
+                              pieces, rows_stride));
   return RI_OK;
 }

@@ -128,3 +128,35 @@ def test_dense_append_forms(form):
         for b, start in enumerate((0, 7, 3)):
             old[b, :, n - start] = rows[b if rows.shape[0] > 1 else 0, 0]
         assert torch.equal(old, now)
+
+
+def test_rows_behind_the_end_of_the_cache_are_reported():
+    """Where the lengths move on without the host, in replays of a captured step, a row that no longer fits is left out and
+    said to be."""
+    from retrievalattention_b200.attn_hub import decode_full_flash_attn, retroinfer_attn as ra
+    from retrievalattention_b200.cache_hub import flash_attn_cache
+
+    n, hk = 40, 2
+    cache = flash_attn_cache([0, 1], 1, 2, n + 2, hk, 8, 128, torch.bfloat16, {"0": "cuda:0"}, 1, 8)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    mk = lambda b, s, h: torch.randn((b, s, h, 128), generator=gen, device="cuda").bfloat16()      # noqa: E731
+    for b in range(2):
+        cache.prefill_update_kv_cache(None, mk(1, n, hk), mk(1, n, hk), 0, b)
+    k, v, q = mk(2, 1, hk), mk(2, 1, hk), mk(2, 1, 8)
+    assert cache._one_launch(cache.key_cache[0], k, v)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = decode_full_flash_attn(q, *cache.decode_update_kv_cache(k, v, 0), 0, cache)
+    for step in range(2):
+        graph.replay()
+        ra.check_prefill_errors()
+        assert cache.valid_length.tolist() == [n + step + 1, n + step] and torch.isfinite(out.float()).all()
+    assert torch.equal(cache.key_cache[0][0, :, n + 1], k[0, 0]) and torch.equal(cache.value_cache[0][1, :, n], v[1, 0])
+    before = [t.clone() for t in (cache.key_cache[0], cache.value_cache[0])]
+    graph.replay()                                  # the first request is full, the second has room for one more row
+    with pytest.raises(RuntimeError, match="did not fit"):
+        ra.check_prefill_errors()
+    ra.check_prefill_errors()
+    for old, now, rows in zip(before, (cache.key_cache[0], cache.value_cache[0]), (k, v)):
+        old[1, :, n + 1] = rows[1, 0]
+        assert torch.equal(old, now)
