@@ -62,16 +62,20 @@ class flash_attn_cache(KV_Cache):
         """The reference waits for its side-stream copy (:129-130); the copy above is in stream order."""
         return None
 
-    def _one_launch(self, keys, key_states, value_states) -> bool:
+    def _one_launch(self, keys, key_states, value_states, values=None) -> bool:
         """Whether the rows can be appended by one kernel for both tensors: what a decode step hands over, 16-bit rows of
-        the cache's own type, dense and aligned, on the current device, and rows that fit (a full cache is
-        refused by the indexing below).  The lengths are counted on the host here; where they move on without it, as in
+        the cache's own type, dense and aligned, on the current device, into tensors as they were made (a caller may have
+        put others in their place), and rows that fit (a full cache is refused by the indexing below).  The lengths are counted on the host here; where they move on without it, as in
         replays of a CUDA graph, the kernel itself leaves out a row that does not fit, and ``check_prefill_errors`` or the
         next ``decode_full_flash_attn`` says so.  Six launches of indexing kernels otherwise."""
         shape, dev, n = (self.batch_size, 1, self.kv_head, self.head_dim), keys.device, self.valid_length
         if not (keys.is_cuda and dev.index == torch.cuda.current_device() and n.device == dev and n.dtype == torch.int32
-                and n.is_contiguous() and self._longest is not None and self._longest < self.max_length):
+                and n.is_contiguous() and n.shape == (self.batch_size,) and self._longest is not None and self._longest < self.max_length):
             return False
+        for x in (keys, keys if values is None else values):
+            if not (x.shape == (self.batch_size, self.kv_head, self.max_length, self.head_dim) and x.dtype == keys.dtype
+                    and x.device == dev and x.is_contiguous() and x.data_ptr() % 16 == 0 and not x.requires_grad):
+                return False
         for x in (key_states, value_states):
             if not (x.shape == shape and x.dtype == keys.dtype and x.element_size() == 2 and x.device == dev
                     and x.is_contiguous() and x.data_ptr() % 16 == 0 and not x.requires_grad):
@@ -81,7 +85,7 @@ class flash_attn_cache(KV_Cache):
     def decode_update_kv_cache(self, key_states, value_states, layer_idx):
         """Append one token per request (:133-151).  key/value_states: [batch, 1, kv_heads, head_dim]."""
         keys, values = self.key_cache[layer_idx], self.value_cache[layer_idx]
-        if self._one_launch(keys, key_states, value_states):
+        if self._one_launch(keys, key_states, value_states, values):
             _lib.check(_lib.lib.ri_dense_append(key_states.data_ptr(), value_states.data_ptr(), keys.data_ptr(),
                                                 values.data_ptr(), self.valid_length.data_ptr(),
                                                 C.addressof(_status_word(keys.device)), self.batch_size, self.kv_head,

@@ -160,3 +160,32 @@ def test_rows_behind_the_end_of_the_cache_are_reported():
     for old, now, rows in zip(before, (cache.key_cache[0], cache.value_cache[0]), (k, v)):
         old[1, :, n + 1] = rows[1, 0]
         assert torch.equal(old, now)
+
+
+@pytest.mark.parametrize("form", ["longer", "strided", "other_type"])
+def test_dense_append_into_tensors_put_in_place_of_the_cache(form):
+    from retrievalattention_b200.cache_hub import flash_attn_cache
+
+    n, hk = 40, 2
+    cache = flash_attn_cache([0, 7], 2, 2, n + 2, hk, 8, 128, torch.bfloat16, {"0": "cuda:0", "1": "cuda:0"}, 1, 8)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    mk = lambda s: torch.randn((2, s, hk, 128), generator=gen, device="cuda").bfloat16()      # noqa: E731
+    for b in range(2):
+        cache.prefill_update_kv_cache(None, mk(n)[:1], mk(n)[:1], 0, b)
+    for tensors in (cache.key_cache, cache.value_cache):
+        old = tensors[0]
+        if form == "longer":
+            tensors[0] = torch.cat((old, torch.zeros_like(old)), dim=2)
+        elif form == "strided":
+            tensors[0] = torch.cat((old, old), dim=3)[..., :128]
+    if form == "other_type":
+        cache.value_cache[0] = cache.value_cache[0].half()
+    k, v = mk(1), mk(1)
+    v = v.to(cache.value_cache[0].dtype)
+    assert not cache._one_launch(cache.key_cache[0], k, v, cache.value_cache[0])
+    before = [cache.key_cache[0].clone(), cache.value_cache[0].clone()]
+    got = cache.decode_update_kv_cache(k, v, 0)
+    for old, now, rows in zip(before, got, (k, v)):
+        for b, start in enumerate((0, 7)):
+            old[b, :, n - start] = rows[b, 0]
+        assert torch.equal(old, now)
