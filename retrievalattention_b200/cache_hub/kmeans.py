@@ -80,11 +80,17 @@ def build_prompt_index(keys: torch.Tensor, values: torch.Tensor, num_segments: i
     assert keys.is_contiguous() and values.is_contiguous() and values.dtype == keys.dtype
     tokens, z, d = keys.shape
     dt, n, c = keys.dtype, tokens - sink - recent, out["centroids"].shape[1]
-    assert all(t.device == keys.device for t in (values, *out.values())), "prompt and index lie on one GPU"
-    assert out["centroids"].shape == out["value_sum"].shape == (z, c, d) and out["cluster_offset"].shape == (z, c + 1)
-    assert all(out[name].shape == (z, c) for name in ("cluster_size", "cluster_count", "empty"))
-    assert all(out[name].dtype == dt for name in ("centroids", "value_sum", "cluster_size"))
-    assert out["cluster_count"].dtype == out["cluster_offset"].dtype == torch.int32 and out["empty"].dtype == torch.bool
+    rows, steady = out["keys"].shape[1], out["steady_keys"].shape[1]
+    gpu = keys.get_device()
+    assert values.get_device() == gpu and rows >= n and steady >= sink + recent
+    at = {}                  # addresses of the results, each of the form the kernels write
+    for name, shape, kind in (("centroids", (z, c, d), dt), ("value_sum", (z, c, d), dt), ("cluster_size", (z, c), dt),
+                              ("cluster_count", (z, c), torch.int32), ("cluster_offset", (z, c + 1), torch.int32),
+                              ("empty", (z, c), torch.bool), ("keys", (z, rows, d), dt), ("values", (z, rows, d), dt),
+                              ("steady_keys", (z, steady, d), dt), ("steady_values", (z, steady, d), dt)):
+        x = out[name]
+        assert x.shape == shape and x.dtype is kind and x.get_device() == gpu and x.is_contiguous(), name
+        at[name] = x.data_ptr()
     p, q = _lib.KMeans(), _lib.KMeansPrompt()
     p.groups, p.n_tokens, p.n_centroids, p.n_segments, p.n_iters = z, n, c, num_segments, num_iters
     p.dtype, p.center = _lib.dtype_code(dt), 1
@@ -95,18 +101,10 @@ def build_prompt_index(keys: torch.Tensor, values: torch.Tensor, num_segments: i
     error = torch.empty((1,), dtype=torch.int32, device=keys.device)
     p.d_keys, p.d_values, p.d_scratch, p.d_error = keys.data_ptr(), values.data_ptr(), scratch.data_ptr(), error.data_ptr()
     for name in ("centroids", "value_sum", "cluster_size", "cluster_count", "cluster_offset"):
-        assert out[name].is_contiguous()
-        setattr(p, "d_" + name, out[name].data_ptr())
-    for name in ("keys", "values", "steady_keys", "steady_values"):
-        assert out[name].is_contiguous() and out[name].dtype == dt and out[name].shape == (z, out[name].shape[1], d)
-    assert out["keys"].shape == out["values"].shape and out["keys"].shape[1] >= n
-    assert out["steady_keys"].shape == out["steady_values"].shape and out["empty"].is_contiguous()
-    assert out["steady_keys"].shape[1] >= sink + recent
-    p.d_keys_out, p.d_values_out = out["keys"].data_ptr(), out["values"].data_ptr()
-    q.n_sink, q.n_recent, q.out_group_rows = sink, recent, out["keys"].shape[1]
-    q.steady_group_rows = out["steady_keys"].shape[1]
-    q.d_steady_keys, q.d_steady_values = out["steady_keys"].data_ptr(), out["steady_values"].data_ptr()
-    q.d_empty = out["empty"].data_ptr()
+        setattr(p, "d_" + name, at[name])
+    p.d_keys_out, p.d_values_out = at["keys"], at["values"]
+    q.n_sink, q.n_recent, q.out_group_rows, q.steady_group_rows = sink, recent, rows, steady
+    q.d_steady_keys, q.d_steady_values, q.d_empty = at["steady_keys"], at["steady_values"], at["empty"]
     _lib.check(_lib.lib.ri_kmeans_build_prompt(C.byref(p), C.byref(q), _lib.current_stream()), "ri_kmeans_build_prompt")
     return error          # the scratch goes back to the allocator, which reuses it in stream order
 
