@@ -90,6 +90,7 @@ class flash_attn_cache(KV_Cache):
                                                 values.data_ptr(), self.valid_length.data_ptr(),
                                                 C.addressof(_status_word(keys.device)), self.batch_size, self.kv_head,
                                                 self.max_length, _lib.current_stream()), "ri_dense_append")
+            torch.autograd.graph.increment_version((keys, values))      # as the indexing form does by itself
         else:
             pos = self.valid_length.to(keys.device).long()
             keys[self._rows.to(pos.device), :, pos] = key_states[:, 0]

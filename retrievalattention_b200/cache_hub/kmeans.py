@@ -106,6 +106,7 @@ def build_prompt_index(keys: torch.Tensor, values: torch.Tensor, num_segments: i
     q.n_sink, q.n_recent, q.out_group_rows, q.steady_group_rows = sink, recent, rows, steady
     q.d_steady_keys, q.d_steady_values, q.d_empty = at["steady_keys"], at["steady_values"], at["empty"]
     _lib.check(_lib.lib.ri_kmeans_build_prompt(C.byref(p), C.byref(q), _lib.current_stream()), "ri_kmeans_build_prompt")
+    torch.autograd.graph.increment_version(tuple(out.values()))      # written in place, as a copy into them would say
     return error          # the scratch goes back to the allocator, which reuses it in stream order
 
 

@@ -189,3 +189,34 @@ def test_dense_append_into_tensors_put_in_place_of_the_cache(form):
         for b, start in enumerate((0, 7)):
             old[b, :, n - start] = rows[b, 0]
         assert torch.equal(old, now)
+
+
+def test_rows_written_by_kernels_count_as_changes_in_place():
+    """A backward pass that saved a cache tensor must not run on rows written since (autograd compares versions)."""
+    from retrievalattention_b200.cache_hub import flash_attn_cache, retroinfer_cache
+
+    n, hk = 1024 + 68, 2
+    dense = flash_attn_cache([0], 2, 1, n + 2, hk, 8, 128, torch.bfloat16, {"0": "cuda:0", "1": "cuda:0"}, 1, 8)
+    cfg = generate_config(n, 0.05, 0.2, n_segments=1)
+    wave = retroinfer_cache([0], 1, 1, n + 6, hk, 8, 128, torch.bfloat16, {"0": "cuda:0"}, 6, num_gpus=1, model_size=8,
+                            **cfg.as_kwargs())
+    k, v = make_kv(hk, n, 128, seed=3, device="cuda")
+    dense.prefill_update_kv_cache(None, k, v, 0, 0)
+    wave_tensors = [getattr(wave, name)[0] for name in ("centroids", "value_sum", "cluster_size", "cluster_count", "cluster_offset",
+                                                        "centroids_mask", "list_keys", "list_values", "steady_zone_keys",
+                                                        "steady_zone_values")]
+    before = [t._version for t in wave_tensors]
+    wave.prefill_update_kv_cache(None, k, v, 0, 0)
+    assert all(t._version > old for t, old in zip(wave_tensors, before))
+    weight = torch.ones(128, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    loss = (dense.key_cache[0] * weight).sum()
+    row = k[:, :1].contiguous()
+    assert dense._one_launch(dense.key_cache[0], row, row, dense.value_cache[0])
+    dense.decode_update_kv_cache(row, row, 0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()
+    with torch.inference_mode():                    # tensors made there keep no version
+        other = flash_attn_cache([0], 2, 1, n + 2, hk, 8, 128, torch.bfloat16, {"0": "cuda:0", "1": "cuda:0"}, 1, 8)
+        other.prefill_update_kv_cache(None, k, v, 0, 0)
+        other.decode_update_kv_cache(row, row, 0)
+        assert torch.equal(other.key_cache[0][0, :, n], row[0, 0])
