@@ -136,8 +136,9 @@ constexpr float RI_LOG2E = 1.4426950408889634f;
 // on: on one GPU it makes no difference to the decode kernel, between several GPUs the wait
 // kernel's launch hides behind the decode kernel and the next decode kernel's behind the wait.
 // The element-wise kernels of the decode layer (id 8) are on: their launch hides behind the library GEMM
-// in front of them (measured: 2 % of the whole model step), and so are those of the clustering build (ids 9, 10)
-// and of the dense cache (id 11: append, attention, merge).
+// in front of them (measured: 2 % of the whole model step), and so are those of the clustering build (id 9: sort and
+// update, id 10: assignment) and of the dense cache (id 11: append, attention, merge).  RI_PDL_MASK (a decimal number, one
+// bit per id) replaces the default.
 __device__ __forceinline__ void ri_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void ri_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void ri_pdl_enter() {
@@ -145,19 +146,36 @@ __device__ __forceinline__ void ri_pdl_enter() {
   ri_pdl_wait();
 }
 
+inline int ri_pdl_mask() {
+  static const int mask = getenv("RI_PDL_MASK") ? atoi(getenv("RI_PDL_MASK")) : 0xf63;
+  return mask;
+}
+
+// cluster: CTAs per cluster along x, for kernels that do not state it themselves (0: as the kernel says).
 template <typename... KArgs, typename... Args>
-inline cudaError_t ri_launch_pdl_id(int id, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                 Args... args) {
+inline cudaError_t ri_launch_pdl_cluster(int id, int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                         cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  static const int mask = getenv("RI_PDL_MASK") ? atoi(getenv("RI_PDL_MASK")) : 0xf63;   // per-kernel switch
+  cudaLaunchAttribute attr[2];
+  if (cluster > 0) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  if ((ri_pdl_mask() >> id) & 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = (mask >> id) & 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t ri_launch_pdl_id(int id, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    Args... args) {
+  return ri_launch_pdl_cluster(id, 0, kernel, grid, block, smem, stream, args...);
 }

@@ -862,21 +862,7 @@ int launch_bucket(BucketArgs a, const BucketPlan& p, int problems, cudaStream_t 
   a.range = ((a.n_tok + p.cl * p.workers - 1) / (p.cl * p.workers) + 31) & ~31;
   if (p.smem > 48 * 1024)
     RI_CUDA_OK(cudaFuncSetAttribute(kmeans_bucket_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(problems * CL);
-  cfg.blockDim = dim3(p.workers * 32);
-  cfg.dynamicSmemBytes = p.smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CL;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  RI_CUDA_OK(cudaLaunchKernelEx(&cfg, kmeans_bucket_kernel<CL>, a));
+  RI_CUDA_OK(ri_launch_pdl_cluster(9, CL, kmeans_bucket_kernel<CL>, dim3(problems * CL), dim3(p.workers * 32), p.smem, s, a));
   return RI_OK;
 }
 

@@ -58,10 +58,17 @@ def test_the_check_sees_a_missing_wait():
 
 def test_programmatically_launched_kernels_wait_on_every_way_out():
     texts = sources()
-    calls = r"(?:ri_launch_pdl_id\(\s*\w+|cudaLaunchKernelEx\(\s*&\w+),\s*(?:\w+::)*(\w+_kernel)\b"
+    calls = r"(?:ri_launch_pdl_id\(\s*\w+|ri_launch_pdl_cluster\(\s*\w+,\s*\w+|cudaLaunchKernelEx\(\s*&\w+),\s*(?:\w+::)*(\w+_kernel)\b"
     bodies = {n: b for t in texts for n, b in kernel_bodies(t)}
     launched = {n for t in texts for n in re.findall(calls, t)} | {n for n, b in bodies.items() if "ri_pdl_" in b}
     assert {"kmeans_assign_wide_kernel", "kmeans_assign_resident_kernel", "kmeans_bucket_kernel", "kmeans_update_kernel",
             "dense_decode_kernel", "dense_combine_kernel", "dense_append_kernel", "rmsnorm_kernel"} <= launched
     found = {n: unguarded_exits(bodies[n]) for n in sorted(launched)}
     assert not any(found.values()), found
+
+
+def test_every_programmatic_launch_asks_the_switch():
+    """RI_PDL_MASK covers them all: the attribute is set in one place, behind the mask."""
+    uses = [t for t in sources() if "cudaLaunchAttributeProgrammaticStreamSerialization" in t]
+    assert len(uses) == 1 and uses[0].count("cudaLaunchAttributeProgrammaticStreamSerialization") == 1
+    assert re.search(r"if \(\(ri_pdl_mask\(\) >> id\) & 1\) \{[^}]*cudaLaunchAttributeProgrammaticStreamSerialization", uses[0])
