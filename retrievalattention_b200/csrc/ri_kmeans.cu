@@ -6,8 +6,9 @@
 //            N = 128 centroids, K = 128 channels as 8 x K16) with operands staged by TMA
 //            (128-byte swizzle) and fp32 accumulators in TMEM; a warp-specialised CTA
 //            (TMA producer / MMA issuer / epilogue warps) overlaps the running arg-max of one
-//            accumulator buffer with the MMAs into the other: 256 tokens per block, persistent
-//            over blocks, eight epilogue warps.
+//            accumulator buffer with the MMAs into the other: blocks of 256 tokens (tiles of 128
+//            where a problem's centroids stay in shared memory, N = 256 there), persistent CTAs
+//            over the blocks of all problems, eight epilogue warps.
 //   bucket   stable counting sort of the tokens of a problem by cluster: counts, offsets and
 //            the member list in ascending token order (deterministic, no global atomics).
 //   update   a warp per run of clusters sums their member rows in list order (fp32), forms the means,
@@ -47,14 +48,14 @@ struct AssignArgs {
 };
 
 // ---- assign kernel --------------------------------------------------------------------------------
-// A CTA works through consecutive 256-token blocks of one problem.  Per block
+// A persistent CTA works through consecutive 256-token blocks of the flat sequence over all problems.  Per block
 // two 128-row token tiles (A, double-buffered per block) meet every centroid tile (B, streamed
 // through three stages) in two MMAs, so a centroid tile fetched into shared memory serves 256 tokens
-// and the CTA's set-up is paid once for many blocks; the accumulators fill all 512 TMEM columns
+// and the CTA's set-up is paid once for all its blocks; the accumulators fill all 512 TMEM columns
 // (2 buffers x 2 token tiles x 128 centroids).  Ten warps: TMA producer, MMA issuer, and eight
 // epilogue warps (four per token tile, one per TMEM lane quarter) that keep the running arg-max
-// of their 32 tokens: per 32 columns a max tree, then the first column equal to the max (ties ->
-// lowest index, the rule of torch.argmax), so nothing in the epilogue is a serial chain.
+// of their 32 tokens: per 32 columns a max tree, the values of the winning block kept; once per token, behind the last tile,
+// the first kept value equal to the max gives the column (ties -> lowest index, the rule of torch.argmax).
 // Every mbarrier wait has a time and an iteration limit; on expiry the CTA records where it gave up, releases its
 // TMEM and returns.
 constexpr int kEpilogueWarps = 8;
@@ -80,18 +81,6 @@ __device__ __forceinline__ void unit_share(const WideArgs& w, int& lo, int& hi) 
 // first token row (of all groups' rows) of a problem
 __device__ __forceinline__ int64_t problem_row(const AssignArgs& a, int problem) {
   return (int64_t)(problem / a.seg_per_group) * a.group_stride + (int64_t)(problem % a.seg_per_group) * a.n_tok;
-}
-
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));   // three-input maximum (sm_100)
-  return d;
-}
-
-__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
 }
 
 // Running arg-max of a token over blocks of 32 accumulator columns.  Which column of a block is the maximum is not looked
@@ -334,7 +323,7 @@ kmeans_assign_wide_kernel(const __grid_constant__ CUtensorMap map_keys, const __
 
 // ---- assign kernel, centroids resident ----------------------------------------------------------------
 // Problems of at most 512 centroids (the segmented iterations of the reference's schedule, the re-index build): the
-// problem's centroid tiles (up to four, 128 KB) are fetched ONCE per CTA and stay in shared memory, and only the
+// problem's centroid tiles (up to four, 128 KB) are fetched once per CTA and problem and stay in shared memory, and only the
 // tokens stream, as single 128-row tiles through a three-slot ring (the wide kernel above re-fetches the centroid
 // tiles for every 256 tokens).  Per token tile two rounds of two centroid tiles each (accumulators: 2 buffers x
 // 2 centroid tiles x 128 columns); the eight epilogue warps are four lane quarters x the two centroid tiles of a
@@ -843,11 +832,12 @@ __global__ void __launch_bounds__(512) kmeans_bucket_kernel(BucketArgs a) {
 // Launch plan of the bucket pass: CTAs per problem, warps per CTA, tokens per warp.
 struct BucketPlan { int cl, workers; size_t smem; };
 
-BucketPlan bucket_plan(int problems, int n_tok, int n_cen) {
+BucketPlan bucket_plan(int problems, int n_tok, int n_cen, int sms) {
   BucketPlan p;
-  // as many CTAs per problem as the chip has room for beside the other problems (two CTAs per SM), up to 8
+  // up to 8 CTAs per problem, as long as all problems together have at most two per SM (with up to about 2800 clusters their
+  // tables let two be resident; with more, the larger launches take two rounds)
   p.cl = 8;
-  while (p.cl > 1 && p.cl * problems > 2 * 148) p.cl >>= 1;
+  while (p.cl > 1 && p.cl * problems > 2 * sms) p.cl >>= 1;
   // 16-bit counts and packed sums: a CTA's tokens stay below 65536
   while (p.cl < 8 && (n_tok + p.cl - 1) / p.cl > 60000) p.cl <<= 1;
   p.workers = 16;
@@ -872,7 +862,6 @@ struct UpdateArgs {
   const uint2* values;       // LAST: V rows (value sums + copy)
   RowPlace src;              // place of a row of `rows` and `values`
   const int32_t* order;
-  const int32_t* count;
   const int32_t* offset;
   uint2* centroids;          // [problems, n_cen, 128] in/out (centred)
   uint2* out_centroids;      // optional final: centroid + mean
@@ -1168,7 +1157,7 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const Place& pl, const void*
     ba.count = last && p->d_cluster_count ? p->d_cluster_count : count_work;
     ba.offset = last && p->d_cluster_offset ? p->d_cluster_offset : offset_work;
     ba.n_tok = n_tok; ba.n_cen = n_cen; ba.seg_per_group = seg; ba.group_stride = N;
-    const BucketPlan bp = bucket_plan(problems, n_tok, n_cen);
+    const BucketPlan bp = bucket_plan(problems, n_tok, n_cen, sms);
     if ((n_tok + bp.cl - 1) / bp.cl <= 60000 && bp.smem <= 200 * 1024) {
       rc = bp.cl == 8 ? launch_bucket<8>(ba, bp, problems, s) : bp.cl == 4 ? launch_bucket<4>(ba, bp, problems, s)
          : bp.cl == 2 ? launch_bucket<2>(ba, bp, problems, s) : launch_bucket<1>(ba, bp, problems, s);
@@ -1188,7 +1177,7 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const Place& pl, const void*
     UpdateArgs ua = {};
     ua.rows = static_cast<const uint2*>(centred);
     ua.src = {N, 1};
-    ua.order = order; ua.count = ba.count; ua.offset = ba.offset;
+    ua.order = order; ua.offset = ba.offset;
     ua.centroids = static_cast<uint2*>(cent);
     ua.n_tok = n_tok; ua.n_cen = n_cen; ua.seg_per_group = seg; ua.normalize = last ? 0 : 1; ua.group_stride = N;
     if (last) {
@@ -1210,7 +1199,7 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const Place& pl, const void*
     ua.n_clusters = n_cen * problems;
     // clusters per warp: a longer run of rows hides more latency, but enough warps for a few rounds of the chip
     int cpw = 8;
-    while (cpw > 1 && ua.n_clusters / cpw < 148 * 96) cpw >>= 1;
+    while (cpw > 1 && ua.n_clusters / cpw < sms * 96) cpw >>= 1;
     ua.clusters_per_warp = cpw;
     constexpr int per_cta = kUpdateThreads / 32;
     const dim3 ugrid((ua.n_clusters / cpw + per_cta - 1) / per_cta);

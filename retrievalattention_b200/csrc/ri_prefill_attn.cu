@@ -96,28 +96,6 @@ __device__ __forceinline__ Item get_item(const AttnArgs& a, int index) {
 }
 
 // ---- softmax arithmetic ---------------------------------------------------------------------------------------------
-// Pairs of floats in one 64-bit register: sm_100 multiplies and adds them two at a time.
-__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ void unpack_f2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));   // three-input maximum (sm_100)
-  return d;
-}
 __device__ __forceinline__ float ex2(float x) {       // 2^x; results below 2^-126 become 0
   float d;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(x));
