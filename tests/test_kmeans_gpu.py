@@ -186,13 +186,13 @@ def test_rejects_bad_shapes():
 
 
 # sizes where the sort, the update and the assignment change form: one problem per 8, 4, 2, 1 CTAs of the sort, more tokens
-# than its 16-bit counts take (the one-CTA form), one partial centroid tile, 512 centroids (resident) and 544 (streamed),
+# than its 16-bit counts take and more clusters than its tables hold (the one-CTA form), one partial centroid tile, 512 centroids (resident) and 544 (streamed),
 # a prompt whose clustered rows are no multiple of anything.  Everything below is exact: the list is a stable sort of the
 # assignment, and the prompt form is the array form on the same rows.
 @pytest.mark.parametrize("heads,n,c,seg,dtype", [
     (1, 333, 32, 1, torch.bfloat16), (3, 5003, 512, 1, torch.bfloat16), (2, 9001, 544, 1, torch.float16),
     (8, 16411, 1024, 16, torch.bfloat16), (8, 20000, 1024, 8, torch.bfloat16), (5, 20011, 1280, 40, torch.float16),
-    (1, 500009, 96, 1, torch.bfloat16),
+    (1, 500009, 96, 1, torch.bfloat16), (1, 41051, 20512, 1, torch.bfloat16),
 ])
 def test_lists_and_prompt_form(heads, n, c, seg, dtype):
     from retrievalattention_b200.cache_hub.kmeans import build_index, build_prompt_index

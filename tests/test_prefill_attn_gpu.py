@@ -117,6 +117,7 @@ def test_pairs_are_as_accurate_as_two_walks(seq, hq, hk, dtype):
     from retrievalattention_b200.attn_hub import retroinfer_attn as ra
     from retrievalattention_b200.synthetic import make_kv
 
+    assert takes_pairs(1, seq, hq)
     q = torch.randn((1, seq, hq, 128), generator=torch.Generator(device="cuda").manual_seed(17), device="cuda").to(dtype)
     k, v = make_kv(hk, seq, 128, seed=93, device="cuda", dtype=dtype)
     out = ra.retroinfer_prefill_attn(q, k, v, True)
@@ -205,3 +206,37 @@ ra.check_prefill_errors()
 assert torch.equal(out, ra.retroinfer_prefill_attn(q, k, k, True))
 """
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
+
+
+def takes_pairs(batch, seq, hq):
+    """Whether a call has a pair of query tiles for every SM, so that CTAs take pairs (else single tiles, split walks)."""
+    tiles = -(-seq // 128)
+    return (tiles + 1) // 2 * hq * batch >= torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.parametrize("batch,seq,hq,hk,causal,dtype,grows", [
+    (1, 1300, 32, 8, True, torch.float16, False),
+    (3, 900, 28, 4, True, torch.bfloat16, False),       # NaN in the middle request, both neighbours compared
+    (3, 901, 28, 4, False, torch.float16, False),
+    (1, 1536, 32, 1, True, torch.bfloat16, True),       # scores grow along the sequence: accumulators are rescaled
+    (1, 1600, 28, 1, True, torch.float16, True),
+    (1, 8192, 8, 8, True, torch.bfloat16, False),       # a walk of 64 key tiles
+])
+def test_pairs_of_query_tiles(batch, seq, hq, hk, causal, dtype, grows):
+    """Same tolerance as above."""
+    from retrievalattention_b200.attn_hub import retroinfer_attn as ra
+
+    assert takes_pairs(batch, seq, hq)
+    g = torch.Generator(device="cuda").manual_seed(seq)
+    q, k, v = (torch.randn((batch, seq, h, 128), generator=g, device="cuda") for h in (hq, hk, hk))
+    if grows:
+        ramp = torch.linspace(0.2, 6.0, seq, device="cuda")[None, :, None, None]
+        k = k * 0.3 + q[:, :, :hk] * 0.05 * ramp
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    if batch > 2:
+        k[1], v[1] = float("nan"), float("nan")
+    out = ra.retroinfer_prefill_attn(q, k, v, causal)
+    ra.check_prefill_errors()
+    for b in range(0, batch, 2):
+        err = (out[b:b + 1].float() - reference(q[b:b + 1], k[b:b + 1], v[b:b + 1], causal)).abs()
+        assert err.max() <= 2e-2 and err.mean() <= 2e-3, (b, float(err.max()), float(err.mean()))
