@@ -20,9 +20,10 @@
 // K, V, P written) = 1792 clocks against 1024 of tensor work, and the kernel ran at 0.51 of the measured peak.  Two query
 // tiles that share K and V, and P in TMEM, make it 128 KB per tile and query tile; V needs no transposed copy.  While one
 // group's softmax runs, the tensor pipe does the other group's two products.
-// 32 query and 8 key/value heads, causal, bf16: 32768 tokens 9.9 -> 7.1 ms (889 -> 1235 TFLOP/s), 8192 tokens 0.52 ms,
-// 777 tokens 36 -> 19 us.  What bounds it now (ncu, 8192 tokens): each group's chain of scores, softmax and product, 1737
-// clocks per tile and group; tensor pipe 59 % and exponentials 59 % of the time, issue slots 36 %.  Doing a quarter of the
+// 32 query and 8 key/value heads, causal, bf16, 32768 tokens: 9.9 -> 7.3 ms from rest (889 -> 1200 TFLOP/s), 10.7 -> 8.3 ms
+// in a repeated run, which the power limit holds at 1055 TFLOP/s; 8192 tokens 0.48 ms repeated, a call for 777 tokens 53 ->
+// 20.5 us.  What bounds it now (ncu, 8192 tokens): each group's chain of scores, softmax and product, about 1700 clocks per
+// tile and group; tensor pipe 56 % and exponentials 56 % of the active cycles, issue slots 35 %.  Doing a quarter of the
 // exponentials as polynomials on the FMA pipe was slower (1170 TFLOP/s): they are not what the chain waits for.
 // SPLIT: for few query tiles a CTA takes one of them, and its groups take the even and the odd key/value tiles.
 // Every mbarrier wait is bounded; on expiry a CTA records where, releases its TMEM and returns.  The word it is recorded in
