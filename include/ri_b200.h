@@ -169,7 +169,7 @@ typedef struct ri_wave_gather {
                                       entry, after this rank's flags are raised, and when the last rank's flag was seen */
 } ri_wave_gather;
 /* ri_wave_decode_layer plus the stores described above (p->d_out is written too).  Geometries beyond the single
- * decode kernel (more than 8192 centroids, e.g. after a re-index of generated tokens) run the three stage
+ * decode kernel (more than 16384 centroids, e.g. after a re-index of generated tokens) run the three stage
  * kernels, whose attend stage does the stores. */
 int ri_wave_decode_layer_gather(const ri_wave_layer* p, const ri_wave_gather* g, void* stream);
 /* Raise this rank's flags, then wait (bounded) for every rank's. */

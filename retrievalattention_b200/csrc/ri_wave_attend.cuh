@@ -77,19 +77,38 @@ struct AttendArgs {
   const uint16_t* prev_out;   // [G, gs, 128]
   const float* prev_lse;      // [G, gs] natural log
   float* lse_out;             // [G, gs] natural log
+  // rows [G, 128] that stand for row `static_len - 1` of the steady zone (null: the steady zone has its own): the single
+  // kernel stores them there itself, and its other CTAs need not wait for that
+  const uint4* new_k;
+  const uint4* new_v;
 };
 
-template <int DT>
-__device__ __forceinline__ void pv_step(float (&acc)[8][4], const uint4 (&v)[4][2], uint32_t b0, uint32_t b1) {
+// acc += P.V for 16 rows.  b0, b1: this lane's four probabilities in the 16-bit type; TWO: l0, l1 is what that rounding left
+// over, multiplied too.
+template <int DT, bool TWO = false>
+__device__ __forceinline__ void pv_step(float (&acc)[8][4], const uint4 (&v)[4][2], uint32_t b0, uint32_t b1, uint32_t l0 = 0,
+                                        uint32_t l1 = 0) {
 #pragma unroll
-  for (int x = 0; x < 8; ++x) {
-    const int piece = x >> 2, w = x & 3;
-    const uint32_t t0 = (&v[0][piece].x)[w], t1 = (&v[1][piece].x)[w];
-    const uint32_t t2 = (&v[2][piece].x)[w], t3 = (&v[3][piece].x)[w];
-    const uint32_t a0 = __byte_perm(t0, t1, 0x5410), a1 = __byte_perm(t0, t1, 0x7632);
-    const uint32_t a2 = __byte_perm(t2, t3, 0x5410), a3 = __byte_perm(t2, t3, 0x7632);
-    Elem<DT>::mma16816(acc[x], a0, a1, a2, a3, b0, b1);
+  for (int piece = 0; piece < 2; ++piece) {      // four tiles at a time: the second products do not wait for the first ones
+    uint32_t m[4][4];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const uint32_t t0 = (&v[0][piece].x)[w], t1 = (&v[1][piece].x)[w];
+      const uint32_t t2 = (&v[2][piece].x)[w], t3 = (&v[3][piece].x)[w];
+      m[w][0] = __byte_perm(t0, t1, 0x5410); m[w][1] = __byte_perm(t0, t1, 0x7632);
+      m[w][2] = __byte_perm(t2, t3, 0x5410); m[w][3] = __byte_perm(t2, t3, 0x7632);
+      Elem<DT>::mma16816(acc[4 * piece + w], m[w][0], m[w][1], m[w][2], m[w][3], b0, b1);
+    }
+    if (TWO)
+#pragma unroll
+      for (int w = 0; w < 4; ++w) Elem<DT>::mma16816(acc[4 * piece + w], m[w][0], m[w][1], m[w][2], m[w][3], l0, l1);
   }
+}
+// Two probabilities in the 16-bit type, and (second word) what the rounding left over.
+template <int DT>
+__device__ __forceinline__ uint2 split2(float p0, float p1) {
+  const uint32_t hi = Elem<DT>::pack2(p0, p1);
+  return make_uint2(hi, Elem<DT>::pack2(p0 - Elem<DT>::from_bits((uint16_t)(hi & 0xffffu)), p1 - Elem<DT>::from_bits((uint16_t)(hi >> 16))));
 }
 
 struct RowIds { int k[2]; int v[4]; };   // >= 0: row of the KV store / cluster id; < 0: steady row -1-id
@@ -97,8 +116,8 @@ struct RowIds { int k[2]; int v[4]; };   // >= 0: row of the KV store / cluster 
 // Shared-memory lists of the single-kernel path (LOCAL mode of attend_group): this CTA's own estimation
 // entries and its range of the group's exact steps, the retrieved rows given by the kept clusters.
 struct LocalLists {
-  const uint16_t* est_idx;   // [n_est] centroid index inside this CTA's slice, ascending
-  const float* est_wt;       // [n_est] weight (cluster size)
+  const uint32_t* est;       // [n_est] centroid index inside this CTA's slice, ascending; above it the weight (cluster size) in
+                             // the 16-bit type
   const float* est_sc;       // [gs][cap] log2-domain scores
   int cap, n_est, slice_lo;
   const uint32_t* dstart;    // [keep + 1] first position of each kept cluster in the retrieved-row list; [keep] = total
@@ -117,31 +136,24 @@ __device__ __forceinline__ void issue_value_sums(const uint4* value_sum, int64_t
   }
 }
 
-// One group's attention by one cluster of CPG CTAs of WARPS warps each (CTA `cl` of it).  `ring`:
-// WARPS * kStages * kStageBytes of 16-byte aligned dynamic shared memory.  `n_exact_known` >= 0: the group's retrieved-row count, when the caller has it at
-// hand (otherwise it is read from a.n_exact).  Ends with a cluster barrier after the last remote read, so the shared
-// memory may be reused (or the CTA may exit) when it returns.
-template <int DT, bool LOCAL = false, int WARPS = 4, int CPG = kAttendCluster>
-__device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, const int cl, uint8_t* ring,
-                                             const LocalLists* ll = nullptr) {
-  __shared__ float sm_m[WARPS][kMaxHeads], sm_l[WARPS][kMaxHeads];
-  __shared__ float cta_m[kMaxHeads], cta_l[kMaxHeads];   // this CTA's partial result: (max, sum) here, O in the ring
-  float (*cta_o)[RI_HEAD_DIM] = reinterpret_cast<float (*)[RI_HEAD_DIM]>(ring + WARPS * kStageBytes);
+// What a warp has gathered over its steps: heads 2t and 2t+1 of the accumulator (see pv_step), maximum (log2 domain) and
+// this lane's share of the sum of head r.
+struct Partial { float acc[8][4]; float m, l; };
 
+// The steps of one group's attention that fall to this warp; CTA `cl` of `cpg` CTAs of WARPS warps each.  `ring`:
+// WARPS * STAGES * kStageBytes of 16-byte aligned dynamic shared memory, free for other use when every warp of the CTA has
+// returned.  static_len: rows of the steady zone; te: those and the retrieved rows.
+template <int DT, bool LOCAL, int WARPS, int STAGES>
+__device__ __forceinline__ void attend_steps(const AttendArgs& a, const int g, const int cl, const int cpg, const int static_len,
+                                             const int te, uint8_t* ring, const LocalLists* ll, Partial& part) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r = lane >> 2, t = lane & 3;
   const int gs = a.gs, es = LOCAL ? (ll->n_est + 15) / 16 : a.e_steps;
-  const int static_len = a.static_len ? *a.static_len : 0;   // null: the exact rows already contain the steady zone
-  cg::cluster_group cluster = cg::this_cluster();
-  constexpr int cpg = CPG;                               // CTAs per group
-  constexpr int kThreads = WARPS * 32;
   // ring: stage-major, slot (stage, warp) at (stage * WARPS + warp) * kStageBytes
   const uint32_t my_ring = (uint32_t)__cvta_generic_to_shared(ring) + warp * kStageBytes + lane * 16;
   const uint8_t* my_ring_ptr = ring + warp * kStageBytes + lane * 16;
   constexpr int kStageStride = WARPS * kStageBytes;
-  auto warp_o = [&](int w) { return reinterpret_cast<float*>(ring + w * kStageBytes); };   // stage 0 of warp w
-
-  const int te = static_len + (LOCAL ? ll->n_rows : __ldcg(a.n_exact + g));           // steady + retrieved rows
+  const int new_row = a.new_k != nullptr ? static_len - 1 : -1;
   // The step sequence this CTA's warps share: LOCAL: its own estimation steps, then its exact steps
   // [x_lo, x_hi); otherwise the whole group's estimation steps, then all exact steps, shared by all 32 warps.
   const int x_first = LOCAL ? ll->x_lo : 0;
@@ -211,7 +223,7 @@ __device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, c
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = min(base + tt[i], last);
-      if (est) id.v[i] = LOCAL ? ll->slice_lo + (int)ll->est_idx[row] : __ldcg(a.est_ids + (int64_t)g * a.e_pad + row);
+      if (est) id.v[i] = LOCAL ? ll->slice_lo + (int)(ll->est[row] & 0xffffu) : __ldcg(a.est_ids + (int64_t)g * a.e_pad + row);
       else id.v[i] = row < static_len ? -1 - row : (a.rows ? __ldcg(a.rows + (int64_t)g * a.max_rows + row - static_len) : row - static_len);
     }
 #pragma unroll
@@ -246,16 +258,16 @@ __device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, c
 #pragma unroll
       for (int jj = 0; jj < 2; ++jj) {
         const int x = id.k[jj];
-        const uint4* p = x < 0 ? a.steady_k + ((int64_t)g * a.steady_stride + (-1 - x)) * 16
-                               : a.keys + ((int64_t)g * a.N + x) * 16;
+        const uint4* p = x >= 0 ? a.keys + ((int64_t)g * a.N + x) * 16
+                       : -1 - x == new_row ? a.new_k + (int64_t)g * 16 : a.steady_k + ((int64_t)g * a.steady_stride + (-1 - x)) * 16;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) cp_async16(dst + (4 * jj + kk) * 512, p + t + kk * 4);
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int x = id.v[i];
-        const uint4* p = x < 0 ? a.steady_v + ((int64_t)g * a.steady_stride + (-1 - x)) * 16
-                               : a.values + ((int64_t)g * a.N + x) * 16;
+        const uint4* p = x >= 0 ? a.values + ((int64_t)g * a.N + x) * 16
+                       : -1 - x == new_row ? a.new_v + (int64_t)g * 16 : a.steady_v + ((int64_t)g * a.steady_stride + (-1 - x)) * 16;
         cp_async16(dst + (8 + 2 * i) * 512, p + r);
         cp_async16(dst + (9 + 2 * i) * 512, p + r + 8);
       }
@@ -264,15 +276,15 @@ __device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, c
 
   // ---- prologue: fill the ring (the ids of all its steps are fetched before the first copy is issued,
   //      so their latencies overlap) ----
-  int j_issue = min(kStages, n_steps);
+  int j_issue = min(STAGES, n_steps);
   RowIds nid;
   {
-    RowIds pid[kStages];
+    RowIds pid[STAGES];
 #pragma unroll
-    for (int st = 0; st < kStages; ++st)
+    for (int st = 0; st < STAGES; ++st)
       if (st < n_steps) pid[st] = load_ids(st);
 #pragma unroll
-    for (int st = 0; st < kStages; ++st) {
+    for (int st = 0; st < STAGES; ++st) {
       if (st < n_steps) issue(st, st, pid[st]);
       cp_async_commit();
     }
@@ -282,7 +294,7 @@ __device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, c
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk)
     qa[kk] = r < gs ? ri_ldg16(a.q + ((int64_t)g * gs + r) * 16 + t + kk * 4) : make_uint4(0, 0, 0, 0);
-  float acc[8][4];
+  float (&acc)[8][4] = part.acc;
 #pragma unroll
   for (int x = 0; x < 8; ++x)
 #pragma unroll
@@ -305,7 +317,7 @@ __device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, c
           rw[jj][e] = Elem<DT>::from_bits(a.row_w[(int64_t)g * a.N + row]);
         }
     }
-    cp_async_wait<kStages - 1>();           // the group of step s has landed (lane-private slots: no barrier)
+    cp_async_wait<STAGES - 1>();           // the group of step s has landed (lane-private slots: no barrier)
     if (j == 0) RI_FT(10);
     const uint8_t* src = my_ring_ptr + stage * kStageStride;
     const int rows_end = is_est ? n_est_rows : te;
@@ -318,10 +330,11 @@ __device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, c
         const int j0 = base + 2 * t;                 // < cap: cap is a multiple of 16 and n_est <= cap
         const float2 a0 = *reinterpret_cast<const float2*>(ll->est_sc + (r < gs ? r : 0) * ll->cap + j0);
         const float2 a1 = *reinterpret_cast<const float2*>(ll->est_sc + (r < gs ? r : 0) * ll->cap + j0 + 8);
-        const float2 w0 = *reinterpret_cast<const float2*>(ll->est_wt + j0);
-        const float2 w1 = *reinterpret_cast<const float2*>(ll->est_wt + j0 + 8);
+        const uint2 w0 = *reinterpret_cast<const uint2*>(ll->est + j0);
+        const uint2 w1 = *reinterpret_cast<const uint2*>(ll->est + j0 + 8);
+        auto size = [](uint32_t x) { return Elem<DT>::from_bits((uint16_t)(x >> 16)); };
         sv = make_float4(a0.x, a0.y, a1.x, a1.y);
-        wv = make_float4(w0.x, w0.y, w1.x, w1.y);
+        wv = make_float4(size(w0.x), size(w0.y), size(w1.x), size(w1.y));
       } else {
         sv = *reinterpret_cast<const float4*>(src);
         wv = *reinterpret_cast<const float4*>(src + 512);
@@ -382,7 +395,10 @@ __device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, c
       v[i][0] = *reinterpret_cast<const uint4*>(src + (8 + 2 * i) * 512);
       v[i][1] = *reinterpret_cast<const uint4*>(src + (9 + 2 * i) * 512);
     }
-    pv_step<DT>(acc, v, Elem<DT>::pack2(p[0][0], p[0][1]), Elem<DT>::pack2(p[1][0], p[1][1]));
+    // both parts of the probabilities: rounded once, they made the result depend on how the rows are split over warps (each
+    // has its own maximum), by one step of the 16-bit output here and there
+    const uint2 pa = split2<DT>(p[0][0], p[0][1]), pb = split2<DT>(p[1][0], p[1][1]);
+    pv_step<DT, true>(acc, v, pa.x, pb.x, pa.y, pb.y);
 
     // refill the stage just consumed (the same lane wrote and read it), then fetch the ids after that
     if (j_issue < n_steps) {
@@ -391,26 +407,47 @@ __device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, c
       if (j_issue < n_steps) nid = load_ids(j_issue);
     }
     cp_async_commit();
-    stage = stage + 1 == kStages ? 0 : stage + 1;
+    stage = stage + 1 == STAGES ? 0 : stage + 1;
   }
   cp_async_wait<0>();
   RI_FT(11);
+  part.m = m_run;
+  part.l = l_run;
+}
+
+// A warp's accumulator as 8 rows (heads) of 128 floats.
+__device__ __forceinline__ void park_partial(const Partial& part, float* my_o) {
+  const int r = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+#pragma unroll
+  for (int x = 0; x < 8; ++x) {
+    const int ch = (x < 4) ? 8 * r + 2 * x : 64 + 8 * r + 2 * (x - 4);
+    *reinterpret_cast<float2*>(my_o + (2 * t) * RI_HEAD_DIM + ch) = make_float2(part.acc[x][0], part.acc[x][2]);
+    *reinterpret_cast<float2*>(my_o + (2 * t + 1) * RI_HEAD_DIM + ch) = make_float2(part.acc[x][1], part.acc[x][3]);
+  }
+}
+
+// One group's attention by one cluster of kAttendCluster CTAs of four warps (CTA `cl` of it): the body of the stand-alone
+// attend kernel.  Ends with a cluster barrier after the last remote read, so the shared memory may be reused (or the CTA may
+// exit) when it returns.
+template <int DT>
+__device__ __forceinline__ void attend_group(const AttendArgs& a, const int g, const int cl, uint8_t* ring) {
+  constexpr int WARPS = 4, cpg = kAttendCluster, kThreads = WARPS * 32;
+  __shared__ float sm_m[WARPS][kMaxHeads], sm_l[WARPS][kMaxHeads];
+  __shared__ float cta_m[kMaxHeads], cta_l[kMaxHeads];   // this CTA's partial result: (max, sum) here, O in the ring
+  float (*cta_o)[RI_HEAD_DIM] = reinterpret_cast<float (*)[RI_HEAD_DIM]>(ring + WARPS * kStageBytes);
+  auto warp_o = [&](int w) { return reinterpret_cast<float*>(ring + w * kStageBytes); };   // stage 0 of warp w
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, t = lane & 3, gs = a.gs;
+  const int static_len = a.static_len ? *a.static_len : 0;   // null: the exact rows already contain the steady zone
+  Partial part;
+  attend_steps<DT, false, WARPS, kStages>(a, g, cl, cpg, static_len, static_len + __ldcg(a.n_exact + g), ring, nullptr, part);
 
   // ---- merge the warps of this CTA (each parks its 8 x 128 accumulator in its own idle ring region) ----
+  float l_run = part.l;
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-  if (t == 0) { sm_m[warp][r] = m_run; sm_l[warp][r] = l_run; }
-  {
-    float* my_o = warp_o(warp);
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-      const int ch = (x < 4) ? 8 * r + 2 * x : 64 + 8 * r + 2 * (x - 4);
-      my_o[(2 * t) * RI_HEAD_DIM + ch] = acc[x][0];
-      my_o[(2 * t + 1) * RI_HEAD_DIM + ch] = acc[x][1];
-      my_o[(2 * t) * RI_HEAD_DIM + ch + 1] = acc[x][2];
-      my_o[(2 * t + 1) * RI_HEAD_DIM + ch + 1] = acc[x][3];
-    }
-  }
+  if (t == 0) { sm_m[warp][r] = part.m; sm_l[warp][r] = l_run; }
+  park_partial(part, warp_o(warp));
   __syncthreads();
   for (int idx = tid; idx < gs * RI_HEAD_DIM; idx += kThreads) {
     const int h = idx >> 7, ch = idx & (RI_HEAD_DIM - 1);
@@ -498,6 +535,7 @@ inline void fill_attend_args(const ri_wave_layer& p, const Layout& L, const Exec
   a.copies = nullptr;
   a.n_copies = 0;
   a.row_w = nullptr; a.prev_out = nullptr; a.prev_lse = nullptr; a.lse_out = nullptr;
+  a.new_k = nullptr; a.new_v = nullptr;
   static const int cost_est = getenv("RI_COST_EST") ? atoi(getenv("RI_COST_EST")) : RI_COST_EST;
   static const int cost_exact = getenv("RI_COST_EXACT") ? atoi(getenv("RI_COST_EXACT")) : RI_COST_EXACT;
   a.cost_est = cost_est > 0 ? cost_est : 1;

@@ -1,46 +1,64 @@
-// The whole decode step of one layer in ONE kernel: a thread-block cluster per group (CL = 4 .. 8 CTAs of
-// 256 threads, one CTA per SM; the host picks the largest size with which all clusters are resident at once) runs
-//   phase 1  scan    s = alpha * q.C^T over the group's centroids (each CTA one slice, streamed
-//                    through the lane-private cp.async ring), per-CTA softmax partials exchanged
-//                    through distributed shared memory;
-//   phase 2  select  the selection of ri_wave_select.cuh reorganised for scores that never leave
-//                    shared memory (select_in_cluster below);
-//   phase 3  attend  the shared attention body (ri_wave_attend.cuh) over the group's estimation
-//                    and exact rows.
-// Groups are independent, so nothing crosses a cluster: the two kernel boundaries of the staged
-// path (drain, launch, ramp-up, and the scores' trip through the per-tile partials) disappear.
-// One CTA per SM on purpose: with two 128-thread CTAs per SM the hardware placed 256 CTAs on 142 SMs
-// as 114 pairs and 28 singles, a single ran its streaming phases 1.6 times faster than a paired CTA,
-// and every cluster waited for its slowest member.  The cluster size is chosen so that the grid
-// fills the SMs once: 4 CTAs per group from 19 groups up, 8 below.
+// The whole decode step of one layer in ONE kernel: a thread-block cluster per group (1 .. 8 CTAs of 256 threads, one CTA
+// per SM; see cluster_size) runs
+//   phase 1  scan    s = alpha * q.C^T over the group's centroids (each CTA one slice, streamed through a lane-private
+//                    cp.async ring), scores kept in shared memory;
+//   phase 2  select  the selection of ri_wave_select.cuh reorganised for scores that never leave shared memory;
+//   phase 3  attend  the shared attention steps (ri_wave_attend.cuh) over the group's estimation and exact rows.
+// Groups are independent, so nothing crosses a cluster: the two kernel boundaries of the staged path (drain, launch, ramp-up,
+// and the scores' trip through the per-tile partials) disappear.
+//
+// What the CTAs of a cluster tell each other (softmax statistics, two histograms, candidates, partial outputs) is PUSHED: the
+// producer stores it into every consumer's shared memory with st.async, which counts its bytes on an mbarrier there, and the
+// consumer waits for the bytes it expects.  An exchange is one trip over the cluster's network; as a cluster barrier followed
+// by loads from the other CTAs it was three (arrive, release, load).  Each of the five mbarriers is used once, so there is
+// nothing to reset, and no CTA has to wait for the others to have read.  Every wait is bounded; one that runs out is recorded
+// in the process's status word, and the CTA leaves without an output.
+//
+// What bounds it: at 128K tokens the scan runs at the copy rate (67 MB in 10.5 us), the scattered rows of the attend phase at
+// 3.7 TB/s (45 MB in 12 us, up to 15 for the groups with most rows), and between them lies a chain of dependent block-wide
+// steps, 8.5 us (of 11), in which no memory is read; at 8K the chain is all there is.  us a layer, before (barriers and loads
+// instead of pushes, candidates pulled, one CTA's first warp held up by the append, nothing asked for ahead of the wait for the
+// kernel in front) and now: 8K x 8 groups 14.8 / 11.3; 45K x 12 19.5 / 15.5; 128K x 32 44.6 / 36.4; 128K x 16 of 8 heads
+// 32.6 / 28.5; 30K x 128 (clusters of 4 taking turns, now one CTA a group) 82 / 35; 100K x 2 25.7 / 16.4 (16 CTAs instead of 8);
+// 256K x 32 (three stage kernels, now 16 keys a thread) 117 / 64.  Measured and left out: asking for the estimation entries'
+// and the candidates' rows in L2 as soon as they are known (36.0 -> 37.6, they hold up what the chain needs).
 // Reference path: cache_hub/retroinfer_cache.py:549-697 (compute).
+#include <atomic>
+#include <mutex>
+
+#include "ri_tc.cuh"
 #include "ri_wave_attend.cuh"
 #include "ri_wave_select.cuh"
 
 namespace ri_wave {
 namespace {
 
+using ri_tc::smem_u32;
+
 constexpr int kFusedThreads = 256;
 constexpr int kFusedWarps = kFusedThreads / 32;
-constexpr int kFusedMaxCentroids = 8192;                             // per group
-constexpr int kScanStages = 2;                                       // the third ring stage holds the scores instead
-constexpr int kScoreOffset = kFusedWarps * kScanStages * kStageBytes;   // 128 KB
-constexpr int kFusedRingBytes = kFusedWarps * kStages * kStageBytes;    // 192 KB
+constexpr int kFusedMaxCentroids = 16384;             // per group: four CTAs of 256 threads of 16 keys
+// CTAs per group.  More than eight are not portable, and a kernel that may be launched so is slower at every size (128K x 32
+// groups in clusters of 4: 36 -> 40 us): the kernel exists for up to 8 and for up to 16 (MAXCL).
+constexpr int kMaxCluster = 16;
+constexpr int kScanStages = 2;
 
-template <int CL>
+// What follows from the centroids a thread looks after in the selection (KEYS; a CTA's slice has at most 256 * KEYS).
+template <int KEYS>
 struct Geom {
-  // centroids a CTA's slice holds at most: 1024 with 8 CTAs per group, 2048 with 4 to 7 (a slice of 8192 / 7 fills
-  // 147 of the 256 threads' runs of keys; the rest hold nothing)
-  static constexpr int kMaxSlice = CL >= 8 ? kFusedMaxCentroids / 8 : kFusedMaxCentroids / 4;
-  static constexpr int kKeys = kMaxSlice / kFusedThreads;            // keys per thread: 8 (CL 4..7) or 4 (CL 8)
-  static_assert(CL >= 4 && CL <= 8, "clusters of 4 to 8 CTAs");
+  static_assert(KEYS == 4 || KEYS == 8 || KEYS == 16, "a thread's keys are loaded in 16-byte pieces");
+  static constexpr int kMaxSlice = KEYS * kFusedThreads;
   // floats per head in shared memory: four words of padding after every 32 (see score_at), eight more between heads
   static constexpr int kScoreStride = kMaxSlice + kMaxSlice / 8 + 8;
-  static_assert(kKeys == 4 || kKeys == 8, "a thread's keys are loaded as one or two 16-byte pieces");
+  // A large slice leaves room for a smaller ring: 16 centroids instead of 32 per warp step, two attend stages instead of three.
+  static constexpr int kScanRows = KEYS == 16 ? 16 : 32;
+  static constexpr int kScanRing = kFusedWarps * kScanStages * kScanRows * 256;
+  static constexpr int kAttendStages = KEYS == 16 ? 2 : 3;
+  static constexpr int kAttendRing = kFusedWarps * kAttendStages * kStageBytes;
 };
 
-// Place of centroid e of the slice in a head's row of scores: a thread of the selection owns a run of 4 or 8
-// consecutive centroids, so without the padding its lanes would sit 8 words apart and collide on 4 banks.
+// Place of centroid e of the slice in a head's row of scores: a thread of the selection owns a run of consecutive
+// centroids, so without the padding its lanes would sit 4, 8 or 16 words apart and collide on a few banks.
 __device__ __forceinline__ int score_at(int e) { return e + ((e >> 5) << 2); }
 
 struct FusedArgs {
@@ -48,17 +66,68 @@ struct FusedArgs {
   AttendArgs att;
   const uint4* cent;
   float* scores;     // global copy of the scores (a view for tests), written only when `views`
+  int32_t* status;   // the process's status word
   float alpha;
   int views;         // also fill the global lists and views (tests, callers that asked for the id outputs)
-  // this step's key/value rows [G, 128] to append to the steady zone (row static_len - 1) first; null: already there
-  const uint4* new_k;
-  const uint4* new_v;
-  uint4* steady_k_w;
+  uint4* steady_k_w;       // att.new_k / new_v go to row static_len - 1 of these
   uint4* steady_v_w;
-  int persist_off;   // byte offset, behind the ring and the scores, of the lists that outlive the selection
+  int page_shift;    // log2 of the page size, or -1
+  int out_aligned;   // d_out is 8-byte aligned
+  int cl;            // CTAs of a cluster
+  // Dynamic shared memory: [scan ring, later the lists that outlive the selection] ... [scores] [mail]; `temp_off` (arrays of
+  // the selection) and `ring_off` (the attend ring, over the scores) lie behind the lists.
+  int scores_off, temp_off, ring_off, mail_off;
   int cap;           // estimation entries a CTA can keep in shared memory (multiple of 16)
-  int cap_limit;     // test hook: upper limit on `cap` (< 0: none)
 };
+
+// Mail: what other CTAs push while this one may still be scanning or attending.
+__host__ __device__ constexpr int chunks_per_cta(int gs, int cl) { return (gs * 32 + cl - 1) / cl; }   // outputs, 4 at a time
+__host__ __device__ constexpr int mail_bytes(int gs, int cl) {
+  return cl * kFusedWarps * kMaxHeads * 8 + cl * chunks_per_cta(gs, cl) * 24;
+}
+// Temporary arrays of the selection: histograms pushed by every CTA (256 and 512 16-bit counts), the candidates, and five words a
+// candidate for ranking.
+__host__ __device__ constexpr int temp_bytes(int p_pad, int cl) { return cl * 1536 + p_pad * 36; }
+__host__ __device__ constexpr int range_bytes(int p_pad) { return (2 * p_pad + 4) * 4; }
+__host__ __device__ constexpr int entry_bytes(int gs) { return 4 * gs + 4; }   // scores; index and size
+
+// ---- pushes between the CTAs of a cluster ----------------------------------------------------------------------
+__device__ __forceinline__ uint32_t peer(uint32_t addr, int rank) {      // the same place in another CTA's shared memory
+  uint32_t d;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(rank));
+  return d;
+}
+__device__ __forceinline__ void push4(uint32_t dst, uint32_t bar, uint32_t x) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(x), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void push8(uint32_t dst, uint32_t bar, uint32_t x, uint32_t y) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+               ::"r"(dst), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void push16(uint32_t dst, uint32_t bar, uint4 v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar) : "memory");
+}
+// Waits until the expected bytes have arrived; false (and *abort set to `where`) when they do not within two seconds.
+__device__ __forceinline__ bool await_mail(uint32_t bar, volatile int* abort, int where) {
+  unsigned long long t0 = 0;
+  for (uint32_t spin = 0; spin < (1u << 26); ++spin) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
+    if (ok) return true;
+    if ((spin & 255u) == 255u) {
+      if (t0 == 0) t0 = ri_tc::global_ns();
+      else if (ri_tc::global_ns() - t0 > ri_tc::kWaitLimitNs) break;
+      if (*abort) return false;
+    }
+  }
+  *abort = where;
+  return false;
+}
+enum Mail { kMailStats, kMailHigh, kMailLow, kMailCandidates, kMailOut, kMails };
 
 // This thread's clusters, fetched before the scan so that their latency is not on the selection's critical path:
 // exact sizes, first row of the first of them, sizes in the 16-bit type.
@@ -67,30 +136,59 @@ struct ThreadClusters {
   int cnt[KEYS];
   int off0;
   uint32_t szw[KEYS / 2];
+
+  __device__ __forceinline__ void fetch(const SelectArgs& sel, int g, int lo, int n_loc) {
+    const int e0 = threadIdx.x * KEYS;
+#pragma unroll
+    for (int i = 0; i < KEYS; ++i) cnt[i] = 0;
+#pragma unroll
+    for (int i = 0; i < KEYS / 2; ++i) szw[i] = 0u;
+    off0 = 0;
+    const int64_t gc = (int64_t)g * sel.C + lo + e0;
+    // volatile: issued here, ahead of the scan, whatever the compiler would prefer.  Slices are multiples of 8, so of a
+    // thread's 16 clusters the second eight may lie behind its end.
+    if (e0 < n_loc) {
+#pragma unroll
+      for (int q4 = 0; q4 < KEYS / 4; ++q4)
+        if (q4 < 2 || e0 + 8 < n_loc)
+          asm volatile("ld.global.nc.v4.s32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(cnt[4 * q4]), "=r"(cnt[4 * q4 + 1]), "=r"(cnt[4 * q4 + 2]), "=r"(cnt[4 * q4 + 3])
+                       : "l"(sel.count + gc + 4 * q4));
+      asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(off0) : "l"(sel.offset + (int64_t)g * (sel.C + 1) + lo + e0));
+      if constexpr (KEYS == 4) {
+        asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(szw[0]), "=r"(szw[1]) : "l"(sel.size_dt + gc));
+      } else {
+#pragma unroll
+        for (int q8 = 0; q8 < KEYS / 8; ++q8)
+          if (q8 == 0 || e0 + 8 < n_loc)
+            asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(szw[4 * q8]), "=r"(szw[4 * q8 + 1]), "=r"(szw[4 * q8 + 2]), "=r"(szw[4 * q8 + 3])
+                         : "l"(sel.size_dt + gc + 8 * q8));
+      }
+    }
+  }
 };
 
-// Phase 1 for this CTA's slice [lo, hi) of group g: scores into shared memory (s_sc[h * kScoreStride + e]),
-// and the slice's per-head (max, sum of exponentials) of the rounded scores into part_m/part_s.
-template <int DT, int CL>
-__device__ __forceinline__ void scan_slice(const FusedArgs& f, int g, int lo, int hi, uint8_t* ring, float* s_sc,
-                                           float* part_m, float* part_s) {
-  constexpr int W = kFusedWarps, kScoreStride = Geom<CL>::kScoreStride;
-  __shared__ float w_m[W][kMaxHeads], w_s[W][kMaxHeads];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// Phase 1 for this CTA's slice [lo, hi) of group g: scores into shared memory (s_sc[h * kScoreStride + score_at(e)]), and this
+// warp's (max, sum of exponentials) of the rounded scores of head lane / 4.  `meanwhile` runs behind the first copies.
+template <int DT, int KEYS, typename F>
+__device__ __forceinline__ void scan_slice(const FusedArgs& f, int g, int lo, int hi, uint8_t* ring, float* s_sc, float& m_run,
+                                           float& s_run, F meanwhile) {
+  constexpr int W = kFusedWarps, kScoreStride = Geom<KEYS>::kScoreStride, ROWS = Geom<KEYS>::kScanRows, NJ = ROWS / 8;
+  constexpr int kSlotBytes = ROWS * 256, kSlotStride = W * kSlotBytes;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = lane >> 2, t = lane & 3;
   const int C = f.sel.C, gs = f.sel.gs;
-  // stage-major ring as in the attend phase; only stages 0 and 1 are used here
-  const uint32_t my_ring = (uint32_t)__cvta_generic_to_shared(ring) + warp * kStageBytes + lane * 16;
-  const uint8_t* my_ring_ptr = ring + warp * kStageBytes + lane * 16;
-  constexpr int kStageStride = W * kStageBytes;
-  const int n_steps = (hi - lo + 31) / 32;            // 32 centroids per warp step
+  const uint32_t my_ring = smem_u32(ring) + warp * kSlotBytes + lane * 16;      // stage-major, as in the attend phase
+  const uint8_t* my_ring_ptr = ring + warp * kSlotBytes + lane * 16;
+  const int n_steps = (hi - lo + ROWS - 1) / ROWS;
 
   // piece j*4+kk of a stage: row j*8+r of the step, bytes 16*(t+4kk) — the fragment layout of the scan kernel
   auto issue = [&](int step, int stage) {
-    const uint32_t dst = my_ring + stage * kStageStride;
-    const int base = lo + step * 32;
+    const uint32_t dst = my_ring + stage * kSlotStride;
+    const int base = lo + step * ROWS;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < NJ; ++j) {
       const int row = min(base + j * 8 + r, hi - 1);   // rows past the slice are masked below
       const uint4* p = f.cent + ((int64_t)g * C + row) * 16 + t;
 #pragma unroll
@@ -108,25 +206,27 @@ __device__ __forceinline__ void scan_slice(const FusedArgs& f, int g, int lo, in
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk)
     qa[kk] = r < gs ? ri_ldg16(f.att.q + ((int64_t)g * gs + r) * 16 + t + kk * 4) : make_uint4(0, 0, 0, 0);
+  meanwhile();
 
-  float m_run = -INFINITY, s_run = 0.f;   // softmax statistics of head r over this warp's centroids
+  m_run = -INFINITY;   // softmax statistics of head r over this warp's centroids
+  s_run = 0.f;
   int stage = 0;
 #pragma unroll 1
   for (int step = warp; step < n_steps; step += W) {
     cp_async_wait<kScanStages - 1>();
-    const uint8_t* src = my_ring_ptr + stage * kStageStride;
-    const int base = lo + step * 32;
+    const uint8_t* src = my_ring_ptr + stage * kSlotStride;
+    const int base = lo + step * ROWS;
     // the stage goes to registers and is refilled at once (the same lane wrote it and reads it), so that two stages
     // are in flight while this one is worked on
-    uint4 kb[16];
+    uint4 kb[NJ * 4];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) kb[i] = *reinterpret_cast<const uint4*>(src + i * 512);
+    for (int i = 0; i < NJ * 4; ++i) kb[i] = *reinterpret_cast<const uint4*>(src + i * 512);
     if (s_issue < n_steps) { issue(s_issue, stage); s_issue += W; }
     cp_async_commit();
     stage ^= 1;
-    float rv[4][2];
+    float rv[NJ][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < NJ; ++j) {
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
@@ -146,14 +246,14 @@ __device__ __forceinline__ void scan_slice(const FusedArgs& f, int g, int lo, in
 
     float mx = -INFINITY;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) mx = fmaxf(mx, fmaxf(rv[j][0], rv[j][1]));
+    for (int j = 0; j < NJ; ++j) mx = fmaxf(mx, fmaxf(rv[j][0], rv[j][1]));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
     const float m_new = fmaxf(m_run, mx);
     if (m_new > -INFINITY) {
       float add = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) add += exp2f((rv[j][0] - m_new) * RI_LOG2E) + exp2f((rv[j][1] - m_new) * RI_LOG2E);
+      for (int j = 0; j < NJ; ++j) add += exp2f((rv[j][0] - m_new) * RI_LOG2E) + exp2f((rv[j][1] - m_new) * RI_LOG2E);
       s_run = s_run * exp2f((m_run - m_new) * RI_LOG2E) + add;   // m_run = -inf: factor 0, s_run was 0
       m_run = m_new;
     }
@@ -161,23 +261,10 @@ __device__ __forceinline__ void scan_slice(const FusedArgs& f, int g, int lo, in
   cp_async_wait<0>();
   s_run += __shfl_xor_sync(0xffffffffu, s_run, 1);
   s_run += __shfl_xor_sync(0xffffffffu, s_run, 2);
-  if (t == 0) { w_m[warp][r] = m_run; w_s[warp][r] = s_run; }
-  __syncthreads();
-  if (tid < kMaxHeads) {
-    const int h = tid;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < W; ++w) M = fmaxf(M, w_m[w][h]);
-    float S = 0.f;
-#pragma unroll
-    for (int w = 0; w < W; ++w)
-      if (w_m[w][h] > -INFINITY) S += w_s[w][h] * exp2f((w_m[w][h] - M) * RI_LOG2E);
-    part_m[h] = M;
-    part_s[h] = S;
-  }
 }
 
 // Exclusive scan of two 64-bit values per thread at once (one pair of block barriers for both).
+// `warp_sums` is used once.
 template <int THREADS>
 __device__ __forceinline__ void block_scan2(uint64_t& a, uint64_t& b, uint64_t (*warp_sums)[2]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -187,7 +274,6 @@ __device__ __forceinline__ void block_scan2(uint64_t& a, uint64_t& b, uint64_t (
     const uint64_t na = __shfl_up_sync(0xffffffffu, ia, o), nb = __shfl_up_sync(0xffffffffu, ib, o);
     if (lane >= o) { ia += na; ib += nb; }
   }
-  __syncthreads();   // protects warp_sums from its previous use
   if (lane == 31) { warp_sums[warp][0] = ia; warp_sums[warp][1] = ib; }
   __syncthreads();
   uint64_t ba = 0, bb = 0;
@@ -209,6 +295,46 @@ __device__ __forceinline__ void note_cut(CutBin* out, int bin, uint64_t pre, uin
     out->at_g = cg_; out->at_l = (int)((v >> 16) & 0xffffu); out->at_m = (int)((v >> 32) & 0xffffu);
   }
 }
+// Counts of one bin as a packed triple: cluster-wide | in the CTAs of lower rank | in this CTA.  `h`: the bin in the first CTA's
+// histogram, the next CTA's `stride` further.
+template <int MAXCL>
+__device__ __forceinline__ uint64_t bin_triple(const uint16_t* h, int stride, int cl, int rank, uint32_t mine) {
+  uint32_t sum = 0, lower = 0;
+  auto add = [&](int rr) {
+    const uint32_t w = h[rr * stride];
+    sum += w;
+    lower += rr < rank ? w : 0u;
+  };
+#pragma unroll
+  for (int rr = 0; rr < 8; ++rr)
+    if (rr < cl) add(rr);
+  if (MAXCL > 8) {
+#pragma unroll
+    for (int rr = 8; rr < MAXCL; ++rr)
+      if (rr < cl) add(rr);
+  }
+  return (uint64_t)sum | ((uint64_t)lower << 16) | ((uint64_t)mine << 32);
+}
+// Eight 32-bit counts as 16-bit ones.
+__device__ __forceinline__ uint4 pack_counts(const uint32_t* h) {
+  const uint4 a = *reinterpret_cast<const uint4*>(h), b = *reinterpret_cast<const uint4*>(h + 4);
+  return make_uint4(a.x | (a.y << 16), a.z | (a.w << 16), b.x | (b.y << 16), b.z | (b.w << 16));
+}
+
+// The n lowest of the bits that are set (n may be negative, or more than there are).
+__device__ __forceinline__ uint32_t lowest_bits(uint32_t x, int n) {
+  if (n <= 0) return 0u;
+  while (__popc(x) > n) x &= ~(0x80000000u >> __clz(x));
+  return x;
+}
+
+// Two values rounded to the 16-bit type.
+template <int DT>
+__device__ __forceinline__ uint64_t round2(float a, float b) {
+  const uint32_t p = Elem<DT>::pack2(a, b);
+  return ri_tc::pack_f2(Elem<DT>::from_bits((uint16_t)(p & 0xffffu)), Elem<DT>::from_bits((uint16_t)(p >> 16)));
+}
+
 // Phase 2.  The arithmetic and the tie rules are those of the selection body in ri_wave_select.cuh;
 // the organisation differs: a thread keeps its keys in registers, the scores come from shared
 // memory, and every histogram is scanned as packed triples (cluster-wide count | count in the CTAs of
@@ -216,52 +342,48 @@ __device__ __forceinline__ void note_cut(CutBin* out, int bin, uint64_t pre, uin
 // needs to place its own entries: how many selected keys, and how many ties on each cut, the CTAs of
 // lower rank hold (they hold the lower ids, and ties are taken in id order: "ties taken before me" =
 // min(ties before me, ties to take)).  The positions in the compacted lists then follow from ONE more
-// packed block scan plus closed forms.  The P retrieval candidates stay with their owners until every
-// CTA pulls a copy, and every CTA ranks them and applies the page budget on its own copy.
-// Three cluster barriers (two histogram levels, candidates) and one split barrier.
+// packed block scan plus closed forms.  A retrieval candidate is pushed to its place in every CTA's list, and every CTA
+// applies the page budget on its own copy (ranking it first where the order matters).
+// Three exchanges (two histogram levels, candidates).
 // What the attend phase needs stays in shared memory (`ll`): this CTA's own estimation entries, the kept
 // clusters' row ranges and this CTA's share of the exact steps (balanced against the estimation work
-// every CTA has).  Returns true when that form is usable; false (some CTA holds more estimation entries
-// than its list takes) after writing the global lists that the stand-alone attend body reads instead.
-template <int DT, int CL>
-__device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int rank, int lo, int n_loc, uint8_t* dyn,
-                                                  const float* s_sc, const float* s_max, const float* s_inv,
-                                                  int static_len, const ThreadClusters<Geom<CL>::kKeys>& tc,
-                                                  LocalLists& ll) {
-  constexpr int T = kFusedThreads, KEYS = Geom<CL>::kKeys, kScoreStride = Geom<CL>::kScoreStride;
+// every CTA has).  Returns 1 when that form is usable; 0 (some CTA holds more estimation entries
+// than its list takes) after writing the global lists that the attend steps read instead; -1 when a wait ran out.
+template <int DT, int KEYS, int MAXCL, typename F>
+__device__ __forceinline__ int select_in_cluster(const FusedArgs& f, int g, int rank, int lo, int n_loc, uint8_t* dyn,
+                                                 const float* s_sc, const float* s_max, const float* s_inv, int static_len,
+                                                 const ThreadClusters<KEYS>& tc, uint32_t bars, volatile int* abort, LocalLists& ll,
+                                                 F meanwhile) {
+  constexpr int T = kFusedThreads, kScoreStride = Geom<KEYS>::kScoreStride;
   static_assert(T == 256, "one histogram bin per thread");
   const SelectArgs& a = f.sel;
-  cg::cluster_group cluster = cg::this_cluster();
-  uint4* own = reinterpret_cast<uint4*>(dyn);           // [p_pad] this CTA's retrieval candidates, in id order:
-                                                       //   key<<16 | (0xffff - id), cluster size, first row, unused
-  uint32_t* cand = reinterpret_cast<uint32_t*>(own + a.p_pad);   // [p_pad] all P candidates of the group (pulled)
-  uint32_t* cand_cnt = cand + a.p_pad;
-  uint32_t* cand_off = cand_cnt + a.p_pad;
-  uint32_t* ranked = cand_off + a.p_pad;               // the same three in rank order, plus the place in the row list
+  const int CL = f.cl;
+  uint16_t* rx_high = reinterpret_cast<uint16_t*>(dyn + f.temp_off);      // [CL][256] pushed by every CTA
+  uint16_t* rx_low = rx_high + CL * 256;                                   // [CL][2][256]
+  uint4* cand = reinterpret_cast<uint4*>(rx_low + CL * 512);              // [p_pad] all P candidates of the group, in id order:
+                                                                          //   key<<16 | (0xffff - id), cluster size, first row
+  uint32_t* cand_key = reinterpret_cast<uint32_t*>(cand + a.p_pad);       // ranking: the keys, then the three in rank order,
+  uint32_t* ranked = cand_key + a.p_pad;                                  // plus the place in the row list
   uint32_t* rcnt = ranked + a.p_pad;
   uint32_t* roff = rcnt + a.p_pad;
-  uint32_t* rstart = roff + a.p_pad;
+  uint4* own = reinterpret_cast<uint4*>(cand_key);                        // [p_pad] before that: this CTA's own candidates
 
-  // lists that outlive this phase (behind the ring and the scores)
-  uint32_t* dstart = reinterpret_cast<uint32_t*>(dyn + f.persist_off);   // [p_pad + 4]
+  // lists that outlive this phase
+  uint32_t* dstart = reinterpret_cast<uint32_t*>(dyn);                   // [p_pad + 4]
   uint32_t* doff = dstart + a.p_pad + 4;                                 // [p_pad]
-  float* est_wt = reinterpret_cast<float*>(doff + a.p_pad);              // [cap]
-  float* est_sc = est_wt + f.cap;                                        // [gs][cap]
-  uint16_t* est_idx = reinterpret_cast<uint16_t*>(est_sc + (size_t)a.gs * f.cap);   // [cap]
+  uint32_t* est = doff + a.p_pad;                                        // [cap] index in the slice, size (16-bit type) above it
+  float* est_sc = reinterpret_cast<float*>(est + f.cap);                 // [gs][cap]
 
-  __shared__ uint32_t hist1[256], hist2a[256], hist2b[256];   // bin 255 = largest keys
+  __shared__ __align__(16) uint32_t hist1[256], hist2[512];   // bin 255 = largest keys; low bytes at the K cut, at the P cut
   __shared__ CutBin fk, fp, lk, lp;   // high byte of the K and P cuts, then their low bytes
-  __shared__ int s_share[4];        // this CTA's exact steps [lo, hi), its estimation entries, whether the lists fit
-  __shared__ int s_nret[CL], s_nest[CL];   // every CTA's candidates / estimation entries
+  __shared__ uint32_t rx_nest[MAXCL];   // every CTA's estimation entries
   __shared__ uint32_t warp_sums[T / 32];
-  __shared__ uint64_t warp_sums64[T / 32];
+  __shared__ uint64_t warp_sums64[3][T / 32];
   __shared__ uint64_t warp_sums2[T / 32][2];
-  __shared__ __align__(16) int s_keep, s_rows;
-  __shared__ __align__(8) int s_pub[2];   // this CTA's retrieval candidates, estimation entries
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int C = a.C, gs = a.gs;
-  hist1[tid] = 0; hist2a[tid] = 0; hist2b[tid] = 0;
+  hist1[tid] = 0; hist2[tid] = 0; hist2[256 + tid] = 0;
   if (tid == 0) {
     const CutBin z = {0, 0, 0, 0, 0, 0, 0};
     fk = z; fp = z; lk = z; lp = z;
@@ -270,64 +392,66 @@ __device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int
 
   // ---- keys of this thread's centroids (ids lo + KEYS*tid ..), first-level histogram ----
   const int e0 = tid * KEYS;
-  const bool live = e0 < n_loc;                  // slices are multiples of 8: all of a thread's keys or none
+  const int n_mine = min(max(n_loc - e0, 0), KEYS);   // slices are multiples of 8: 0, 4, 8 or all 16
   const int64_t gc = (int64_t)g * C + lo + e0;
   uint16_t key[KEYS];
-  int cnt[KEYS], off[KEYS];
+  {
+    uint64_t dist2[KEYS / 2];        // two centroids each
 #pragma unroll
-  for (int i = 0; i < KEYS; ++i) { key[i] = 0; cnt[i] = 0; off[i] = 0; }
-  if (live) {
-    int run = tc.off0;
+    for (int i = 0; i < KEYS; ++i) { dist2[i / 2] = 0ull; key[i] = 0; }
+    const uint64_t log2e = ri_tc::pack_f2(RI_LOG2E, RI_LOG2E);
+    // round(exp(round(s) - max) / sum) of two centroids, two to an instruction where there is one
+    auto share = [&](float s0, float s1, int h) {
+      const uint64_t x = ri_tc::mul_f2(ri_tc::add_f2(round2<DT>(s0, s1), ri_tc::pack_f2(-s_max[h], -s_max[h])), log2e);
+      float x0, x1;
+      ri_tc::unpack_f2(x, x0, x1);
+      ri_tc::unpack_f2(ri_tc::mul_f2(ri_tc::pack_f2(exp2f(x0), exp2f(x1)), ri_tc::pack_f2(s_inv[h], s_inv[h])), x0, x1);
+      return round2<DT>(x0, x1);
+    };
+    if (n_mine > 0) {
 #pragma unroll
-    for (int i = 0; i < KEYS; ++i) { cnt[i] = tc.cnt[i]; off[i] = run; run += cnt[i]; }
-    float dist[KEYS];
+      for (int h = 0; h < kMaxHeads; ++h)
+        if (h < gs) {
 #pragma unroll
-    for (int i = 0; i < KEYS; ++i) dist[i] = 0.f;
-#pragma unroll
-    for (int h = 0; h < kMaxHeads; ++h)
-      if (h < gs) {
-#pragma unroll
-        for (int q4 = 0; q4 < KEYS / 4; ++q4) {
-          const float4 s4 = *reinterpret_cast<const float4*>(s_sc + h * kScoreStride + score_at(e0 + 4 * q4));
-          const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            dist[4 * q4 + i] += Elem<DT>::round(exp2f((Elem<DT>::round(sv[i]) - s_max[h]) * RI_LOG2E) * s_inv[h]);
+          for (int q4 = 0; q4 < KEYS / 4; ++q4) {      // behind the slice's end: scores that are never used
+            const float4 s4 = *reinterpret_cast<const float4*>(s_sc + h * kScoreStride + score_at(e0 + 4 * q4));
+            dist2[2 * q4] = ri_tc::add_f2(dist2[2 * q4], share(s4.x, s4.y, h));
+            dist2[2 * q4 + 1] = ri_tc::add_f2(dist2[2 * q4 + 1], share(s4.z, s4.w, h));
+          }
         }
-      }
 #pragma unroll
-    for (int i = 0; i < KEYS; ++i) {
-      uint16_t b = Elem<DT>::bits(dist[i]);
-      if (cnt[i] == 0) b = DT == RI_BF16 ? 0xFF7Fu : 0xFBFFu;   // most negative finite value
-      key[i] = ri_ordered_key(b);
-      atomicAdd(&hist1[key[i] >> 8], 1u);
-    }
-    if (f.views) {
-      uint32_t kw[KEYS / 2];
+      for (int i = 0; i < KEYS; ++i)
+        if (i < n_mine) {
+          float d0, d1;
+          ri_tc::unpack_f2(dist2[i / 2], d0, d1);
+          uint16_t b = Elem<DT>::bits(i & 1 ? d1 : d0);
+          if (tc.cnt[i] == 0) b = DT == RI_BF16 ? 0xFF7Fu : 0xFBFFu;   // most negative finite value
+          key[i] = ri_ordered_key(b);
+          atomicAdd(&hist1[key[i] >> 8], 1u);
+        }
+      if (f.views)
 #pragma unroll
-      for (int i = 0; i < KEYS / 2; ++i) kw[i] = key[2 * i] | ((uint32_t)key[2 * i + 1] << 16);
-      if constexpr (KEYS == 8) *reinterpret_cast<uint4*>(a.dist_keys + gc) = make_uint4(kw[0], kw[1], kw[2], kw[3]);
-      else *reinterpret_cast<uint2*>(a.dist_keys + gc) = make_uint2(kw[0], kw[1]);
+        for (int q4 = 0; q4 < KEYS / 4; ++q4)
+          if (4 * q4 < n_mine)
+            *reinterpret_cast<uint2*>(a.dist_keys + gc + 4 * q4) =
+                make_uint2(key[4 * q4] | ((uint32_t)key[4 * q4 + 1] << 16), key[4 * q4 + 2] | ((uint32_t)key[4 * q4 + 3] << 16));
     }
   }
   __syncthreads();
   RI_FT(3);
-  cluster.sync();
-  RI_FT(4);
 
   // ---- high byte of the two cuts: thread tid looks after bin 255 - tid ----
+#pragma unroll 1
+  for (int dst = warp; dst < (MAXCL > 8 ? CL : min(CL, warp + 1)); dst += T / 32)      // a lane pushes eight bins
+    push16(peer(smem_u32(rx_high + rank * 256 + lane * 8), dst), peer(bars + 8 * kMailHigh, dst), pack_counts(hist1 + lane * 8));
   const int K = a.P + a.E;
   const int my_bin = 255 - tid;
+  await_mail(bars + 8 * kMailHigh, abort, 52);
+  RI_FT(4);
   {
-    uint32_t w[CL];
-#pragma unroll
-    for (int rr = 0; rr < CL; ++rr) w[rr] = cluster.map_shared_rank(hist1, rr)[my_bin];
-    uint32_t sum = 0, lower = 0;
-#pragma unroll
-    for (int rr = 0; rr < CL; ++rr) { sum += w[rr]; lower += rr < rank ? w[rr] : 0u; }
-    const uint64_t v = (uint64_t)sum | ((uint64_t)lower << 16) | ((uint64_t)hist1[my_bin] << 32);
+    const uint64_t v = bin_triple<MAXCL>(rx_high + my_bin, 256, CL, rank, hist1[my_bin]);
     uint64_t total;
-    const uint64_t pre = block_scan<T, uint64_t>(v, warp_sums64, total);
+    const uint64_t pre = block_scan<T, uint64_t, false>(v, warp_sums64[0], total);
     note_cut(&fk, my_bin, pre, v, K);
     note_cut(&fp, my_bin, pre, v, a.P);
     __syncthreads();
@@ -335,31 +459,24 @@ __device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int
   const int binK = fk.bin, binP = fp.bin;
 
   // ---- low byte ----
-  if (live) {
 #pragma unroll
-    for (int i = 0; i < KEYS; ++i) {
-      if ((key[i] >> 8) == binK) atomicAdd(&hist2a[key[i] & 255], 1u);
-      if ((key[i] >> 8) == binP) atomicAdd(&hist2b[key[i] & 255], 1u);
+  for (int i = 0; i < KEYS; ++i)
+    if (i < n_mine) {
+      if ((key[i] >> 8) == binK) atomicAdd(&hist2[key[i] & 255], 1u);
+      if ((key[i] >> 8) == binP) atomicAdd(&hist2[256 + (key[i] & 255)], 1u);
     }
-  }
   __syncthreads();
-  cluster.sync();
+#pragma unroll 1
+  for (int dst = warp; dst < (MAXCL > 8 ? CL : min(CL, warp + 1)); dst += T / 32)
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      push16(peer(smem_u32(rx_low + rank * 512 + u * 256 + lane * 8), dst), peer(bars + 8 * kMailLow, dst),
+             pack_counts(hist2 + u * 256 + lane * 8));
+  await_mail(bars + 8 * kMailLow, abort, 53);
   RI_FT(5);
   {
-    uint32_t wa[CL], wb[CL];
-#pragma unroll
-    for (int rr = 0; rr < CL; ++rr) {
-      wa[rr] = cluster.map_shared_rank(hist2a, rr)[my_bin];
-      wb[rr] = cluster.map_shared_rank(hist2b, rr)[my_bin];
-    }
-    uint32_t sa = 0, sb = 0, la = 0, lb = 0;
-#pragma unroll
-    for (int rr = 0; rr < CL; ++rr) {
-      sa += wa[rr]; sb += wb[rr];
-      la += rr < rank ? wa[rr] : 0u; lb += rr < rank ? wb[rr] : 0u;
-    }
-    const uint64_t va = (uint64_t)sa | ((uint64_t)la << 16) | ((uint64_t)hist2a[my_bin] << 32);
-    const uint64_t vb = (uint64_t)sb | ((uint64_t)lb << 16) | ((uint64_t)hist2b[my_bin] << 32);
+    const uint64_t va = bin_triple<MAXCL>(rx_low + my_bin, 512, CL, rank, hist2[my_bin]);
+    const uint64_t vb = bin_triple<MAXCL>(rx_low + 256 + my_bin, 512, CL, rank, hist2[256 + my_bin]);
     uint64_t pa = va, pb = vb;
     block_scan2<T>(pa, pb, warp_sums2);
     note_cut(&lk, my_bin, pa, va, K - fk.above_g);
@@ -377,115 +494,101 @@ __device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int
   const int remK = max(needK - tieK_before, 0), remP = max(needP - tieP_before, 0);   // ties this CTA and later ones take
 
   // ---- ordered compaction ----
-  uint64_t c4 = 0;     // 16-bit counters: above K cut | on K cut | above P cut | on P cut
-  if (live) {
+  uint32_t gtK = 0, eqK = 0, gtP = 0, eqP = 0;     // of this thread's keys: those above and on the two cuts
 #pragma unroll
-    for (int i = 0; i < KEYS; ++i)
-      c4 += (key[i] > TK ? 1ull : 0ull) | (key[i] == TK ? 1ull << 16 : 0ull) | (key[i] > TP ? 1ull << 32 : 0ull) |
-            (key[i] == TP ? 1ull << 48 : 0ull);
-  }
-  uint64_t c4_total;
-  const uint64_t pre = block_scan<T, uint64_t>(c4, warp_sums64, c4_total);
-  int gtK = (int)(pre & 0xffffu), eqK = (int)((pre >> 16) & 0xffffu);
-  int gtP = (int)((pre >> 32) & 0xffffu), eqP = (int)(pre >> 48);
-  RI_FT(6);
-  uint32_t est_mask = 0;     // which of this thread's keys are estimation entries, and their positions in this CTA's list
-  int est_lp[KEYS];
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < KEYS; ++i) {
-      const bool inK = key[i] > TK || (key[i] == TK && eqK < remK);
-      const bool inP = key[i] > TP || (key[i] == TP && eqP < remP);
-      const int posK = gtK + min(eqK, remK), posP = gtP + min(eqP, remP);   // taken keys before this one, in this CTA
-      est_lp[i] = posK - posP;
-      if (inP) {
-        own[posP] = make_uint4(((uint32_t)key[i] << 16) | (uint32_t)(0xffff - (lo + e0 + i)), (uint32_t)cnt[i],
-                               (uint32_t)off[i], 0u);
-      } else if (inK) {
-        est_mask |= 1u << i;
-        const int lpos = est_lp[i];
-        if (lpos < f.cap) {      // the scores follow below, one entry per thread
-          est_idx[lpos] = (uint16_t)(e0 + i);
-          est_wt[lpos] = Elem<DT>::from_bits((uint16_t)(tc.szw[i >> 1] >> (16 * (i & 1))));
-        }
-      }
-      gtK += key[i] > TK; eqK += key[i] == TK; gtP += key[i] > TP; eqP += key[i] == TP;
+  for (int i = 0; i < KEYS; ++i)
+    if (i < n_mine) {
+      gtK |= (uint32_t)(key[i] > TK) << i; eqK |= (uint32_t)(key[i] == TK) << i;
+      gtP |= (uint32_t)(key[i] > TP) << i; eqP |= (uint32_t)(key[i] == TP) << i;
     }
-  }
+  // 16-bit counters: above K cut | on K cut | above P cut | on P cut
+  uint64_t c4_total;
+  const uint64_t pre = block_scan<T, uint64_t, false>(
+      (uint64_t)(__popc(gtK) | (__popc(eqK) << 16)) | ((uint64_t)(__popc(gtP) | (__popc(eqP) << 16)) << 32), warp_sums64[1], c4_total);
+  const int eqK0 = (int)((pre >> 16) & 0xffffu), eqP0 = (int)(pre >> 48);
+  const int posP0 = (int)((pre >> 32) & 0xffffu) + min(eqP0, remP);        // taken keys before this thread's, in this CTA
+  const int est0 = (int)(pre & 0xffffu) + min(eqK0, remK) - posP0;
+  const uint32_t retrieved = gtP | lowest_bits(eqP, remP - eqP0), estimated = (gtK | lowest_bits(eqK, remK - eqK0)) & ~retrieved;
   const int my_ret = (int)((c4_total >> 32) & 0xffffu) + min((int)(c4_total >> 48), remP);
   const int my_est = (int)(c4_total & 0xffffu) + min((int)((c4_total >> 16) & 0xffffu), remK) - my_ret;
-  if (tid == 0) {
-    s_pub[0] = my_ret;
-    s_pub[1] = my_est;
+  RI_FT(6);
+  auto size_bits = [&](int i) { return (tc.szw[i >> 1] >> (16 * (i & 1))) & 0xffffu; };
+  {
+    int pos = est0;
+#pragma unroll
+    for (int i = 0; i < KEYS; ++i)
+      if (estimated >> i & 1u) {      // the scores follow below, one entry per thread
+        if (pos < f.cap) est[pos] = (uint32_t)(e0 + i) | (size_bits(i) << 16);
+        ++pos;
+      }
   }
+  if (retrieved) {
+    int pos = posP0, off = tc.off0;
+#pragma unroll
+    for (int i = 0; i < KEYS; ++i) {
+      if (retrieved >> i & 1u) {
+        if (pos < a.P) own[pos] = make_uint4(((uint32_t)key[i] << 16) | (uint32_t)(0xffff - (lo + e0 + i)), (uint32_t)tc.cnt[i], (uint32_t)off, 0u);
+        ++pos;
+      }
+      off += tc.cnt[i];
+    }
+  }
+  if (tid < CL) push4(peer(smem_u32(rx_nest + rank), tid), peer(bars + 8 * kMailCandidates, tid), (uint32_t)my_est);
+  meanwhile();
   __syncthreads();
+  // the pushes in dense warps: st.async from a few lanes of every warp, key after key, took 9 us for 16 keys a thread
+#pragma unroll 1
+  for (int dst = warp; dst < (MAXCL > 8 ? CL : min(CL, warp + 1)); dst += T / 32)
+    for (int j = lane; j < my_ret; j += 32)
+      if (inP_before + j < a.P) push16(peer(smem_u32(cand + inP_before + j), dst), peer(bars + 8 * kMailCandidates, dst), own[j]);
   // log2-domain scores of the estimation entries, entry by entry (uniform work, consecutive stores)
   for (int j = tid; j < min(my_est, f.cap); j += T) {
-    const int e = score_at((int)est_idx[j]);
+    const int e = score_at((int)(est[j] & 0xffffu));
 #pragma unroll
     for (int h = 0; h < kMaxHeads; ++h)
       if (h < gs) est_sc[h * f.cap + j] = s_sc[h * kScoreStride + e] * RI_LOG2E;
   }
-  __syncthreads();
-  cluster.sync();       // every CTA's candidate list, estimation list and counts are complete
   RI_FT(7);
-
-  // ---- every CTA: pull the P candidates of the group, rank them, page budget, place in the row list ----
-  if (tid < CL) {
-    const int2 pub = *reinterpret_cast<const int2*>(cluster.map_shared_rank(s_pub, tid));
-    s_nret[tid] = pub.x;
-    s_nest[tid] = pub.y;
-  }
+  await_mail(bars + 8 * kMailCandidates, abort, 54);
   __syncthreads();
-  {
-    int nret[CL];
-#pragma unroll
-    for (int rr = 0; rr < CL; ++rr) nret[rr] = s_nret[rr];
-    for (int i = tid; i < a.p_pad; i += T) {
-      int src = 0, j = i, lim = nret[0];     // candidate i of the group = candidate j of CTA src, which holds lim
-#pragma unroll
-      for (int rr = 0; rr < CL - 1; ++rr)
-        if (src == rr && j >= nret[rr]) { j -= nret[rr]; ++src; lim = nret[rr + 1]; }
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);  // padding compares below every real candidate
-      if (i < a.P && j < lim) v = cluster.map_shared_rank(own, src)[j];
-      cand[i] = v.x; cand_cnt[i] = v.y; cand_off[i] = v.z;
-    }
-  }
-  __syncthreads();
-  cluster_arrive();     // this CTA's remote reads of the other CTAs' `own` lists are over (awaited before the ring is reused)
+  if (*abort) return -1;
   RI_FT(16);
+
   // Page budget (wave_buffer_cpu.cpp:207-216): the clusters are taken in rank order while their pages fit.
   // When ALL P candidates fit — the usual case — the order plays no part in what is attended, so unless the
   // caller wants the ranked ids the ranking is skipped and the rows are laid out in cluster-id order: one scan.
   constexpr int kPer = 1024 / T;    // P <= 1024
   int pc[kPer], pages[kPer];
-  uint32_t before;
   // pages (low half) and rows (high half) of the candidates in id order, one packed scan
   uint64_t pr = 0;
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int i = tid * kPer + u;
-    pc[u] = i < a.P ? (int)cand_cnt[i] : 0;
-    pages[u] = (pc[u] + a.page - 1) / a.page;
+    pc[u] = i < a.P ? (int)cand[i].y : 0;
+    pages[u] = f.page_shift >= 0 ? (pc[u] + a.page - 1) >> f.page_shift : (pc[u] + a.page - 1) / a.page;
     pr += (uint64_t)(uint32_t)pages[u] | ((uint64_t)(uint32_t)pc[u] << 32);
   }
   uint64_t pr_total;
-  const uint64_t pr_pre = block_scan<T, uint64_t>(pr, warp_sums64, pr_total);
+  const uint64_t pr_pre = block_scan<T, uint64_t, false>(pr, warp_sums64[2], pr_total);
+  int keep, rows_kept;
   if (!f.views && (int)(uint32_t)pr_total <= a.buffer_pages) {
     // everything fits: id order serves as the order of the row list, each cluster starts at the rows before it
-    rcnt = cand_cnt;
-    roff = cand_off;
+    keep = a.P;
+    rows_kept = (int)(pr_total >> 32);
     uint32_t row_start = (uint32_t)(pr_pre >> 32);
 #pragma unroll
     for (int u = 0; u < kPer; ++u) {
       const int i = tid * kPer + u;
-      if (i < a.P) rstart[i] = row_start;
+      if (i < a.P) {
+        dstart[i] = row_start;
+        doff[i] = cand[i].z;
+      }
       row_start += (uint32_t)pc[u];
     }
-    if (tid == 0) { s_keep = a.P; s_rows = (int)(pr_total >> 32); }
     RI_FT(17);
-    __syncthreads();
   } else {
+    for (int i = tid; i < a.p_pad; i += T) cand_key[i] = i < a.P ? cand[i].x : 0u;   // padding compares below every real candidate
+    __syncthreads();
     {
       // rank = number of larger candidates (distinct values: distinct ranks); four lanes share a candidate,
       // each counting over a quarter of the list
@@ -493,16 +596,16 @@ __device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int
       const int q_lo = quads * seg / 4, q_hi = quads * (seg + 1) / 4;
       for (int base = 0; base < a.P; base += T / 4) {      // uniform trip count: the shuffles below need whole warps
         const int i = base + (tid >> 2);
-        const uint32_t mine = i < a.P ? cand[i] : 0xffffffffu;
+        const uint32_t mine = i < a.P ? cand_key[i] : 0xffffffffu;
         int r0 = 0, r1 = 0;
         int q = q_lo;
         for (; q + 2 <= q_hi; q += 2) {
-          const uint4 c0 = *reinterpret_cast<const uint4*>(cand + 4 * q), c1 = *reinterpret_cast<const uint4*>(cand + 4 * q + 4);
+          const uint4 c0 = *reinterpret_cast<const uint4*>(cand_key + 4 * q), c1 = *reinterpret_cast<const uint4*>(cand_key + 4 * q + 4);
           r0 += (c0.x > mine) + (c0.y > mine) + (c0.z > mine) + (c0.w > mine);
           r1 += (c1.x > mine) + (c1.y > mine) + (c1.z > mine) + (c1.w > mine);
         }
         if (q < q_hi) {
-          const uint4 c = *reinterpret_cast<const uint4*>(cand + 4 * q);
+          const uint4 c = *reinterpret_cast<const uint4*>(cand_key + 4 * q);
           r0 += (c.x > mine) + (c.y > mine) + (c.z > mine) + (c.w > mine);
         }
         int rk = r0 + r1;
@@ -510,8 +613,8 @@ __device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int
         rk += __shfl_xor_sync(0xffffffffu, rk, 2);
         if (seg == 0 && i < a.P) {
           ranked[rk] = mine;
-          rcnt[rk] = cand_cnt[i];
-          roff[rk] = cand_off[i];
+          rcnt[rk] = cand[i].y;
+          roff[rk] = cand[i].z;
         }
       }
     }
@@ -524,7 +627,7 @@ __device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int
       pages[u] = (pc[u] + a.page - 1) / a.page;
       psum += (uint32_t)pages[u];
     }
-    before = block_scan<T, uint32_t>(psum, warp_sums, total);
+    uint32_t before = block_scan<T, uint32_t>(psum, warp_sums, total);
     RI_FT(17);
     // pages are non-negative, so the clusters that fit the budget form a prefix of the order
     bool fits[kPer];
@@ -540,89 +643,73 @@ __device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int
     uint32_t both_total;
     const uint32_t both_pre = block_scan<T, uint32_t>((nfit << 20) | rsum, warp_sums, both_total);
     uint32_t row_start = both_pre & 0xfffffu;
+    keep = (int)(both_total >> 20);
+    rows_kept = (int)(both_total & 0xfffffu);
 #pragma unroll
     for (int u = 0; u < kPer; ++u) {
       const int i = tid * kPer + u;
-      if (i < a.P) rstart[i] = row_start;
+      if (i < keep) {
+        dstart[i] = row_start;
+        doff[i] = roff[i];
+      }
       row_start += fits[u] ? (uint32_t)pc[u] : 0u;
     }
-    if (tid == 0) { s_keep = (int)(both_total >> 20); s_rows = (int)(both_total & 0xfffffu); }
-    __syncthreads();
   }
+  if (tid == 0) dstart[keep] = (uint32_t)rows_kept;
   RI_FT(8);
-  const int keep = s_keep, rows_kept = s_rows;
 
-  // ---- what the attend phase reads: kept clusters' row ranges, and this CTA's share of the exact steps ----
-  for (int i = tid; i <= keep; i += T) {
-    dstart[i] = i < keep ? rstart[i] : (uint32_t)rows_kept;
-    if (i < keep) doff[i] = roff[i];
-  }
-  // Share out the exact steps: level the cost units (kCostEst per estimation step a CTA already has,
+  // ---- this CTA's share of the exact steps (every warp works it out: lane c stands for CTA c) ----
+  // Level the cost units (kCostEst per estimation step a CTA already has,
   // kCostExact per exact step to hand out) so that sum_c max(0, level - e_c) >= X, then cut the exact steps at the
-  // running sums.  Lane c of the last warp stands for CTA c (warp 0 is busy with the loop above for longest).
+  // running sums.
   // Two rounds of levelling (CTAs above the first level drop out of the second) are enough in practice; whatever
   // imbalance is left only costs time.
-  if (warp == T / 32 - 1) {
+  const int n_e = lane < CL ? (int)rx_nest[lane] : 0;
+  {
     const int xs_total = (static_len + rows_kept + 15) / 16;
     const int X = f.att.cost_exact * xs_total;
-    const int n_e = lane < CL ? s_nest[lane] : 0;
     const int e_u = f.att.cost_est * ((n_e + 15) / 16);
     bool act = lane < CL;
     int level = 0;
 #pragma unroll
     for (int it = 0; it < 2; ++it) {
-      int sum_e = act ? e_u : 0;
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) sum_e += __shfl_xor_sync(0xffffffffu, sum_e, o);   // lanes 0..7 hold the sum
-      sum_e = __shfl_sync(0xffffffffu, sum_e, 0);
+      const int sum_e = __reduce_add_sync(0xffffffffu, act ? e_u : 0);
       const int n = __popc(__ballot_sync(0xffffffffu, act));                             // >= 1: the least loaded CTA stays
       level = (int)__fdividef((float)(X + sum_e + n - 1), (float)n);
       act = act && e_u <= level;
     }
     const int x_u = lane < CL ? max(0, level - e_u) : 0;
-    int incl = x_u;
-#pragma unroll
-    for (int o = 1; o < CL; o <<= 1) {
-      const int nb = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += nb;
-    }
-    const int b_lo = min(xs_total, (incl - x_u + f.att.cost_exact - 1) / f.att.cost_exact);
-    const int b_hi = lane == CL - 1 ? xs_total : min(xs_total, (incl + f.att.cost_exact - 1) / f.att.cost_exact);
-    int est_max = n_e;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) est_max = max(est_max, __shfl_xor_sync(0xffffffffu, est_max, o));
-    if (lane == rank) { s_share[0] = b_lo; s_share[1] = b_hi; s_share[2] = n_e; s_share[3] = est_max <= f.cap; }
+    const int before = __reduce_add_sync(0xffffffffu, lane < rank ? x_u : 0);
+    const int mine = __shfl_sync(0xffffffffu, x_u, rank);
+    ll.x_lo = min(xs_total, (before + f.att.cost_exact - 1) / f.att.cost_exact);
+    ll.x_hi = rank == CL - 1 ? xs_total : min(xs_total, (before + mine + f.att.cost_exact - 1) / f.att.cost_exact);
   }
-  __syncthreads();
-  const bool local = s_share[3] != 0;
-  ll.est_idx = est_idx; ll.est_wt = est_wt; ll.est_sc = est_sc;
-  ll.cap = f.cap; ll.n_est = s_share[2]; ll.slice_lo = lo;
+  const bool local = __reduce_max_sync(0xffffffffu, n_e) <= f.cap;
+  ll.est = est; ll.est_sc = est_sc;
+  ll.cap = f.cap; ll.n_est = my_est; ll.slice_lo = lo;
   ll.dstart = dstart; ll.doff = doff; ll.keep = keep; ll.n_rows = rows_kept;
-  ll.x_lo = s_share[0]; ll.x_hi = s_share[1];
+  __syncthreads();
 
   RI_FT(18);
-  // ---- the global lists: for callers that asked for them, and for the attend body when the lists above
+  // ---- the global lists: for callers that asked for them, and for the attend steps when the lists above
   //      do not fit ----
   if (f.views || !local) {
-    int est_base = inK_before - inP_before;   // estimation entries in the CTAs of lower rank
-    if (est_mask) {
+    int pe = inK_before - inP_before + est0;        // behind the estimation entries in the CTAs of lower rank
 #pragma unroll
-      for (int i = 0; i < KEYS; ++i)
-        if (est_mask >> i & 1u) {
-          const int pe = est_base + est_lp[i];
-          if (pe < a.E) {
-            a.est_ids[(int64_t)g * a.e_pad + pe] = lo + e0 + i;
-            a.est_w[(int64_t)g * a.e_pad + pe] = Elem<DT>::from_bits((uint16_t)(tc.szw[i >> 1] >> (16 * (i & 1))));
-#pragma unroll
-            for (int h = 0; h < kMaxHeads; ++h)
-              if (h < gs) a.est_s2[((int64_t)g * kMaxHeads + h) * a.e_pad + pe] = s_sc[h * kScoreStride + score_at(e0 + i)] * RI_LOG2E;
-            if (a.estimated_ids) a.estimated_ids[(int64_t)g * a.E + pe] = lo + e0 + i;
-          }
+    for (int i = 0; i < KEYS; ++i)
+      if (estimated >> i & 1u) {
+        if (pe < a.E) {
+          a.est_ids[(int64_t)g * a.e_pad + pe] = lo + e0 + i;
+          a.est_w[(int64_t)g * a.e_pad + pe] = Elem<DT>::from_bits((uint16_t)size_bits(i));
+          for (int h = 0; h < gs; ++h)
+            a.est_s2[((int64_t)g * kMaxHeads + h) * a.e_pad + pe] = s_sc[h * kScoreStride + score_at(e0 + i)] * RI_LOG2E;
+          if (a.estimated_ids) a.estimated_ids[(int64_t)g * a.E + pe] = lo + e0 + i;
         }
-    }
-    constexpr int kWarpsTotal = CL * (T / 32);   // the cluster's warps share the kept clusters out
-    for (int i = rank * (T / 32) + warp; i < keep; i += kWarpsTotal) {
-      const int o = (int)roff[i], n = (int)rcnt[i], start = (int)rstart[i];
+        ++pe;
+      }
+    // the cluster's warps share the kept clusters out
+    for (int i = rank * (T / 32) + warp; i < keep; i += CL * (T / 32)) {
+      const int o = (int)doff[i], start = (int)dstart[i], n = (int)dstart[i + 1] - start;
       for (int j = lane; j < n; j += 32)
         if (start + j < a.max_rows) a.rows[(int64_t)g * a.max_rows + start + j] = o + j;
     }
@@ -634,95 +721,190 @@ __device__ __forceinline__ bool select_in_cluster(const FusedArgs& f, int g, int
       if (a.retrieved_ids)
         for (int i = tid; i < a.P; i += T) a.retrieved_ids[(int64_t)g * a.P + i] = 0xffff - (int)(ranked[i] & 0xffffu);
     }
-    __syncthreads();    // the arrays read above lie in a ring slot that a faster warp is about to fill
+    __syncthreads();    // the arrays read above lie where a faster warp is about to fill the ring
   }
-  cluster_wait();       // every CTA is done reading this CTA's `own` list: the ring may be reused
   if (!local) {         // the global lists are read by the other CTAs of the cluster in the next phase
     __threadfence();
-    cluster.sync();
+    cluster_arrive();
+    cluster_wait();
   }
-  return local;
+  return local ? 1 : 0;
 }
 
-template <int DT, int CL>
-__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kFusedThreads, 1)
-wave_fused_kernel(FusedArgs f) {
-  ri_pdl_enter();
-  constexpr int KEYS = Geom<CL>::kKeys;
-  extern __shared__ __align__(16) uint8_t ring[];
-  __shared__ float part_m[kMaxHeads], part_s[kMaxHeads], s_max[kMaxHeads], s_inv[kMaxHeads];
+template <int DT, int KEYS, int MAXCL>
+__global__ void __launch_bounds__(kFusedThreads, 1) wave_fused_kernel(FusedArgs f) {
+  extern __shared__ __align__(128) uint8_t dyn[];
+  __shared__ float s_max[kMaxHeads], s_inv[kMaxHeads];
+  __shared__ float sm_m[kFusedWarps][kMaxHeads], sm_l[kFusedWarps][kMaxHeads];
+  __shared__ __align__(8) uint64_t s_bars[kMails];
+  __shared__ int s_abort;
+  using Geo = Geom<KEYS>;
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int g = blockIdx.y, tid = threadIdx.x;
-  const int C = f.sel.C;
+  const int rank = (int)cluster.block_rank(), CL = f.cl;
+  const int g = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, t = lane & 3;
+  const int C = f.sel.C, gs = f.sel.gs;
   const int lo = min(C, rank * f.sel.slice), hi = min(C, lo + f.sel.slice);
-  float* s_sc = reinterpret_cast<float*>(ring + kScoreOffset);
+  float* s_sc = reinterpret_cast<float*>(dyn + f.scores_off);
+  float2* rx_stat = reinterpret_cast<float2*>(dyn + f.mail_off);             // [CL][warps][heads] (max, sum)
+  // partial outputs pushed to this CTA, which finishes chunks (4 channels of a head) first .. first + own - 1 of the group's
+  const int per = chunks_per_cta(gs, CL), first = rank * per, own = min(max(gs * 32 - first, 0), per);
+  float4* rx_out = reinterpret_cast<float4*>(rx_stat + CL * kFusedWarps * kMaxHeads);      // [CL][per]
+  float2* rx_ml = reinterpret_cast<float2*>(rx_out + CL * per);                             // [CL][per] (max, sum)
+  const uint32_t bars = smem_u32(s_bars);
+  volatile int* abort = &s_abort;
+
+  // one phase each; what will arrive is known from the start
+  if (tid == 0) {
+    s_abort = 0;
+    const int bytes[kMails] = {CL * kFusedWarps * kMaxHeads * 8, CL * 512, CL * 1024, f.sel.P * 16 + CL * 4, own * CL * 24};
+    for (int i = 0; i < kMails; ++i) ri_tc::mbar_init(bars + 8 * i, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < kMails; ++i) ri_tc::mbar_arrive_expect_tx(bars + 8 * i, bytes[i]);
+  }
+  cluster_arrive();
+  ri_pdl_trigger();
+  // the scan's first rows on their way into L2 while the kernel in front ends (nothing is read before the wait)
+  {
+    const uint8_t* from = reinterpret_cast<const uint8_t*>(f.cent + ((int64_t)g * C + lo) * 16);
+    const int lines = min((hi - lo) * 2, Geo::kScanRing / 128);
+    for (int i = tid; i < lines; i += kFusedThreads) asm volatile("prefetch.global.L2 [%0];" ::"l"(from + (int64_t)i * 128));
+  }
+  ri_pdl_wait();
 
   int static_len;     // fetched now (not where the compiler would sink the load to: the middle of phase 2)
   asm volatile("ld.global.b32 %0, [%1];" : "=r"(static_len) : "l"(f.att.static_len));
-
-  // this thread's clusters (sizes, first row): requested now, needed after the scan
   ThreadClusters<KEYS> tc;
-  {
-    const int e0 = tid * KEYS;
-    const int64_t gc = (int64_t)g * C + lo + e0;
-    if (e0 < hi - lo) {
-#pragma unroll
-      // volatile: issued here, ahead of the scan, whatever the compiler would prefer
-      for (int q4 = 0; q4 < KEYS / 4; ++q4)
-        asm volatile("ld.global.nc.v4.s32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(tc.cnt[4 * q4]), "=r"(tc.cnt[4 * q4 + 1]), "=r"(tc.cnt[4 * q4 + 2]), "=r"(tc.cnt[4 * q4 + 3])
-                     : "l"(f.sel.count + gc + 4 * q4));
-      asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(tc.off0) : "l"(f.sel.offset + (int64_t)g * (C + 1) + lo + e0));
-      if constexpr (KEYS == 8)
-        asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(tc.szw[0]), "=r"(tc.szw[1]), "=r"(tc.szw[2]), "=r"(tc.szw[3]) : "l"(f.sel.size_dt + gc));
-      else
-        asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(tc.szw[0]), "=r"(tc.szw[1]) : "l"(f.sel.size_dt + gc));
-    } else {
-#pragma unroll
-      for (int i = 0; i < KEYS; ++i) tc.cnt[i] = 0;
-#pragma unroll
-      for (int i = 0; i < KEYS / 2; ++i) tc.szw[i] = 0u;
-      tc.off0 = 0;
-    }
-  }
-
-  // the new token's rows go into the steady zone now; the attend phase reads them several cluster barriers later
-  if (f.new_k != nullptr && rank == 0 && tid < 32 && static_len >= 1 && static_len <= f.att.steady_stride) {
-    const int64_t dst = ((int64_t)g * f.att.steady_stride + static_len - 1) * 16 + (tid & 15);
-    if (tid < 16) f.steady_k_w[dst] = f.new_k[(int64_t)g * 16 + tid];
-    else f.steady_v_w[dst] = f.new_v[(int64_t)g * 16 + (tid & 15)];
-  }
+  uint4 new_row = make_uint4(0u, 0u, 0u, 0u);        // this step's key (lanes 0..15) and value row: CTA 0's first warp
+  const bool appends = f.att.new_k != nullptr && rank == 0 && warp == 0;
 
   // ---- phase 1: scores of this CTA's slice ----
   RI_FT(0);
-  scan_slice<DT, CL>(f, g, lo, hi, ring, s_sc, part_m, part_s);
-  RI_FT(1);
-  cluster.sync();     // the partials of all slices are published
-  if (tid < f.sel.gs) {
-    float M = -INFINITY, S = 0.f;
-#pragma unroll
-    for (int rr = 0; rr < CL; ++rr) {
-      const float m = cluster.map_shared_rank(part_m, rr)[tid], sv = cluster.map_shared_rank(part_s, rr)[tid];
-      const float Mn = fmaxf(M, m);
-      if (Mn > -INFINITY) S = S * exp2f((M - Mn) * RI_LOG2E) + sv * exp2f((m - Mn) * RI_LOG2E);
-      M = Mn;
+  float m_run, s_run;
+  scan_slice<DT, KEYS>(f, g, lo, hi, dyn, s_sc, m_run, s_run, [&] {
+    tc.fetch(f.sel, g, lo, hi - lo);
+    if (appends) {
+      const uint4* from = (lane < 16 ? f.att.new_k : f.att.new_v) + (int64_t)g * 16 + (lane & 15);
+      asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(new_row.x), "=r"(new_row.y), "=r"(new_row.z), "=r"(new_row.w) : "l"(from));
     }
-    s_max[tid] = M;
-    s_inv[tid] = 1.0f / S;
+  });
+  RI_FT(1);
+  cluster_wait();     // every CTA's barriers are set up (they arrived before their scans)
+  for (int dst = t; dst < CL; dst += 4)
+    push8(peer(smem_u32(rx_stat + (rank * kFusedWarps + warp) * kMaxHeads + r), dst), peer(bars + 8 * kMailStats, dst),
+          __float_as_uint(m_run), __float_as_uint(s_run));
+  if (warp < gs) {     // warp h: head h
+    await_mail(bars + 8 * kMailStats, abort, 51);
+    constexpr int kPer = MAXCL * kFusedWarps / 32;
+    float m[kPer], M = -INFINITY, S = 0.f;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int i = u * 32 + lane;
+      m[u] = i < CL * kFusedWarps ? rx_stat[i * kMaxHeads + warp].x : -INFINITY;
+      M = fmaxf(M, m[u]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if (m[u] > -INFINITY) S += rx_stat[(u * 32 + lane) * kMaxHeads + warp].y * exp2f((m[u] - M) * RI_LOG2E);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) S += __shfl_xor_sync(0xffffffffu, S, o);
+    if (lane == 0) { s_max[warp] = M; s_inv[warp] = 1.0f / S; }
   }
 
-  // ---- phase 2: selection (its arrays live in the idle ring stages) ----
+  // ---- phase 2: selection (its arrays lie where the scan's ring was) ----
   RI_FT(2);
   LocalLists ll;
-  const bool local = select_in_cluster<DT, CL>(f, g, rank, lo, hi - lo, ring, s_sc, s_max, s_inv, static_len, tc, ll);
+  const int form = select_in_cluster<DT, KEYS, MAXCL>(f, g, rank, lo, hi - lo, dyn, s_sc, s_max, s_inv, static_len, tc, bars, abort, ll, [&] {
+    // the steady zone gets the new token's rows; the attend steps of this kernel take them from where they came from
+    if (appends && static_len >= 1 && static_len <= f.att.steady_stride)
+      (lane < 16 ? f.steady_k_w : f.steady_v_w)[((int64_t)g * f.att.steady_stride + static_len - 1) * 16 + (lane & 15)] = new_row;
+  });
   RI_FT(9);
 
-  // ---- phase 3: attention over the estimation and exact rows selected above ----
-  if (local) attend_group<DT, true, kFusedWarps, CL>(f.att, g, rank, ring, &ll);
-  else attend_group<DT, false, kFusedWarps, CL>(f.att, g, rank, ring);
-  RI_FT(13);
+  if (form >= 0) {
+    // ---- phase 3: attention over the estimation and exact rows selected above ----
+    uint8_t* ring = dyn + f.ring_off;
+    Partial part;
+    if (form == 1)
+      attend_steps<DT, true, kFusedWarps, Geo::kAttendStages>(f.att, g, rank, CL, static_len, static_len + ll.n_rows, ring, &ll, part);
+    else
+      attend_steps<DT, false, kFusedWarps, Geo::kAttendStages>(f.att, g, rank, CL, static_len, static_len + ll.n_rows, ring, nullptr, part);
+
+    // ---- merge the warps of this CTA (each parks its accumulator in its own idle ring region), a thread per chunk ----
+    float l_run = part.l;
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+    if (t == 0) { sm_m[warp][r] = part.m; sm_l[warp][r] = l_run; }
+    park_partial(part, reinterpret_cast<float*>(ring + warp * kStageBytes));
+    __syncthreads();
+    if (tid < gs * 32) {
+      const int h = tid >> 5;
+      float M = -INFINITY, L = 0.f;
+      float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < kFusedWarps; ++w) M = fmaxf(M, sm_m[w][h]);
+      const float Ms = M == -INFINITY ? 0.f : M;
+#pragma unroll
+      for (int w = 0; w < kFusedWarps; ++w) {
+        const float x = exp2f(sm_m[w][h] - Ms);
+        const float4 o = *reinterpret_cast<const float4*>(ring + w * kStageBytes + tid * 16);
+        L += sm_l[w][h] * x;
+        O.x += o.x * x; O.y += o.y * x; O.z += o.z * x; O.w += o.w * x;
+      }
+      const int dst = tid / per, slot = rank * per + tid - dst * per;
+      const uint32_t bar = peer(bars + 8 * kMailOut, dst);
+      push16(peer(smem_u32(rx_out + slot), dst), bar,
+             make_uint4(__float_as_uint(O.x), __float_as_uint(O.y), __float_as_uint(O.z), __float_as_uint(O.w)));
+      push8(peer(smem_u32(rx_ml + slot), dst), bar, __float_as_uint(M), __float_as_uint(L));
+    }
+    RI_FT(12);
+
+    // ---- merge the partial results of the group's CTAs: this CTA finishes its chunks ----
+    if (tid < own && await_mail(bars + 8 * kMailOut, abort, 55)) {
+      float M = -INFINITY, L = 0.f;
+      float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+      float2 ml[MAXCL];
+#pragma unroll
+      for (int c = 0; c < MAXCL; ++c) {
+        ml[c] = c < CL ? rx_ml[c * per + tid] : make_float2(-INFINITY, 0.f);
+        M = fmaxf(M, ml[c].x);
+      }
+      const float Ms = M == -INFINITY ? 0.f : M;
+#pragma unroll
+      for (int c = 0; c < MAXCL; ++c)
+        if (c < CL) {
+          const float x = exp2f(ml[c].x - Ms);
+          const float4 o = rx_out[c * per + tid];
+          L += ml[c].y * x;
+          O.x += o.x * x; O.y += o.y * x; O.z += o.z * x; O.w += o.w * x;
+        }
+      const float inv[4] = {O.x, O.y, O.z, O.w};
+      uint16_t bits[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bits[i] = Elem<DT>::bits(L > 0.f ? inv[i] / L : 0.f);
+      const int64_t at = (int64_t)g * gs * RI_HEAD_DIM + (first + tid) * 4;
+      uint16_t* out = reinterpret_cast<uint16_t*>(f.att.out) + at;
+      if (f.out_aligned) {
+        *reinterpret_cast<uint2*>(out) = make_uint2(bits[0] | ((uint32_t)bits[1] << 16), bits[2] | ((uint32_t)bits[3] << 16));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) out[i] = bits[i];
+      }
+      for (int c = 0; c < f.att.n_copies; ++c)      // several GPUs: the other ranks' gather buffers
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f.att.copies[c][at + i] = bits[i];
+    }
+    RI_FT(13);
+  }
+  // A CTA leaves when all that was meant for it has arrived.  One that gave up does not know that: it waits here until the
+  // others, which do not arrive at this barrier, have left.
+  __syncthreads();
+  if (s_abort) {
+    if (tid == 0) *f.status = s_abort;
+    cluster_arrive();
+    cluster_wait();
+  }
 }
 
 // After the decode kernel of the same stream: raise this rank's flag on every rank, then wait (bounded) until
@@ -759,72 +941,141 @@ __global__ void gather_signal_wait_kernel(uint32_t* const* flag_slots, const uin
   }
 }
 
-// Shared memory the kernel's one CTA per SM may use, minus the kernel's static part; and the SM count.
-template <int DT, int CL>
-int dynamic_budget(int* out, int* sms_out) {
-  static int cached[64] = {0}, cached_sms[64] = {0};
+// ---- host side ----------------------------------------------------------------------------------------------------
+// Where things lie in the dynamic shared memory for clusters of `cl` CTAs; false where they do not fit.
+int g_cap_limit = -1;   // ri_wave_test_local_cap
+
+int slice_of(int n_centroids, int cl) { return ((n_centroids / 8 + cl - 1) / cl) * 8; }
+int keys_of(int slice) { return slice <= 4 * kFusedThreads ? 4 : slice <= 8 * kFusedThreads ? 8 : 16; }
+
+template <int KEYS>
+bool lay_out(const ri_wave_layer& p, int cl, int budget, FusedArgs* f) {
+  using Geo = Geom<KEYS>;
+  const int p_pad = (int)ri_align_up(p.nprobe, 4), gs = p.group_size;
+  const int mail_off = (budget - mail_bytes(gs, cl)) & ~127;
+  const int scores_off = (mail_off - gs * Geo::kScoreStride * (int)sizeof(float)) & ~127;
+  const int ring_off = (mail_off - Geo::kAttendRing) & ~127;
+  const int room = (scores_off - temp_bytes(p_pad, cl) < ring_off ? scores_off - temp_bytes(p_pad, cl) : ring_off) - range_bytes(p_pad) - 16;
+  if (slice_of(p.n_centroids, cl) > Geo::kMaxSlice || Geo::kScanRing > scores_off || room < 0) return false;
+  int cap = room / entry_bytes(gs);
+  if (g_cap_limit >= 0 && cap > g_cap_limit) cap = g_cap_limit;
+  cap = (cap > Geo::kMaxSlice ? Geo::kMaxSlice : cap) & ~15;
+  f->cap = cap;
+  f->temp_off = (int)ri_align_up(range_bytes(p_pad) + (int64_t)cap * entry_bytes(gs), 16);
+  f->scores_off = scores_off; f->ring_off = ring_off; f->mail_off = mail_off; f->cl = cl;
+  f->sel.slice = slice_of(p.n_centroids, cl);
+  return true;
+}
+
+// Per device: the shared memory the kernel's one CTA per SM may use, and how many clusters of each size the device can hold
+// at once (clusters are placed inside one GPC, so that is less than SMs / size: a B200 with 148 SMs holds 15 clusters of
+// 8 or 7 CTAs, 22 of 6, 26 of 5, 33 of 4).
+struct Device { int budget; int fit[kMaxCluster + 1]; };   // fit: of up to MAXCL CTAs
+
+template <int DT, int KEYS, int MAXCL>
+int ask_device(Device* out) {
+  static Device cached[64];
+  static std::atomic<bool> known[64];
   int dev = 0;
   RI_CUDA_OK(cudaGetDevice(&dev));
   const bool track = dev >= 0 && dev < 64;
-  if (!track || cached[dev] == 0) {
-    int per_sm = 0, reserved = 0, optin = 0, sms = 0;
-    RI_CUDA_OK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-    RI_CUDA_OK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
-    RI_CUDA_OK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    RI_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    cudaFuncAttributes fa;
-    RI_CUDA_OK(cudaFuncGetAttributes(&fa, wave_fused_kernel<DT, CL>));
-    int budget = per_sm - reserved - (int)fa.sharedSizeBytes;
-    if (budget > optin - (int)fa.sharedSizeBytes) budget = optin - (int)fa.sharedSizeBytes;
-    budget &= ~15;
-    if (!track) { *out = budget; *sms_out = sms; return RI_OK; }
-    cached[dev] = budget;
-    cached_sms[dev] = sms;
+  if (track && known[dev].load(std::memory_order_acquire)) { *out = cached[dev]; return RI_OK; }
+  static std::mutex lock;
+  std::lock_guard<std::mutex> hold(lock);
+  int per_sm = 0, reserved = 0, optin = 0, sms = 0;
+  RI_CUDA_OK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  RI_CUDA_OK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+  RI_CUDA_OK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  RI_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  cudaFuncAttributes fa;
+  RI_CUDA_OK(cudaFuncGetAttributes(&fa, wave_fused_kernel<DT, KEYS, MAXCL>));
+  if (MAXCL > 8)
+    RI_CUDA_OK(cudaFuncSetAttribute(wave_fused_kernel<DT, KEYS, MAXCL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  Device d;
+  d.budget = ((per_sm - reserved < optin ? per_sm - reserved : optin) - (int)fa.sharedSizeBytes) & ~127;
+  RI_CUDA_OK(cudaFuncSetAttribute(wave_fused_kernel<DT, KEYS, MAXCL>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.budget));
+  for (int cl = 0; cl <= kMaxCluster; ++cl) d.fit[cl] = 0;
+  for (int cl = MAXCL > 8 ? 9 : 1; cl <= MAXCL; ++cl) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cl, 64);
+    cfg.blockDim = dim3(kFusedThreads);
+    cfg.dynamicSmemBytes = (size_t)d.budget;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cl;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&d.fit[cl], wave_fused_kernel<DT, KEYS, MAXCL>, &cfg) != cudaSuccess || d.fit[cl] <= 0) {
+      (void)cudaGetLastError();
+      d.fit[cl] = cl > 8 ? 0 : sms / cl;       // the query is unavailable: the bound that ignores GPC boundaries
+    }
   }
-  *out = cached[dev];
-  *sms_out = cached_sms[dev];
+  if (track) {
+    cached[dev] = d;
+    known[dev].store(true, std::memory_order_release);
+  }
+  *out = d;
   return RI_OK;
 }
 
-int g_cap_limit = -1;   // ri_wave_test_local_cap
-
-template <int DT, int CL>
-int launch(const ri_wave_layer& p, const Layout& L, cudaStream_t s, const ri_wave_gather* gather) {
+template <int DT, int KEYS, int MAXCL = 8>
+int launch(const ri_wave_layer& p, const Layout& L, int cl, cudaStream_t s, const ri_wave_gather* gather) {
   FusedArgs f;
-  int rc = fill_select_args(p, L, f.sel);
-  if (rc != RI_OK) return rc;
-  f.sel.slice = ((p.n_centroids / 8 + CL - 1) / CL) * 8;        // centroids per CTA of this kernel's cluster
+  Device d;
+  int rc = ask_device<DT, KEYS, MAXCL>(&d);
+  if (rc != RI_OK || (rc = fill_select_args(p, L, f.sel)) != RI_OK) return rc;
   fill_attend_args(p, L, nullptr, f.att);
   f.cent = static_cast<const uint4*>(p.d_centroids);
   f.scores = reinterpret_cast<float*>(static_cast<uint8_t*>(p.d_scratch) + L.scores);
+  f.status = ri_status_word();
+  if (!f.status) return RI_ERR_CUDA;
   f.alpha = 0.08838834764831845f;
   f.views = p.d_retrieved_ids != nullptr;
-  f.new_k = static_cast<const uint4*>(p.d_new_keys);
-  f.new_v = static_cast<const uint4*>(p.d_new_values);
+  f.att.new_k = static_cast<const uint4*>(p.d_new_keys);
+  f.att.new_v = static_cast<const uint4*>(p.d_new_values);
   f.steady_k_w = static_cast<uint4*>(const_cast<void*>(p.d_steady_keys));
   f.steady_v_w = static_cast<uint4*>(const_cast<void*>(p.d_steady_values));
+  f.page_shift = -1;
+  for (int i = 0; i < 20; ++i)
+    if (p.page_size == 1 << i) f.page_shift = i;
+  f.out_aligned = (uintptr_t)p.d_out % 8 == 0;
   if (gather) {
     f.att.copies = reinterpret_cast<uint16_t* const*>(gather->d_out_slots);
     f.att.n_copies = gather->n_ranks;
   }
-  RI_REQUIRE(fused_supported(p), "the single-kernel path needs n_centroids <= %d", kFusedMaxCentroids);
-  RI_REQUIRE((size_t)f.sel.p_pad * 44 <= (size_t)kScoreOffset, "nprobe=%d too large", p.nprobe);
-  // dynamic shared memory: [ring | scores (over ring stage 2 and beyond)] [kept-cluster ranges] [estimation lists]
-  int budget = 0, sms = 0;
-  if ((rc = dynamic_budget<DT, CL>(&budget, &sms)) != RI_OK) return rc;
-  const int scores_end = kScoreOffset + p.group_size * Geom<CL>::kScoreStride * (int)sizeof(float);
-  f.persist_off = (int)ri_align_up(scores_end > kFusedRingBytes ? scores_end : kFusedRingBytes, 16);
-  const int ranges = (2 * f.sel.p_pad + 4) * 4;
-  const int per_entry = 4 * p.group_size + 4 + 2;
-  int cap = (budget - f.persist_off - ranges) / per_entry;
-  if (g_cap_limit >= 0 && cap > g_cap_limit) cap = g_cap_limit;
-  cap = cap < 0 ? 0 : (cap > Geom<CL>::kMaxSlice ? Geom<CL>::kMaxSlice : cap) & ~15;
-  f.cap = cap;
-  const size_t smem = ri_align_up((size_t)f.persist_off + ranges + (size_t)cap * per_entry, 16);
-  RI_REQUIRE((int)smem <= budget, "nprobe=%d needs %zu bytes of shared memory per CTA (limit %d)", p.nprobe, smem, budget);
-  RI_CUDA_OK(cudaFuncSetAttribute(wave_fused_kernel<DT, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  RI_CUDA_OK(ri_launch_pdl_id(5, wave_fused_kernel<DT, CL>, dim3(CL, p.groups), dim3(kFusedThreads), smem, s, f));
+  RI_REQUIRE(lay_out<KEYS>(p, cl, d.budget, &f), "the single-kernel path does not take this geometry");
+  RI_CUDA_OK(ri_launch_pdl_cluster(5, cl, wave_fused_kernel<DT, KEYS, MAXCL>, dim3(cl, p.groups), dim3(kFusedThreads), (size_t)d.budget, s, f));
   return RI_OK;
+}
+
+int cluster_size(const ri_wave_layer& p, const Device& d, const Device& big) {
+  // The largest size with which all groups' clusters are resident at once (a cluster that has to wait for another one to
+  // finish doubles the layer's time), as long as a CTA's slice is worth its share of the exchanges.  us a layer, one group of
+  // 11776 centroids: 28.7 with 8 CTAs, 20.4 with 16; four groups of 992: 12.7 with 8, 13.6 with 16; eight of 512: 11.1 with 4,
+  // 11.4 with 8, 15.8 with one.
+  int cl = kMaxCluster;
+  while (cl > 1 && p.groups > (cl > 8 ? big : d).fit[cl]) --cl;
+  while (cl > 8 && p.n_centroids < 160 * cl) --cl;
+  while (cl > 4 && p.n_centroids < 96 * cl) --cl;
+  // a thread's keys limit the slice: more groups than fit at once take turns
+  while (slice_of(p.n_centroids, cl) > Geom<16>::kMaxSlice) ++cl;
+  return cl;
+}
+
+template <int DT>
+int launch_fused_dt(const ri_wave_layer& p, const Layout& L, cudaStream_t s, const ri_wave_gather* gather) {
+  Device d, big;
+  int rc = ask_device<DT, 8, 8>(&d);
+  if (rc != RI_OK || (rc = ask_device<DT, 4, 16>(&big)) != RI_OK) return rc;
+  const int cl = cluster_size(p, d, big), keys = keys_of(slice_of(p.n_centroids, cl));
+  if (cl > 8) return keys == 4 ? launch<DT, 4, 16>(p, L, cl, s, gather) : launch<DT, 8, 16>(p, L, cl, s, gather);
+  switch (keys) {
+    case 4: return launch<DT, 4>(p, L, cl, s, gather);
+    case 8: return launch<DT, 8>(p, L, cl, s, gather);
+    default: return launch<DT, 16>(p, L, cl, s, gather);
+  }
 }
 
 }  // namespace
@@ -836,56 +1087,6 @@ bool fused_supported(const ri_wave_layer& p) { return p.n_centroids <= kFusedMax
 extern "C" int ri_wave_test_local_cap(int cap) {
   g_cap_limit = cap;
   return RI_OK;
-}
-
-// How many clusters of CL CTAs of this kernel the device can hold at once (asked once per device).  Clusters are placed
-// inside one GPC, so this is less than SMs / CL: a B200 with 148 SMs holds 15 clusters of 8, not 18.
-template <int DT, int CL>
-int resident_clusters(int* out) {
-  static int cached[64] = {0};
-  int dev = 0;
-  RI_CUDA_OK(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && cached[dev] > 0) { *out = cached[dev]; return RI_OK; }
-  int budget = 0, sms = 0;
-  const int rc = dynamic_budget<DT, CL>(&budget, &sms);
-  if (rc != RI_OK) return rc;
-  RI_CUDA_OK(cudaFuncSetAttribute(wave_fused_kernel<DT, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CL, 64);
-  cfg.blockDim = dim3(kFusedThreads);
-  cfg.dynamicSmemBytes = (size_t)budget;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CL;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, wave_fused_kernel<DT, CL>, &cfg) != cudaSuccess || n <= 0) {
-    (void)cudaGetLastError();
-    n = sms / CL;               // the query is unavailable: the bound that ignores GPC boundaries
-  }
-  if (dev >= 0 && dev < 64) cached[dev] = n;
-  *out = n;
-  return RI_OK;
-}
-
-template <int DT>
-int launch_fused_dt(const ri_wave_layer& p, const Layout& L, cudaStream_t s, const ri_wave_gather* gather) {
-  // cluster size: the largest of 8 .. 4 CTAs per group with which all groups' clusters are resident at once (a cluster
-  // that has to wait for another one to finish doubles the layer's time).  Clusters are placed inside a GPC, so the
-  // counts are not SMs / size: a B200 holds 15 clusters of 8 or 7 CTAs, 22 of 6, 26 of 5, 33 of 4.
-  int fit = 0, rc;
-  if ((rc = resident_clusters<DT, 8>(&fit)) != RI_OK) return rc;
-  if (p.groups <= fit) return launch<DT, 8>(p, L, s, gather);
-  if ((rc = resident_clusters<DT, 7>(&fit)) != RI_OK) return rc;
-  if (p.groups <= fit) return launch<DT, 7>(p, L, s, gather);
-  if ((rc = resident_clusters<DT, 6>(&fit)) != RI_OK) return rc;
-  if (p.groups <= fit) return launch<DT, 6>(p, L, s, gather);
-  if ((rc = resident_clusters<DT, 5>(&fit)) != RI_OK) return rc;
-  if (p.groups <= fit) return launch<DT, 5>(p, L, s, gather);
-  return launch<DT, 4>(p, L, s, gather);
 }
 
 int launch_fused(const ri_wave_layer& p, const Layout& L, cudaStream_t s, const ri_wave_gather* gather) {

@@ -74,8 +74,9 @@ inline int fill_select_args(const ri_wave_layer& p, const Layout& L, SelectArgs&
   return RI_OK;
 }
 
-// Exclusive scan of one value per thread over the block.  `total` = block sum.
-template <int THREADS, typename T>
+// Exclusive scan of one value per thread over the block.  `total` = block sum.  REUSED: `warp_sums` may still be read by a
+// scan before.
+template <int THREADS, typename T, bool REUSED = true>
 __device__ __forceinline__ T block_scan(T v, T* warp_sums, T& total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   T inc = v;
@@ -84,7 +85,7 @@ __device__ __forceinline__ T block_scan(T v, T* warp_sums, T& total) {
     const T n = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += n;
   }
-  __syncthreads();   // protects warp_sums from its previous use
+  if (REUSED) __syncthreads();
   if (lane == 31) warp_sums[warp] = inc;
   __syncthreads();
   T base = 0, tot = 0;
