@@ -188,4 +188,5 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def current_stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream (``torch.cuda.current_stream()`` builds an object for it: 3 us)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

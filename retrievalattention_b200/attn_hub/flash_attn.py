@@ -19,18 +19,21 @@ def prefill_full_flash_attn(query_states, key_states, value_states, causal):
 
 def _dense_form(q, k, v, valid_length) -> bool:
     """Whether the call has the form the dense cache's own kernel takes (everything as ``flash_attn_cache`` keeps it);
-    any other goes through the general operator."""
-    if not (q.dim() == 4 and k.dim() == 4 and q.is_cuda and q.device.index == torch.cuda.current_device()
-            and q.dtype in (torch.bfloat16, torch.float16)):
+    any other goes through the general operator.  Written out: it runs once per layer and token."""
+    if q.dim() != 4 or k.dim() != 4 or not q.is_cuda:
+        return False
+    dev, dtype = q.device, q.dtype
+    if dev.index != torch.cuda.current_device() or (dtype != torch.bfloat16 and dtype != torch.float16):
         return False
     b, one, hq, d = q.shape
-    hk = k.shape[1]
-    return (one == 1 and d == 128 and k.shape == (b, hk, k.shape[2], 128) and v.shape == k.shape and hk > 0 and hq % hk == 0
-            and 1 <= hq // hk <= 8 and 1 <= b * hk <= 65535 and b * hk * k.shape[2] < (1 << 31) - 16 and k.shape[2] > 0
-            and valid_length.shape == (b,) and valid_length.dtype == torch.int32 and valid_length.device == q.device
-            and valid_length.is_contiguous()
-            and all(x.is_contiguous() and x.device == q.device and x.dtype == q.dtype and x.data_ptr() % 16 == 0
-                    for x in (q, k, v)))
+    kb, hk, length, kd = kv = k.shape
+    g = b * hk
+    return (one == 1 and d == 128 and kb == b and kd == 128 and v.shape == kv and hk > 0 and hq % hk == 0
+            and 1 <= hq // hk <= 8 and 1 <= g <= 65535 and g * length < (1 << 31) - 16 and length > 0
+            and valid_length.shape == (b,) and valid_length.dtype == torch.int32 and valid_length.device == dev
+            and valid_length.is_contiguous() and q.is_contiguous() and k.is_contiguous() and v.is_contiguous()
+            and k.device == dev and v.device == dev and k.dtype == dtype and v.dtype == dtype
+            and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % 16 == 0)
 
 
 def decode_full_flash_attn(query_states, key_states, value_states, layer_idx, full_attn_cache):

@@ -68,17 +68,19 @@ class flash_attn_cache(KV_Cache):
         put others in their place), and rows that fit (a full cache is refused by the indexing below).  The lengths are counted on the host here; where they move on without it, as in
         replays of a CUDA graph, the kernel itself leaves out a row that does not fit, and ``check_prefill_errors`` or the
         next ``decode_full_flash_attn`` says so.  Six launches of indexing kernels otherwise."""
-        shape, dev, n = (self.batch_size, 1, self.kv_head, self.head_dim), keys.device, self.valid_length
-        if not (keys.is_cuda and dev.index == torch.cuda.current_device() and n.device == dev and n.dtype == torch.int32
-                and n.is_contiguous() and n.shape == (self.batch_size,) and self._longest is not None and self._longest < self.max_length):
+        if not keys.is_cuda or self._longest is None or self._longest >= self.max_length:
             return False
-        for x in (keys, keys if values is None else values):
-            if not (x.shape == (self.batch_size, self.kv_head, self.max_length, self.head_dim) and x.dtype == keys.dtype
-                    and x.device == dev and x.is_contiguous() and x.data_ptr() % 16 == 0 and not x.requires_grad):
-                return False
-        for x in (key_states, value_states):
-            if not (x.shape == shape and x.dtype == keys.dtype and x.element_size() == 2 and x.device == dev
-                    and x.is_contiguous() and x.data_ptr() % 16 == 0 and not x.requires_grad):
+        if values is None:
+            values = keys
+        dev, dtype, n, b, hk, d = keys.device, keys.dtype, self.valid_length, self.batch_size, self.kv_head, self.head_dim
+        if not (dev.index == torch.cuda.current_device() and n.device == dev and n.dtype == torch.int32
+                and n.is_contiguous() and n.shape == (b,) and key_states.element_size() == 2):
+            return False
+        cache, rows = (b, hk, self.max_length, d), (b, 1, hk, d)
+        if not (keys.shape == cache and values.shape == cache and key_states.shape == rows and value_states.shape == rows):
+            return False
+        for x in (keys, values, key_states, value_states):
+            if x.dtype != dtype or x.device != dev or x.requires_grad or not x.is_contiguous() or x.data_ptr() % 16:
                 return False
         return True
 

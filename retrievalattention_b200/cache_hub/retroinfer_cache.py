@@ -448,7 +448,8 @@ class retroinfer_cache(KV_Cache):
             # every layer of a step attends static_pattern_total(+1) rows (:559); advance for the next step
             for p in self._per_device.values():
                 p["static_len"].add_(1)
-        return out.view(self.batch_size, 1, self.num_heads, self.head_dim)
+        shape = (self.batch_size, 1, self.num_heads, self.head_dim)
+        return out if out.shape == shape else out.view(shape)
 
     def _compute_with_estimation(self, queries, layer_idx, queries_next, out):
         """``use_cluster_estimation`` (:565, :582-595): attend the clusters searched one layer ahead if there are

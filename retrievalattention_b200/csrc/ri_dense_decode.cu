@@ -18,6 +18,8 @@
 // (r = lane/4, t = lane%4) reads K row 8jj + s(r) and of V rows t + 4i the 16-byte pieces s(r) and 8 + s(r), where s
 // rotates the three bits of r so that the eight lanes of a quarter read eight different bank groups.  Column n
 // of the scores is therefore key 8jj + s(n), which makes a lane's two columns keys t and t + 4: the rows of V it holds.
+#include <atomic>
+
 #include "ri_tc.cuh"
 #include "ri_wave_attend.cuh"
 
@@ -396,7 +398,14 @@ int make_step_map(CUtensorMap* map, const void* base, int64_t rows, int dtype) {
 
 template <int DT>
 int launch_dense(const DenseArgs& a, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t s) {
-  RI_CUDA_OK(cudaFuncSetAttribute(dense_decode_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem));
+  static std::atomic<bool> known[64];                   // per device; asked for again where it is not remembered
+  int dev = 0;
+  RI_CUDA_OK(cudaGetDevice(&dev));
+  const bool track = dev >= 0 && dev < 64;
+  if (!track || !known[dev].load(std::memory_order_relaxed)) {
+    RI_CUDA_OK(cudaFuncSetAttribute(dense_decode_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem));
+    if (track) known[dev].store(true, std::memory_order_relaxed);
+  }
   RI_CUDA_OK(ri_launch_pdl_id(11, dense_decode_kernel<DT>, dim3(a.max_ctas), dim3(kDenseThreads), (size_t)kDenseSmem, s,
                               map_k, map_v, a));
   RI_CUDA_OK(ri_launch_pdl_id(11, dense_combine_kernel<DT>, dim3(a.gs, a.batch * a.hk), dim3(kCombineThreads), 0, s, a));
