@@ -906,15 +906,31 @@ constexpr int kUpdateThreads = 128;
 constexpr int kWindow = 4;          // rows per step
 constexpr int kWindows = 4;         // steps in the ring
 
-template <int DT, bool LAST>
+// LONG: clusters of kLongCluster members and more are left to the whole CTA, which sums them when its warps are done with the
+// others.  Through the ring such a cluster is one warp's chain of 75 clocks a row, every four rows of which wait, shuffle and
+// compare; the CTA streams its rows through twice the depth, and a thread adds one channel of a row after the other, in the same
+// order.  The initial centroids are rows as they are, and those of the longest keys win most of a segment: the first two updates
+// are launched in this form (8 heads x 128K rows: 75 -> 92 and 294 -> 136 us, 8K rows 28 and 14 us either way), the later ones
+// without it.
+constexpr int kLongCluster = 512;
+constexpr int kLongRows = 32;       // rows of a batch
+constexpr int kLongBatches = 5;     // batches in shared memory
+
+template <int DT, bool LAST, bool LONG>
 __global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArgs a) {
   ri_pdl_enter();
   constexpr int kWarps = kUpdateThreads / 32, kRowsBytes = kWindows * kWindow * 256;
-  __shared__ __align__(16) uint8_t ring[kWarps][(LAST ? 2 : 1) * kRowsBytes];
+  static_assert(!(LAST && LONG) && kLongBatches * kLongRows * 256 >= kWarps * kRowsBytes, "the batches lie over the warps' rings");
+  __shared__ __align__(16) uint8_t ring[kWarps][LONG ? kLongBatches * kLongRows * 256 / kWarps : (LAST ? 2 : 1) * kRowsBytes];
+  __shared__ int s_long[LONG ? kWarps : 1][3];                // per warp: a long cluster's place in its run, first member, end
+  __shared__ float s_sum[LONG ? 128 : 1];
   const int lane = threadIdx.x & 31;
   const int job = (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5);
-  const int idx0 = job * a.clusters_per_warp;                 // clusters_per_warp divides n_cen: one problem per warp
-  if (idx0 >= a.n_clusters) return;
+  // clusters_per_warp divides n_cen: one problem per warp.  LONG: a warp without clusters takes the last ones, which another warp
+  // of the CTA has, and leaves them alone
+  const bool idle = job * a.clusters_per_warp >= a.n_clusters;
+  if (!LONG && idle) return;
+  const int idx0 = LONG && idle ? a.n_clusters - a.clusters_per_warp : job * a.clusters_per_warp;
   const int problem = idx0 / a.n_cen, z = problem / a.seg_per_group;
   int c = idx0 - problem * a.n_cen;
   const int tok_in_group = (problem - z * a.seg_per_group) * a.n_tok;
@@ -976,8 +992,9 @@ __global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArg
     end = __shfl_sync(0xffffffffu, my_end, min(done, 31));
   };
 
-  const int n = last - first;                                 // members of all of this warp's clusters
+  // clusters `done` .. to - 1 through the ring, whatever their sizes
   uint8_t* my_ring = ring[threadIdx.x >> 5];
+  auto stream = [&](const int to, const int first, const int n) {      // first: their first member, n: how many they have
   const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(my_ring);
   int ids = lane < n ? ord[first + lane] : 0;                 // 32 list entries; the next 32 below
   int ids_next = 32 + lane < n ? ord[first + 32 + lane] : 0;
@@ -1041,13 +1058,99 @@ __global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArg
           if (LAST) add_row<DT>(vs, in ? vv[u] : make_uint2(0u, 0u));
         }
       }
-      if (hi > kWindow || done == a.clusters_per_warp) break;
+      if (hi > kWindow || done == to) break;
       finish();
       lo = hi;
-      if (done == a.clusters_per_warp) break;
+      if (done == to) break;
     }
   }
-  while (done < a.clusters_per_warp) finish();
+  while (done < to) finish();
+  };
+  if (!LONG) {
+    stream(a.clusters_per_warp, first, last - first);
+    return;
+  }
+  const int end_before = __shfl_up_sync(0xffffffffu, my_end, 1), my_start = lane > 0 ? end_before : first;
+  unsigned todo = __ballot_sync(0xffffffffu, !idle && lane < a.clusters_per_warp && my_end - my_start >= kLongCluster);
+  if (idle) done = a.clusters_per_warp;
+  for (unsigned rest = todo;; rest &= rest - 1) {
+    const int at = rest ? __ffs(rest) - 1 : a.clusters_per_warp;      // the next long one, or the end
+    if (done < at) {
+      stream(at, start, __shfl_sync(0xffffffffu, my_end, at - 1) - start);
+      cp_async_wait<0>();
+    }
+    if (!rest) break;
+    start = end;                                              // not now
+    ++done;
+    end = __shfl_sync(0xffffffffu, my_end, min(done, 31));
+  }
+  // the long clusters, one of every warp after the other
+  const int warp = threadIdx.x >> 5, tid = threadIdx.x;
+  for (;;) {
+    const int at = todo ? __ffs(todo) - 1 : -1;
+    const int from = __shfl_sync(0xffffffffu, my_start, max(at, 0)), to = __shfl_sync(0xffffffffu, my_end, max(at, 0));
+    if (lane == 0) { s_long[warp][0] = at; s_long[warp][1] = from; s_long[warp][2] = to; }
+    if (!__syncthreads_or(at >= 0)) break;
+    for (int w = 0; w < kWarps; ++w) {
+      if (s_long[w][0] < 0) continue;                         // the same for every warp of the CTA
+      const int l_from = s_long[w][1], l_n = s_long[w][2] - l_from;
+      // the problem of that warp's clusters (a CTA's warps may work on several)
+      const int l_idx = min(((int)blockIdx.x * kWarps + w) * a.clusters_per_warp, a.n_clusters - 1);
+      const int l_problem = l_idx / a.n_cen, l_z = l_problem / a.seg_per_group, l_tok = (l_problem - l_z * a.seg_per_group) * a.n_tok;
+      const int32_t* l_ord = a.order + (int64_t)l_z * a.group_stride + l_tok + l_from;
+      const uint4* l_rows = reinterpret_cast<const uint4*>(a.rows) + ((int64_t)l_z * a.src.group + (int64_t)l_tok * a.src.row) * 16 + (tid & 15);
+      const uint32_t batch = (uint32_t)__cvta_generic_to_shared(&ring[0][0]);
+      constexpr int kCopies = kLongRows * 16 / kUpdateThreads;      // 16-byte pieces of a batch per thread
+      int id[kCopies];
+      auto list = [&](int r) {                                // of the batch's rows, those whose pieces this thread copies
+#pragma unroll
+        for (int u = 0; u < kCopies; ++u) id[u] = l_ord[min(r + u * (kUpdateThreads / 16) + (tid >> 4), l_n - 1)];
+      };
+      auto copy = [&](int r) {
+#pragma unroll
+        for (int u = 0; u < kCopies; ++u)
+          cp_async16(batch + ((r / kLongRows) % kLongBatches) * kLongRows * 256 + (u * kUpdateThreads + tid) * 16, l_rows + id[u] * row_step);
+      };
+      constexpr int kAhead = (kLongBatches - 1) * kLongRows;
+#pragma unroll
+      for (int r = 0; r < kAhead; r += kLongRows) {
+        list(r);
+        copy(r);
+        cp_async_commit();
+      }
+      list(kAhead);
+      float sum = 0.f;
+      for (int r = 0; r < l_n; r += kLongRows) {
+        if (r + kAhead < l_n) copy(r + kAhead);
+        cp_async_commit();
+        list(r + kAhead + kLongRows);
+        cp_async_wait<kLongBatches - 1>();
+        __syncthreads();                                      // every thread's pieces of the batch
+        const uint16_t* v = reinterpret_cast<const uint16_t*>(&ring[0][0] + ((r / kLongRows) % kLongBatches) * kLongRows * 256) + tid;
+        if (r + kLongRows <= l_n) {
+#pragma unroll
+          for (int u = 0; u < kLongRows; ++u) sum += Elem<DT>::from_bits(v[u * 128]);
+        } else {
+          for (int u = 0; u < l_n - r; ++u) sum += Elem<DT>::from_bits(v[u * 128]);
+        }
+        __syncthreads();                                      // the batch may be overwritten
+      }
+      cp_async_wait<0>();
+      s_sum[tid] = sum;
+      __syncthreads();
+      if (warp == w) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ks[i] = s_sum[lane * 4 + i];
+        done = at;
+        start = from;
+        end = to;
+        finish();
+        todo &= todo - 1;
+      }
+      __syncthreads();
+    }
+    __syncthreads();                                          // the list has been read by all
+  }
 }
 
 // ---- host side --------------------------------------------------------------------------------
@@ -1203,8 +1306,9 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const Place& pl, const void*
     ua.clusters_per_warp = cpw;
     constexpr int per_cta = kUpdateThreads / 32;
     const dim3 ugrid((ua.n_clusters / cpw + per_cta - 1) / per_cta);
-    RI_CUDA_OK(last ? ri_launch_pdl_id(9, kmeans_update_kernel<DT, true>, ugrid, dim3(kUpdateThreads), 0, s, ua)
-                    : ri_launch_pdl_id(9, kmeans_update_kernel<DT, false>, ugrid, dim3(kUpdateThreads), 0, s, ua));
+    RI_CUDA_OK(last     ? ri_launch_pdl_id(9, kmeans_update_kernel<DT, true, false>, ugrid, dim3(kUpdateThreads), 0, s, ua)
+               : it < 2 ? ri_launch_pdl_id(9, kmeans_update_kernel<DT, false, true>, ugrid, dim3(kUpdateThreads), 0, s, ua)
+                        : ri_launch_pdl_id(9, kmeans_update_kernel<DT, false, false>, ugrid, dim3(kUpdateThreads), 0, s, ua));
   }
   if (!p->center)
     RI_CUDA_OK(cudaMemcpyAsync(p->d_centroids, cent, (size_t)Z * C * 256, cudaMemcpyDeviceToDevice, s));

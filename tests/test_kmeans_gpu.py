@@ -247,3 +247,28 @@ def test_infinite_scores_keep_every_token():
         assert int(r["error"].item()) == 0 and int(r["cluster_count"].sum()) == n
         got = r["values"][0].float().cpu()
         assert (got[:, 0] + 32 * got[:, 1]).sort().values.tolist() == list(range(n))
+
+
+# members of the long cluster: around the size from which a whole CTA sums it, a batch of rows more, and several rounds of batches
+# with a remainder
+@pytest.mark.parametrize("per_seg,segs,cents,dtype", [(511, 1, 32, torch.bfloat16), (512, 2, 64, torch.float16), (545, 1, 32, torch.bfloat16),
+                                                       (701, 3, 96, torch.bfloat16), (2117, 2, 128, torch.float16), (6000, 1, 512, torch.bfloat16)])
+def test_cluster_that_holds_a_whole_segment(per_seg, segs, cents, dtype):
+    """The first initial centroid of every segment is a long key that wins all its tokens: after one update of that cluster (the
+    others keep their rows) the assignments are the oracle's except for ties."""
+    from retrievalattention_b200.cache_hub import kmeans as gk
+
+    heads, n = 2, per_seg * segs
+    gen = torch.Generator().manual_seed(per_seg)
+    u = torch.randn((heads, 1, 128), generator=gen)
+    k = (u + torch.randn((heads, n, 128), generator=gen)).to(dtype)
+    start = okm.initial_centroid_indices(n, cents)
+    k[:, start[::cents // segs]] = (u * 20).to(dtype)
+    v = torch.randn((heads, n, 128), generator=gen).to(dtype)
+    data = k.reshape(-1, per_seg, 128)
+    cen = torch.index_select(k, 1, start).reshape(-1, cents // segs, 128)
+    assert (okm.assign(data, cen) == 0).all()                    # the case is what it says
+    want = okm.segment_k_means(k, v, cents, 2, segs, return_assignments=True)[4]
+    got = gk._run(k.cuda(), v.cuda(), cents, 2, segs, False, False)
+    assert int(got["error"]) == 0
+    check_assignments(got["assign"].cpu(), want.to(torch.int32), k, cents, 2, segs)
