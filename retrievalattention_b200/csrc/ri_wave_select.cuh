@@ -15,8 +15,7 @@
 //      rule (wave_buffer_cpu.cpp:207-216) and computes each kept cluster's place in the row list;
 //   6. all CTAs expand the kept clusters into row indices.
 //
-// The body is a device function so that the stand-alone selection kernel (256 threads) and the
-// single-kernel decode path (128 threads, selection between its scan and attend phases) share it.
+// The single-kernel decode path has its own organisation of the same steps (ri_wave_fused.cu).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -125,32 +124,6 @@ __device__ __forceinline__ void find_bins(const int* ga, const int* la, int ka, 
     const int above_b = (int)((pre >> 32) & 0xffffu), above_lb = (int)(pre >> 48);
     if (above_a < ka && above_a + ca >= ka) { outa[0] = bin; outa[1] = above_a; outa[2] = above_la; }
     if (above_b < kb && above_b + cb >= kb) { outb[0] = bin; outb[1] = above_b; outb[2] = above_lb; }
-    pre += v[j];
-  }
-  __syncthreads();
-}
-
-// The same search with the counts of a thread's two bins (255-2*tid, then 254-2*tid) given in registers.
-template <int THREADS>
-__device__ __forceinline__ void find_bins_regs(const int (&ga)[2], const int (&la)[2], int ka, int* outa,
-                                               const int (&gb)[2], const int (&lb)[2], int kb, int* outb,
-                                               uint64_t* warp_sums) {
-  static_assert(THREADS == 128, "two bins per thread");
-  uint64_t v[2], sum = 0;
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    v[j] = (uint64_t)ga[j] | ((uint64_t)la[j] << 16) | ((uint64_t)gb[j] << 32) | ((uint64_t)lb[j] << 48);
-    sum += v[j];
-  }
-  uint64_t total;
-  uint64_t pre = block_scan<THREADS, uint64_t>(sum, warp_sums, total);
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int bin = 255 - ((int)threadIdx.x * 2 + j);
-    const int above_a = (int)(pre & 0xffffu), above_la = (int)((pre >> 16) & 0xffffu);
-    const int above_b = (int)((pre >> 32) & 0xffffu), above_lb = (int)(pre >> 48);
-    if (above_a < ka && above_a + ga[j] >= ka) { outa[0] = bin; outa[1] = above_a; outa[2] = above_la; }
-    if (above_b < kb && above_b + gb[j] >= kb) { outb[0] = bin; outb[1] = above_b; outb[2] = above_lb; }
     pre += v[j];
   }
   __syncthreads();
