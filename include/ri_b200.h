@@ -96,7 +96,9 @@ typedef struct ri_wave_layer {
 int64_t ri_wave_scratch_bytes(const ri_wave_layer* p);
 
 /* Launch scan + select + attend for one layer on `stream`.  The scratch needs no initialisation:
- * every stage writes what a later stage reads. */
+ * every stage writes what a later stage reads.
+ * The single kernel's CTAs wait for one another (bounded): a wait that runs out leaves its number, 51 .. 55, in the process's
+ * status word (ri_status_word) and d_out without that group's result.  Look at the word after the call. */
 int ri_wave_decode_layer(const ri_wave_layer* p, void* stream);
 
 /* Same work as ri_wave_decode_layer for callers that cannot allocate device memory at all: an
@@ -109,7 +111,8 @@ int ri_wave_decode_layer(const ri_wave_layer* p, void* stream);
  * which no stage depends on.  All calls share the one
  * array, so calls whose GPU work overlaps (other streams, unordered threads) race: order them.
  * The first call on each device looks up the array's device address; make it at start-up,
- * before any stream capture.  This entry point has no counterpart in the reference. */
+ * before any stream capture.  Like ri_wave_decode_layer it reports in the status word, four bytes of page-locked HOST memory
+ * that the first call of the process makes (no device memory).  This entry point has no counterpart in the reference. */
 #define RI_WAVE_STATIC_SCRATCH_BYTES (16u << 20)
 int ri_wave_decode_layer_static(const ri_wave_layer* p, void* stream);
 

@@ -9,7 +9,8 @@ import torch
 
 from .. import _lib
 from ..kernels import weighted_flash_decoding
-from .retroinfer_attn import _status_word, check_prefill_errors, retroinfer_prefill_attn
+from ..status import report
+from .retroinfer_attn import _status_word, check_prefill_errors, retroinfer_prefill_attn  # noqa: F401
 
 
 def prefill_full_flash_attn(query_states, key_states, value_states, causal):
@@ -52,8 +53,7 @@ def decode_full_flash_attn(query_states, key_states, value_states, layer_idx, fu
             query_states.data_ptr(), key_states.data_ptr(), value_states.data_ptr(), c.valid_length.data_ptr(), extra,
             out.data_ptr(), scratch.data_ptr(), C.addressof(status), b, hk, gs, length, _lib.dtype_code(out.dtype), _lib.current_stream()),
             "ri_dense_decode")
-        if status.value and not torch.cuda.is_current_stream_capturing():
-            check_prefill_errors()
+        report(status)
         return out
     valid = c.valid_length + extra
     seqlens = valid.to(query_states.device).to(torch.int32).repeat_interleave(hk)

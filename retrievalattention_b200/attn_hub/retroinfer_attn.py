@@ -5,24 +5,9 @@ import ctypes as C
 
 import torch
 
-from .. import _lib
+from .. import _lib, status as _status
 
-# Where the prefill and dense decode kernels record that a device-side wait gave up, and the dense append that a row did not
-# fit (0: none of it): one word in page-locked host memory for all devices and streams, replays of CUDA graphs among them.  The kernels only write it, so a failure stays
-# inside its call; it stays set until it is reported, by ``check_prefill_errors`` or by the first call that finds it set.
-_word = None
-_devices: set = set()
-
-
-def _status_word(device) -> C.c_int32:
-    global _word
-    if _word is None:
-        address = _lib.lib.ri_status_word()          # the same for every thread that gets here
-        if not address:
-            raise RuntimeError(f"ri_status_word: {_lib.lib.ri_last_error().decode()}")
-        _word = C.c_int32.from_address(address)
-    _devices.add(device)
-    return _word
+_status_word = _status.word
 
 
 def retroinfer_prefill_attn(query_states, key_states, value_states, causal):
@@ -43,22 +28,14 @@ def retroinfer_prefill_attn(query_states, key_states, value_states, causal):
     _lib.check(_lib.lib.ri_prefill_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), None,
                                         C.addressof(status), b, s, hq, hk, int(bool(causal)), _lib.dtype_code(q.dtype),
                                         _lib.current_stream()), "ri_prefill_attn")
-    if status.value and not torch.cuda.is_current_stream_capturing():
-        check_prefill_errors()
+    _status.report(status)
     return out
 
 
 def check_prefill_errors() -> None:
-    """Raise if any prefill or dense decode call since the last check, replays of captured ones among them, gave up on a
-    device-side wait, or a dense cache was full when a row was appended (synchronises)."""
-    for device in list(_devices):
-        torch.cuda.synchronize(device)
-    code = 0 if _word is None else _word.value
-    if code:
-        _word.value = 0
-        if code == _lib.RI_STATUS_CACHE_FULL:
-            raise RuntimeError("a token's rows did not fit the dense cache (more decode steps than max_length has room for)")
-        raise RuntimeError(f"ri_prefill_attn or ri_dense_decode gave up on a device-side wait (code {code})")
+    """Raise if any prefill or decode call (dense or wave index) since the last check, replays of captured ones among them, gave
+    up on a device-side wait, or a dense cache was full when a row was appended (synchronises)."""
+    _status.check()
 
 
 def retroinfer_decode_attn(query_states, key_states, value_states, layer_idx, retroinfer_cache, query_states_next=None):

@@ -16,7 +16,7 @@ from dataclasses import dataclass
 
 import torch
 
-from . import _lib
+from . import _lib, status
 
 
 @dataclass
@@ -103,6 +103,7 @@ class WaveIndexLayer:
         p.d_retrieved_kept = _lib.ptr(self.retrieved_kept)
         p.d_estimated_ids = _lib.ptr(self.estimated_ids)
         self.params = p
+        self._status = status.word(dev)      # where the decode kernel says that a wait ran out
 
     def _bind(self, q: torch.Tensor, out: torch.Tensor) -> None:
         s = self.shape
@@ -136,6 +137,7 @@ class WaveIndexLayer:
         else:
             _lib.check(_lib.lib.ri_wave_decode_layer_gather(C.byref(self.params), C.byref(gather), _lib.current_stream()),
                        "ri_wave_decode_layer_gather")
+        status.report(self._status)
         return out
 
     def compute_staged(self, q: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -158,6 +160,7 @@ class WaveIndexLayer:
         self._bind(q, out)
         _lib.check(_lib.lib.ri_wave_decode_layer_static(C.byref(self.params), _lib.current_stream()),
                    "ri_wave_decode_layer_static")
+        status.report(self._status)
         return out
 
     def attend_buffer(self, q: torch.Tensor, out: torch.Tensor, exec_keys: torch.Tensor, exec_values: torch.Tensor,
