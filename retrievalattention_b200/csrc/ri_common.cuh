@@ -63,6 +63,12 @@ struct Elem<RI_BF16> {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
   }
+  // two values, infinities replaced by the largest finite value of their sign
+  __device__ __forceinline__ static uint32_t finite2(uint32_t x) {
+    uint32_t d;
+    asm("min.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(x), "r"(0x7f7f7f7fu));
+    return d;
+  }
   __device__ __forceinline__ static void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                                   uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -81,6 +87,12 @@ struct Elem<RI_F16> {
   __device__ __forceinline__ static uint32_t pack2(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
+  }
+  // two values, infinities replaced by the largest finite value of their sign
+  __device__ __forceinline__ static uint32_t finite2(uint32_t x) {
+    uint32_t d;
+    asm("min.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(d) : "r"(x), "r"(0x7bff7bffu));
+    return d;
   }
   __device__ __forceinline__ static void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                                   uint32_t a3, uint32_t b0, uint32_t b1) {

@@ -84,7 +84,8 @@ struct AttendArgs {
 };
 
 // acc += P.V for 16 rows.  b0, b1: this lane's four probabilities in the 16-bit type; TWO: l0, l1 is what that rounding left
-// over, multiplied too.
+// over, multiplied too.  Those may be zero or have the other sign, and an infinite value times them would make NaN of the
+// infinity that the first product gives: the second one takes the largest finite value instead.
 template <int DT, bool TWO = false>
 __device__ __forceinline__ void pv_step(float (&acc)[8][4], const uint4 (&v)[4][2], uint32_t b0, uint32_t b1, uint32_t l0 = 0,
                                         uint32_t l1 = 0) {
@@ -101,7 +102,9 @@ __device__ __forceinline__ void pv_step(float (&acc)[8][4], const uint4 (&v)[4][
     }
     if (TWO)
 #pragma unroll
-      for (int w = 0; w < 4; ++w) Elem<DT>::mma16816(acc[4 * piece + w], m[w][0], m[w][1], m[w][2], m[w][3], l0, l1);
+      for (int w = 0; w < 4; ++w)
+        Elem<DT>::mma16816(acc[4 * piece + w], Elem<DT>::finite2(m[w][0]), Elem<DT>::finite2(m[w][1]), Elem<DT>::finite2(m[w][2]),
+                           Elem<DT>::finite2(m[w][3]), l0, l1);
   }
 }
 // Two probabilities in the 16-bit type, and (second word) what the rounding left over.
