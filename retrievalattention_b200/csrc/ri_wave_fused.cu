@@ -898,12 +898,16 @@ __global__ void __launch_bounds__(kFusedThreads, 1) wave_fused_kernel(FusedArgs 
     RI_FT(13);
   }
   // A CTA leaves when all that was meant for it has arrived.  One that gave up does not know that: it waits here until the
-  // others, which do not arrive at this barrier, have left.
+  // others have left or gave up too (a CTA that has left counts as arrived).  Twice, because the others' next barrier may be the
+  // one behind the global lists, after which they still push; and a while longer, for what a CTA pushed just before it left.
   __syncthreads();
   if (s_abort) {
     if (tid == 0) *f.status = s_abort;
     cluster_arrive();
     cluster_wait();
+    cluster_arrive();
+    cluster_wait();
+    for (int i = 0; i < 20; ++i) __nanosleep(1000);
   }
 }
 
