@@ -155,7 +155,8 @@ int ri_wave_attend_buffer_lse(const ri_wave_layer* p, const void* d_exec_keys, c
  * then, so its stores are ordered before the flags, and each flag store follows a system-scope fence
  * — and (2) waits until the flag words of all ranks hold the epoch; whatever is enqueued after it
  * may read the complete gather buffer.  The wait is bounded: after wait_limit_us it sets *d_error
- * and returns, so a missing rank never hangs the GPU.
+ * and returns, so a missing rank never hangs the GPU.  Where the decode kernel itself gave up (see ri_wave_decode_layer) it leaves
+ * 2 in *d_error; the wait behind it then raises no flags, so that every other rank's wait runs out, sets *d_error to 1 and returns.
  * *d_epoch is read on the device: the caller increases it once per step (the same value on every
  * rank) before the step's first launch. */
 typedef struct ri_wave_gather {
@@ -167,7 +168,7 @@ typedef struct ri_wave_gather {
   uint32_t* const* d_flag_slots;   /* device array [n_ranks]: this rank's flag word (this layer) on each rank */
   const uint32_t* d_flags;         /* local: this layer's flag words, one per rank */
   const uint32_t* d_epoch;         /* local: [1] the current step's epoch */
-  int32_t* d_error;                /* local: set to 1 when a wait ran out */
+  int32_t* d_error;                /* local: set to 1 when a wait ran out or this rank's slice is missing */
   unsigned long long* d_stamps;    /* optional (may be NULL), local [3]: the wait kernel's global-timer readings (ns) at
                                       entry, after this rank's flags are raised, and when the last rank's flag was seen */
 } ri_wave_gather;

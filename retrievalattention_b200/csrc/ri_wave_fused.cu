@@ -42,6 +42,8 @@ constexpr int kFusedMaxCentroids = 16384;             // per group: four CTAs of
 // groups in clusters of 4: 36 -> 40 us): the kernel exists for up to 8 and for up to 16 (MAXCL).
 constexpr int kMaxCluster = 16;
 constexpr int kScanStages = 2;
+// In a gather's error word, from a decode kernel that gave up to the wait kernel behind it: a slice is missing.
+constexpr int kSliceMissing = 2;
 
 // What follows from the centroids a thread looks after in the selection (KEYS; a CTA's slice has at most 256 * KEYS).
 template <int KEYS>
@@ -67,6 +69,7 @@ struct FusedArgs {
   const uint4* cent;
   float* scores;     // global copy of the scores (a view for tests), written only when `views`
   int32_t* status;   // the process's status word
+  int32_t* gather_error;   // several GPUs: the gather's error word
   float alpha;
   int views;         // also fill the global lists and views (tests, callers that asked for the id outputs)
   uint4* steady_k_w;       // att.new_k / new_v go to row static_len - 1 of these
@@ -902,7 +905,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) wave_fused_kernel(FusedArgs 
   // one behind the global lists, after which they still push; and a while longer, for what a CTA pushed just before it left.
   __syncthreads();
   if (s_abort) {
-    if (tid == 0) *f.status = s_abort;
+    if (tid == 0) {
+      *f.status = s_abort;
+      if (f.gather_error) *f.gather_error = kSliceMissing;
+    }
     cluster_arrive();
     cluster_wait();
     cluster_arrive();
@@ -912,15 +918,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) wave_fused_kernel(FusedArgs 
 }
 
 // After the decode kernel of the same stream: raise this rank's flag on every rank, then wait (bounded) until
-// every rank's flag here holds this step's epoch.  Thread r looks after rank r.
+// every rank's flag here holds this step's epoch.  Thread r looks after rank r.  Where the decode kernel left a slice out, no flag
+// is raised: the other ranks' waits run out and say so too.
 __global__ void gather_signal_wait_kernel(uint32_t* const* flag_slots, const uint32_t* flags, const uint32_t* epoch,
                                           int32_t* error, int n_ranks, long long limit_ns, unsigned long long* stamps) {
   ri_pdl_enter();
   const int r = threadIdx.x;
-  if (r >= n_ranks) return;
   unsigned long long t_in;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_in));
   const uint32_t expected = *epoch;
+  if (__syncthreads_or(*error == kSliceMissing)) {     // both words are on their way at once
+    if (r == 0) *error = 1;
+    return;
+  }
+  if (r >= n_ranks) return;
   // the decode kernel has completed (stream order), so its stores to the other GPUs happen before this fence,
   // and the fence orders them before the flag at system scope
   asm volatile("fence.acq_rel.sys;" ::: "memory");
@@ -1045,6 +1056,7 @@ int launch(const ri_wave_layer& p, const Layout& L, int cl, cudaStream_t s, cons
   for (int i = 0; i < 20; ++i)
     if (p.page_size == 1 << i) f.page_shift = i;
   f.out_aligned = (uintptr_t)p.d_out % 8 == 0;
+  f.gather_error = gather ? gather->d_error : nullptr;
   if (gather) {
     f.att.copies = reinterpret_cast<uint16_t* const*>(gather->d_out_slots);
     f.att.n_copies = gather->n_ranks;

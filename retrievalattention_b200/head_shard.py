@@ -202,5 +202,5 @@ class PeerGather:
                 "wait_min": round(float(wait.min()), 2), "wait_max": round(float(wait.max()), 2)}
 
     def timed_out(self) -> bool:
-        """True when some wait gave up (reads one word from the device)."""
+        """True when some wait gave up or this rank's decode kernel left a slice out (reads one word from the device)."""
         return bool(self.error.item())
