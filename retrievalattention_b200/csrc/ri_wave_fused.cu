@@ -888,15 +888,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) wave_fused_kernel(FusedArgs 
       for (int i = 0; i < 4; ++i) bits[i] = Elem<DT>::bits(L > 0.f ? inv[i] / L : 0.f);
       const int64_t at = (int64_t)g * gs * RI_HEAD_DIM + (first + tid) * 4;
       uint16_t* out = reinterpret_cast<uint16_t*>(f.att.out) + at;
-      if (f.out_aligned) {
-        *reinterpret_cast<uint2*>(out) = make_uint2(bits[0] | ((uint32_t)bits[1] << 16), bits[2] | ((uint32_t)bits[3] << 16));
-      } else {
+      const uint2 all = make_uint2(bits[0] | ((uint32_t)bits[1] << 16), bits[2] | ((uint32_t)bits[3] << 16));
+      auto store = [&](uint16_t* to, bool aligned) {
+        if (aligned) {
+          *reinterpret_cast<uint2*>(to) = all;
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) out[i] = bits[i];
+          for (int i = 0; i < 4; ++i) to[i] = bits[i];
+        }
+      };
+      store(out, f.out_aligned);
+      for (int c = 0; c < f.att.n_copies; ++c) {    // several GPUs: every rank's gather buffer
+        uint16_t* to = f.att.copies[c] + at;
+        store(to, (uintptr_t)to % 8 == 0);
       }
-      for (int c = 0; c < f.att.n_copies; ++c)      // several GPUs: the other ranks' gather buffers
-#pragma unroll
-        for (int i = 0; i < 4; ++i) f.att.copies[c][at + i] = bits[i];
     }
     RI_FT(13);
   }
