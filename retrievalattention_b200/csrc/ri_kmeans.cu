@@ -908,13 +908,16 @@ constexpr int kWindows = 4;         // steps in the ring
 
 // LONG: clusters of kLongCluster members and more are left to the whole CTA, which sums them when its warps are done with the
 // others.  Through the ring such a cluster is one warp's chain of 75 clocks a row, every four rows of which wait, shuffle and
-// compare; the CTA streams its rows through twice the depth, and a thread adds one channel of a row after the other, in the same
-// order.  The initial centroids are rows as they are, and those of the longest keys win most of a segment: the first two updates
-// are launched in this form (8 heads x 128K rows: 75 -> 92 and 294 -> 136 us, 8K rows 28 and 14 us either way), the later ones
-// without it.
+// compare; the CTA streams its rows in batches of 32, two of them ahead of the one that is added (a warp's ring: 12 rows), and a
+// thread adds one channel of a row after the other, in the same order.  The initial centroids are rows as they are, and those of
+// the longest keys may win most of a segment: the first two updates are launched in this form, the later ones without it.  Whole
+// builds against all updates without it (us, B200): 8 heads x 128K rows 3979 -> 3782, 4 x 20K 835 -> 566, 8 x 17K fp16 894 -> 662;
+// where no cluster is long 2420 -> 2417 (8 x 91K) and 1915 -> 1913 (8 x 75K).  Three batches are 24 KB, nine CTAs an SM; with five
+// (40 KB, five CTAs) the last two took 2441 and 1939, the others no less; with four of 16 rows 8 x 17K took 680.  For the second
+// update alone: 4 x 32K fp16 847 instead of 761, 2 x 59K 652 instead of 622.
 constexpr int kLongCluster = 512;
 constexpr int kLongRows = 32;       // rows of a batch
-constexpr int kLongBatches = 5;     // batches in shared memory
+constexpr int kLongBatches = 3;     // batches in shared memory
 
 template <int DT, bool LAST, bool LONG>
 __global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArgs a) {
