@@ -1081,6 +1081,7 @@ __global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArg
     if (done < at) {
       stream(at, start, __shfl_sync(0xffffffffu, my_end, at - 1) - start);
       cp_async_wait<0>();
+      __syncwarp();                                           // all lanes are done with the ring: the next stream fills it anew
     }
     if (!rest) break;
     start = end;                                              // not now
