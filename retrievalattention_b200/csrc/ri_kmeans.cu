@@ -874,7 +874,7 @@ struct UpdateArgs {
   int64_t out_group;
   int n_tok, n_cen, seg_per_group, normalize;
   int64_t group_stride;
-  int clusters_per_warp, n_clusters;   // n_clusters: over all problems
+  int clusters_per_warp;
 };
 
 template <int DT>
@@ -929,11 +929,8 @@ __global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArg
   __shared__ float s_sum[LONG ? 128 : 1];
   const int lane = threadIdx.x & 31;
   const int job = (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5);
-  // clusters_per_warp divides n_cen: one problem per warp.  LONG: a warp without clusters takes the last ones, which another warp
-  // of the CTA has, and leaves them alone
-  const bool idle = job * a.clusters_per_warp >= a.n_clusters;
-  if (!LONG && idle) return;
-  const int idx0 = LONG && idle ? a.n_clusters - a.clusters_per_warp : job * a.clusters_per_warp;
+  // n_cen is a multiple of 32 and clusters_per_warp 1, 2, 4 or 8: the warps of a CTA all have clusters, and of one problem
+  const int idx0 = job * a.clusters_per_warp;
   const int problem = idx0 / a.n_cen, z = problem / a.seg_per_group;
   int c = idx0 - problem * a.n_cen;
   const int tok_in_group = (problem - z * a.seg_per_group) * a.n_tok;
@@ -1074,8 +1071,7 @@ __global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArg
     return;
   }
   const int end_before = __shfl_up_sync(0xffffffffu, my_end, 1), my_start = lane > 0 ? end_before : first;
-  unsigned todo = __ballot_sync(0xffffffffu, !idle && lane < a.clusters_per_warp && my_end - my_start >= kLongCluster);
-  if (idle) done = a.clusters_per_warp;
+  unsigned todo = __ballot_sync(0xffffffffu, lane < a.clusters_per_warp && my_end - my_start >= kLongCluster);
   for (unsigned rest = todo;; rest &= rest - 1) {
     const int at = rest ? __ffs(rest) - 1 : a.clusters_per_warp;      // the next long one, or the end
     if (done < at) {
@@ -1098,11 +1094,8 @@ __global__ void __launch_bounds__(kUpdateThreads) kmeans_update_kernel(UpdateArg
     for (int w = 0; w < kWarps; ++w) {
       if (s_long[w][0] < 0) continue;                         // the same for every warp of the CTA
       const int l_from = s_long[w][1], l_n = s_long[w][2] - l_from;
-      // the problem of that warp's clusters (a CTA's warps may work on several)
-      const int l_idx = min(((int)blockIdx.x * kWarps + w) * a.clusters_per_warp, a.n_clusters - 1);
-      const int l_problem = l_idx / a.n_cen, l_z = l_problem / a.seg_per_group, l_tok = (l_problem - l_z * a.seg_per_group) * a.n_tok;
-      const int32_t* l_ord = a.order + (int64_t)l_z * a.group_stride + l_tok + l_from;
-      const uint4* l_rows = reinterpret_cast<const uint4*>(a.rows) + ((int64_t)l_z * a.src.group + (int64_t)l_tok * a.src.row) * 16 + (tid & 15);
+      const int32_t* l_ord = ord + l_from;
+      const uint4* l_rows = reinterpret_cast<const uint4*>(a.rows) + src0;
       const uint32_t batch = (uint32_t)__cvta_generic_to_shared(&ring[0][0]);
       constexpr int kCopies = kLongRows * 16 / kUpdateThreads;      // 16-byte pieces of a batch per thread
       int id[kCopies];
@@ -1303,13 +1296,13 @@ int run_fit(const ri_kmeans* p, const FitLayout& L, const Place& pl, const void*
       }
     }
     RI_REQUIRE((int64_t)n_cen * problems < (1ll << 30), "too many clusters in one launch (%d x %d)", n_cen, problems);
-    ua.n_clusters = n_cen * problems;
+    const int n_clusters = n_cen * problems;
     // clusters per warp: a longer run of rows hides more latency, but enough warps for a few rounds of the chip
     int cpw = 8;
-    while (cpw > 1 && ua.n_clusters / cpw < sms * 96) cpw >>= 1;
+    while (cpw > 1 && n_clusters / cpw < sms * 96) cpw >>= 1;
     ua.clusters_per_warp = cpw;
     constexpr int per_cta = kUpdateThreads / 32;
-    const dim3 ugrid((ua.n_clusters / cpw + per_cta - 1) / per_cta);
+    const dim3 ugrid(n_clusters / cpw / per_cta);               // without remainder: n_cen is a multiple of 32
     RI_CUDA_OK(last     ? ri_launch_pdl_id(9, kmeans_update_kernel<DT, true, false>, ugrid, dim3(kUpdateThreads), 0, s, ua)
                : it < 2 ? ri_launch_pdl_id(9, kmeans_update_kernel<DT, false, true>, ugrid, dim3(kUpdateThreads), 0, s, ua)
                         : ri_launch_pdl_id(9, kmeans_update_kernel<DT, false, false>, ugrid, dim3(kUpdateThreads), 0, s, ua));
