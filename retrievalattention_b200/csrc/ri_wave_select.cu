@@ -33,7 +33,7 @@ wave_select_kernel(SelectArgs a) {
     }
     if (lane == 0) { s_max[warp] = M; s_inv[warp] = 1.0f / S; }
   }
-  select_body<DT, kSelectThreads, false>(a, dyn, g, s_max, s_inv);
+  select_body<DT, kSelectThreads>(a, dyn, g, s_max, s_inv);
 }
 
 template <int DT>

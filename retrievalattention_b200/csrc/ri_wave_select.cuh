@@ -131,11 +131,9 @@ __device__ __forceinline__ void find_bins(const int* ga, const int* la, int ka, 
 
 // Steps 2-6 for group `g`.  `dyn`: select_dyn_bytes() of 16-byte aligned shared memory; `s_max`,
 // `s_inv`: the per-head softmax statistics in shared memory (a block barrier inside orders the
-// caller's writes before their first use).  LATE_ARRIVE = false: the last cluster barrier is
-// armed before the row list is stored, so that its release does not wait for those stores (nothing
-// in the same kernel reads them).  LATE_ARRIVE = true: it is armed after them, behind a fence, so
-// that the other CTAs of the cluster may read every global result of this function afterwards.
-template <int DT, int THREADS, bool LATE_ARRIVE>
+// caller's writes before their first use).  The last cluster barrier is armed before the row list is
+// stored, so that its release does not wait for those stores (nothing in the same kernel reads them).
+template <int DT, int THREADS>
 __device__ __forceinline__ void select_body(const SelectArgs& a, uint8_t* dyn, int g, const float* s_max,
                                             const float* s_inv) {
   static_assert(THREADS == 128 || THREADS == 256, "select_body: 128 or 256 threads");
@@ -399,7 +397,7 @@ __device__ __forceinline__ void select_body(const SelectArgs& a, uint8_t* dyn, i
     d_cnt = (int)cluster.map_shared_rank(rcnt, 0)[my_i];
     d_start = (int)cluster.map_shared_rank(rstart, 0)[my_i];
   }
-  if (!LATE_ARRIVE) cluster_arrive();
+  cluster_arrive();
   const int n_mine = (keep - (rank * kWarps + warp) + kWarpsTotal - 1) / kWarpsTotal;
   for (int l = 0; l < n_mine; ++l) {
     const int off = __shfl_sync(0xffffffffu, d_off, l), cnt = __shfl_sync(0xffffffffu, d_cnt, l);
@@ -420,10 +418,6 @@ __device__ __forceinline__ void select_body(const SelectArgs& a, uint8_t* dyn, i
     }
     if (a.retrieved_ids)
       for (int i = tid; i < a.P; i += THREADS) a.retrieved_ids[(int64_t)g * a.P + i] = 0xffff - (int)(ranked[i] & 0xffffu);
-  }
-  if (LATE_ARRIVE) {
-    __threadfence();
-    cluster_arrive();
   }
   cluster_wait();   // CTA 0's shared memory must outlive the remote reads above
 }
