@@ -135,11 +135,12 @@ __device__ __forceinline__ void cluster_wait() {
 constexpr float RI_LOG2E = 1.4426950408889634f;
 
 // ---- programmatic dependent launch ------------------------------------------------------------
-// Every kernel of the decode chain starts with ri_pdl_enter(): it lets the next kernel in the
-// stream be scheduled right away (its CTAs become resident and run up to their own
-// ri_pdl_enter) and then waits until the previous kernel has completed and its writes are
-// visible.  All global reads and writes of a kernel come after this call, so the chain keeps
-// plain stream-order semantics while the launch latency between dependent kernels is hidden.
+// A kernel launched so starts with ri_pdl_enter(): it lets the next kernel in the stream be
+// scheduled right away (its CTAs become resident and run up to their own wait) and then waits until
+// the previous kernel has completed and its writes are visible.  All global reads and writes of a
+// kernel come after the wait, so the chain keeps plain stream-order semantics while the launch
+// latency between dependent kernels is hidden.  The single decode kernel calls the two halves
+// itself: between them it sets up its barriers and asks for centroids in L2, which reads nothing.
 // Launched without the attribute (or after a non-kernel operation) both instructions are no-ops.
 // Measured on B200: worth a few tenths of a microsecond per launch for scan and select (ids 0, 1,
 // on by default).  The attend kernel (id 2: 8-CTA clusters with ~100 KB of shared memory each)

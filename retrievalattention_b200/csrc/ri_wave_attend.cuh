@@ -5,8 +5,8 @@
 // (reference: the two weighted_flash_decoding calls, cache_hub/retroinfer_cache.py:611-617 and
 // :666-674, with gather_copy_vectors :601-605 and gather_copy_and_concat :642-648 in between).
 //
-// Work decomposition: a fixed, SM-filling grid of 8-CTA clusters (2 CTAs per SM, 4 warps each); a
-// cluster works on one group at a time.  Inside a group the 16-row steps (ceil(E/16) estimation steps, then
+// Work decomposition of the stand-alone kernel: a fixed, SM-filling grid of 8-CTA clusters (2 CTAs
+// per SM, 4 warps each); a cluster works on one group at a time.  Inside a group the 16-row steps (ceil(E/16) estimation steps, then
 // ceil((steady + retrieved rows)/16) exact steps) are cut into equal-cost contiguous ranges, one
 // per warp (an exact step moves twice the bytes of an estimation step).  A warp streams its steps
 // through a lane-private three-stage cp.async ring in shared memory (256 bytes per lane and step;
@@ -23,8 +23,8 @@
 // row r is channel ch(x) = (x<4 ? 8r+2x : 64+8r+2(x-4)) and row r+8 is ch(x)+1.  The probabilities
 // come straight from the QK^T accumulators as the B fragment.
 //
-// The per-group body is a device function shared by the stand-alone kernel and the single-kernel
-// decode path.
+// A warp's steps (attend_steps) are shared by the stand-alone kernel and the single decode kernel
+// (clusters of 1 .. 16 CTAs of 8 warps), which shares them out and merges in its own way.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -116,7 +116,7 @@ __device__ __forceinline__ uint2 split2(float p0, float p1) {
 
 struct RowIds { int k[2]; int v[4]; };   // >= 0: row of the KV store / cluster id; < 0: steady row -1-id
 
-// Shared-memory lists of the single-kernel path (LOCAL mode of attend_group): this CTA's own estimation
+// Shared-memory lists of the single-kernel path (LOCAL mode of attend_steps): this CTA's own estimation
 // entries and its range of the group's exact steps, the retrieved rows given by the kept clusters.
 struct LocalLists {
   const uint32_t* est;       // [n_est] centroid index inside this CTA's slice, ascending; above it the weight (cluster size) in
@@ -158,7 +158,7 @@ __device__ __forceinline__ void attend_steps(const AttendArgs& a, const int g, c
   constexpr int kStageStride = WARPS * kStageBytes;
   const int new_row = a.new_k != nullptr ? static_len - 1 : -1;
   // The step sequence this CTA's warps share: LOCAL: its own estimation steps, then its exact steps
-  // [x_lo, x_hi); otherwise the whole group's estimation steps, then all exact steps, shared by all 32 warps.
+  // [x_lo, x_hi); otherwise the whole group's estimation steps, then all exact steps, shared by all cpg * WARPS warps.
   const int x_first = LOCAL ? ll->x_lo : 0;
   const int xs = LOCAL ? ll->x_hi - ll->x_lo : (te + 15) / 16;
   const int n_est_rows = LOCAL ? ll->n_est : a.E;

@@ -1,4 +1,4 @@
-// The whole decode step of one layer in ONE kernel: a thread-block cluster per group (1 .. 8 CTAs of 256 threads, one CTA
+// The whole decode step of one layer in ONE kernel: a thread-block cluster per group (1 .. 16 CTAs of 256 threads, one CTA
 // per SM; see cluster_size) runs
 //   phase 1  scan    s = alpha * q.C^T over the group's centroids (each CTA one slice, streamed through a lane-private
 //                    cp.async ring), scores kept in shared memory;
@@ -88,9 +88,9 @@ __host__ __device__ constexpr int chunks_per_cta(int gs, int cl) { return (gs * 
 __host__ __device__ constexpr int mail_bytes(int gs, int cl) {
   return cl * kFusedWarps * kMaxHeads * 8 + cl * chunks_per_cta(gs, cl) * 24;
 }
-// Temporary arrays of the selection: histograms pushed by every CTA (256 and 512 16-bit counts), the candidates, and five words a
-// candidate for ranking.
-__host__ __device__ constexpr int temp_bytes(int p_pad, int cl) { return cl * 1536 + p_pad * 36; }
+// Temporary arrays of the selection: histograms pushed by every CTA (256 and 512 16-bit counts), and of each candidate its entry
+// (four words) and four words for ranking.
+__host__ __device__ constexpr int temp_bytes(int p_pad, int cl) { return cl * 1536 + p_pad * 32; }
 __host__ __device__ constexpr int range_bytes(int p_pad) { return (2 * p_pad + 4) * 4; }
 __host__ __device__ constexpr int entry_bytes(int gs) { return 4 * gs + 4; }   // scores; index and size
 
