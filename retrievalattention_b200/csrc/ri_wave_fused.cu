@@ -158,15 +158,18 @@ struct ThreadClusters {
                        : "=r"(cnt[4 * q4]), "=r"(cnt[4 * q4 + 1]), "=r"(cnt[4 * q4 + 2]), "=r"(cnt[4 * q4 + 3])
                        : "l"(sel.count + gc + 4 * q4));
       asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(off0) : "l"(sel.offset + (int64_t)g * (sel.C + 1) + lo + e0));
-      if constexpr (KEYS == 4) {
-        asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(szw[0]), "=r"(szw[1]) : "l"(sel.size_dt + gc));
-      } else {
+      if (KEYS >= 8 && (uintptr_t)sel.size_dt % 16 == 0) {      // 8-byte alignment is all that the sizes need
 #pragma unroll
         for (int q8 = 0; q8 < KEYS / 8; ++q8)
           if (q8 == 0 || e0 + 8 < n_loc)
             asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
                          : "=r"(szw[4 * q8]), "=r"(szw[4 * q8 + 1]), "=r"(szw[4 * q8 + 2]), "=r"(szw[4 * q8 + 3])
                          : "l"(sel.size_dt + gc + 8 * q8));
+      } else {
+#pragma unroll
+        for (int q4 = 0; q4 < KEYS / 4; ++q4)
+          if (q4 < 2 || e0 + 8 < n_loc)
+            asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(szw[2 * q4]), "=r"(szw[2 * q4 + 1]) : "l"(sel.size_dt + gc + 4 * q4));
       }
     }
   }
