@@ -154,7 +154,7 @@ __device__ __forceinline__ void attend_steps(const AttendArgs& a, const int g, c
   const int gs = a.gs, es = LOCAL ? (ll->n_est + 15) / 16 : a.e_steps;
   // ring: stage-major, slot (stage, warp) at (stage * WARPS + warp) * kStageBytes
   const uint32_t my_ring = (uint32_t)__cvta_generic_to_shared(ring) + warp * kStageBytes + lane * 16;
-  const uint8_t* my_ring_ptr = ring + warp * kStageBytes + lane * 16;
+  uint8_t* my_ring_ptr = ring + warp * kStageBytes + lane * 16;
   constexpr int kStageStride = WARPS * kStageBytes;
   const int new_row = a.new_k != nullptr ? static_len - 1 : -1;
   // The step sequence this CTA's warps share: LOCAL: its own estimation steps, then its exact steps
@@ -324,6 +324,17 @@ __device__ __forceinline__ void attend_steps(const AttendArgs& a, const int g, c
     if (j == 0) RI_FT(10);
     const uint8_t* src = my_ring_ptr + stage * kStageStride;
     const int rows_end = is_est ? n_est_rows : te;
+    // rows past the end have probability zero but are copies of the last one, whose values may be infinite: zeros in their place,
+    // written by the lane that reads them
+    if (base + 16 > rows_end) {
+      uint8_t* own = my_ring_ptr + stage * kStageStride;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (base + (i >> 1) * 8 + 2 * t + (i & 1) >= rows_end) {
+          *reinterpret_cast<uint4*>(own + (8 + 2 * i) * 512) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(own + (9 + 2 * i) * 512) = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
 
     float s2[2][2];
     float w[2][2] = {{1.f, 1.f}, {1.f, 1.f}};
