@@ -49,7 +49,7 @@ SINK, RECENT = 4, 64
 FALLBACK_HBM_GBS = 6650.0
 FALLBACK_BF16_TFLOPS = 1590.0
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, from ncu captures of one layer of configuration 1 (32 groups)
-NCU_TRAFFIC = {"decode": 118.4e6, "scan": 70.18e6, "select": 6.33e6, "attend": 46.67e6}
+NCU_TRAFFIC = {"decode": 118.0e6, "scan": 70.18e6, "select": 6.33e6, "attend": 46.67e6}
 METRIC = "decode tok/s at 128K ctx (Llama-3-8B geometry); attn kernel HBM GB/s vs peak"
 
 
